@@ -790,13 +790,12 @@ lsmps_status lsmps_step_operators_backward(lsmps_ctx* ctx, const lsmps_fluid* fl
                                            const lsmps_step_operator_out* cotangent, const lsmps_vector* u_bar,
                                            double* p_bar, const lsmps_vector* x_bar);
 /* Form of lsmps_operators_backward (no counterpart in the reference).
- * 0 (default): deterministic -- the CSR is transposed (entries sorted stably
- * by neighbour) and every particle gathers the terms of its own row and of
- * the rows that list it in a fixed order, with no atomics; repeated calls give
- * the same bits.  Costs a sort of the K entries and 20 bytes of scratch per
- * entry.  1: each row scatters its terms into its neighbours with FP64
- * atomics (no transpose; the sums' order, and so the last bits, may vary
- * between calls). */
+ * 0 (default): deterministic -- each row's entries are evaluated once, the
+ * neighbours' shares kept as records that every particle adds in a fixed order
+ * (ascending entries); repeated calls give the same bits.  Costs 64 bytes of
+ * scratch per entry, at most 16 GB: a larger table is done in passes.  1: each
+ * row scatters its terms into its neighbours with FP64 atomics (no records;
+ * the sums' order, and so the last bits, may vary between calls). */
 lsmps_status lsmps_ctx_set_adjoint_atomic(lsmps_ctx* ctx, int on);
 
 #ifdef __cplusplus

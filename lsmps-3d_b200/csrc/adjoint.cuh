@@ -1,69 +1,67 @@
-// adjoint.cuh - pieces shared by the two differentiable operator pairs
-// (adjoint.cu: fluid-only operators; step_adjoint.cu: the step's operators
-// with their wall terms).
+// adjoint.cuh - what the two differentiable operator pairs share (adjoint.cu:
+// fluid-only operators; step_adjoint.cu: the step's operators with their wall
+// terms): the arguments of their kernels and the queueing of them
+// (operators.cu).
 #pragma once
 
 #include "common.cuh"
 
 namespace lsmps {
 
-constexpr int kAdjThreads = 128;
-
-// s = d / r_e and the Type-A basis of s (moment_matrix.cu:152-175).
-__device__ __forceinline__ void basis_div(double dx, double dy, double dz, double inv_re, double b[9], double s[3]) {
-  s[0] = dx * inv_re;
-  s[1] = dy * inv_re;
-  s[2] = dz * inv_re;
-  b[0] = s[0];
-  b[1] = s[1];
-  b[2] = s[2];
-  b[3] = s[0] * s[0];
-  b[4] = s[1] * s[1];
-  b[5] = s[2] * s[2];
-  b[6] = s[0] * s[1];
-  b[7] = s[1] * s[2];
-  b[8] = s[2] * s[0];
-}
-
-__device__ __forceinline__ double dot9(const double* a, const double* b) {
-  double v = 0.0;
-#pragma unroll
-  for (int k = 0; k < 9; ++k) v = fma(a[k], b[k], v);
-  return v;
-}
-
-// y = X r for the column-major symmetric 9x9 X.
-__device__ __forceinline__ void apply(const double* __restrict__ x, const double r[9], double y[9]) {
-#pragma unroll
-  for (int a = 0; a < 9; ++a) y[a] = 0.0;
-#pragma unroll
-  for (int c = 0; c < 9; ++c) {
-#pragma unroll
-    for (int a = 0; a < 9; ++a) y[a] = fma(x[a + c * 9], r[c], y[a]);
-  }
-}
-
-// J_b(s)^T beta: the derivative of b . beta with respect to s.
-__device__ __forceinline__ void basis_jt(const double s[3], const double beta[9], double out[3]) {
-  out[0] = beta[0] + 2.0 * s[0] * beta[3] + s[1] * beta[6] + s[2] * beta[8];
-  out[1] = beta[1] + 2.0 * s[1] * beta[4] + s[0] * beta[6] + s[2] * beta[7];
-  out[2] = beta[2] + 2.0 * s[2] * beta[5] + s[1] * beta[7] + s[0] * beta[8];
-}
-
-// The transpose of a CSR table (entries sorted stably by neighbour): the
-// entries that list particle j are tsrc[tb[j] .. te[j]) (entry offsets, in
-// ascending order; tb[j] = -1 when none), owner[o] the row of entry o.
-struct CsrTranspose {
-  index_t total;
-  index_t* tb;
-  index_t* te;
-  const index_t* tsrc;
-  index_t* owner;
+struct OperatorArgs {
+  index_t n;
+  const double4* fp;  // fluid {x, y, z, scalar}
+  const double4* fv;  // fluid {u_x, u_y, u_z, -}
+  const double4* wp;  // walls {x, y, z, -}, velocities, normals (with walls)
+  const double4* wv;
+  const double4* wn;
+  const index_t* fo;
+  const index_t* fi;
+  const index_t* wo;
+  const index_t* wi;
+  const int32_t* label;
+  const double* inv_v;  // [n][81] column-major
+  const double* inv_p;  // (= inv_v in the fluid-only pair)
+  const double* tr_v;   // traces before regularisation
+  const double* tr_p;
+  double re;
+  double inv_re;
+  double lam_w;
+  double lambda;
+  double rho;
+  double inv_dt;
+  double c_ppe;  // 2 / (r_e^2 rho)
+  double gx, gy, gz;
+  // Forward: the outputs.  Backward: their cotangents.  NULL: not wanted / 0.
+  double* lap_u[3];  // with walls
+  double* lap_f;     // fluid-only
+  double* grad[3];
+  double* div;
+  double* rhs;
+  double* wall_rhs;  // with walls
+  double* values;
+  index_t* row_offsets;  // forward only
+  index_t* columns;
+  // Backward: gradients (x, y, z components of u, the scalar, positions).
+  double* phibar[4];
+  double* xbar[3];
+  // Backward, deterministic form: per incoming entry of a particle a 64-byte
+  // record {4 field terms, 3 position terms, entry id}, in the order the owners'
+  // warps finish; next[j] the next free record of particle j, begin[j] its first
+  // and begin[j + 1] its end; own[8 j ..] the terms of j's own row.  Only the
+  // particles [j0, j1) have records in this pass, j0's first at records[0].
+  index_t* next;
+  const index_t* begin;
+  double4* records;
+  double* own;
+  index_t j0, j1;
 };
 
-// Queues the transpose of fn (its first n rows) on the context's stream, in
-// scratch taken from `scratch`; reads the entry count back first.
-lsmps_status build_csr_transpose(lsmps_ctx* ctx, Scratch& scratch, const lsmps_csr& fn, index_t n,
-                                 CsrTranspose* out);
+// Queue the forward (outputs in `a`), and the backward (cotangents in `a`,
+// deterministic or atomic as the context is set; reads the entry count back in
+// the deterministic form).  walls: the step's operators, else the fluid-only
+// ones.  The moments and the packs of `a` are queued before.
+lsmps_status operators_forward(lsmps_ctx* ctx, const OperatorArgs& a, bool walls);
+lsmps_status operators_backward(lsmps_ctx* ctx, const lsmps_csr& fn, OperatorArgs a, bool walls);
 
 }  // namespace lsmps

@@ -280,13 +280,12 @@ struct lsmps_ctx {
   // 1e6.
   double kappa_threshold = 1.0e4;
   // Operator forward/backward pair (adjoint.cu): fluid-only inverse, its
-  // trace / regularisation / info, and the backward's per-particle stash.
+  // trace / regularisation / info.
   double* adj_inverse = nullptr;
   double* adj_trace = nullptr;
   double* adj_reg = nullptr;
   int32_t* adj_info = nullptr;
   int32_t* adj_count = nullptr;
-  double* adj_stash = nullptr;
   size_t adj_cap = 0;
   // Backward form: false = transpose + gather (deterministic, the default),
   // true = scatter with FP64 atomics (lsmps_ctx_set_adjoint_atomic).
@@ -300,13 +299,12 @@ struct lsmps_ctx {
   const lsmps::PpeBoxOut* box_ppe = nullptr;
   // The step operator pair (step_adjoint.cu): inverses, traces,
   // regularisations, info and counts of the velocity Dirichlet-A and pressure
-  // Neumann-A kinds, and the backward's stash.
+  // Neumann-A kinds.
   double* sop_inverse[2] = {nullptr, nullptr};
   double* sop_trace[2] = {nullptr, nullptr};
   double* sop_reg[2] = {nullptr, nullptr};
   int32_t* sop_info[2] = {nullptr, nullptr};
   int32_t* sop_count = nullptr;
-  double* sop_stash = nullptr;
   size_t sop_cap = 0;
 };
 
