@@ -167,6 +167,41 @@ __device__ __forceinline__ double group_sum(double v, unsigned mask) {
   return v;
 }
 
+// Sums of N values over 2 D consecutive lanes (a lane group, or the warp with
+// D = 16), each exchange halving the values a lane still carries: lane l ends
+// with the totals of values base .. base + count - 1 in v[0 ..] (count 0, 1 or
+// more; call with base = 0, count = N).  About N exchanges instead of the
+// N log2(2 D) of N separate butterflies.  The order of the additions is fixed.
+template <int N, int D>
+__device__ __forceinline__ void lane_totals(double* v, int& base, int& count) {
+  if constexpr (D > 0) {
+    if constexpr (N == 1) {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], D);
+      lane_totals<1, D / 2>(v, base, count);
+    } else {
+      constexpr int H = (N + 1) / 2;
+      const bool upper = (threadIdx.x & D) != 0;
+#pragma unroll
+      for (int k = 0; k < H; ++k) {
+        const double hi = k + H < N ? v[k + H] : 0.0;
+        const double keep = upper ? hi : v[k];
+        const double send = upper ? v[k] : hi;
+        v[k] = keep + __shfl_xor_sync(0xffffffffu, send, D);
+      }
+      base += upper ? H : 0;
+      const int rest = count - H;
+      count = upper ? (rest > 0 ? rest : 0) : (count < H ? count : H);
+      lane_totals<H, D / 2>(v, base, count);
+    }
+  }
+}
+
+// The most values a lane may end lane_totals<N, D> with.
+__host__ __device__ constexpr int lane_totals_left(int n, int d) {
+  for (; d > 0; d /= 2) n = (n + 1) / 2;
+  return n;
+}
+
 }  // namespace lsmps
 
 // Opaque context of the C ABI.
@@ -259,11 +294,17 @@ struct lsmps_ctx {
   double4* pack_wall[3] = {nullptr, nullptr, nullptr};
   size_t pack_fluid_cap = 0;
   size_t pack_wall_cap = 0;
-  // Mixed form (LSMPS_PRECISION_MIXED): per fluid particle the 31 FP64 fluid
-  // moment sums ([31][n]) and the compact FP32 operator rows of the velocity
+  // Moment stage: per fluid particle the 31 (Type-B: 35) FP64 fluid moment
+  // sums ([sum][n]) and, plain form, at moment_cap x 35 the wall terms of both
+  // boundaries ([31][n], then [45][n]), all by visiting position.
+  double* moment_sums = nullptr;
+  int32_t* moment_walled = nullptr;   // plain form: visiting positions of the particles with walls
+  unsigned int* moment_walls = nullptr;  // ... and how many (0 between calls)
+  size_t moment_cap = 0;
+  // Mixed form (LSMPS_PRECISION_MIXED): per fluid particle the compact FP32
+  // operator rows of the velocity
   // and pressure inverses ([n][36]: Laplacian row, then rows 0, 1, 2), both
   // by visiting position (lsmps_ctx::order), as are the FP64 rows and flags.
-  double* mixed_sums = nullptr;
   float* mixed_rows[2] = {nullptr, nullptr};
   double* mixed_rows64[2] = {nullptr, nullptr};  // rows of matrices factorised in FP64
   uint8_t* mixed_flag[2] = {nullptr, nullptr};   // 1: the particle's rows are in mixed_rows64
@@ -339,6 +380,9 @@ bool ensure_sorted_rows(lsmps_ctx* ctx, size_t entries, size_t nf);
 // Grow the mixed-form arrays to nf fluid particles (outside stream capture).
 bool ensure_mixed(lsmps_ctx* ctx, size_t nf);
 void free_mixed(lsmps_ctx* ctx);
+// Grow the moment stage's sums to nf fluid particles (outside stream capture).
+bool ensure_moment_sums(lsmps_ctx* ctx, size_t nf);
+void free_moment_sums(lsmps_ctx* ctx);
 // Grow / free the operator pair's scratch (adjoint.cu).
 bool ensure_adjoint(lsmps_ctx* ctx, size_t n);
 void free_adjoint(lsmps_ctx* ctx);

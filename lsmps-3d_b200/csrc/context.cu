@@ -27,8 +27,6 @@ bool Scratch::reserve(size_t bytes) {
 }
 
 void free_mixed(lsmps_ctx* ctx) {
-  if (ctx->mixed_sums) cudaFree(ctx->mixed_sums);
-  ctx->mixed_sums = nullptr;
   if (ctx->mixed_count) cudaFree(ctx->mixed_count);
   ctx->mixed_count = nullptr;
   for (int k = 0; k < 2; ++k) {
@@ -51,8 +49,7 @@ bool ensure_mixed(lsmps_ctx* ctx, size_t nf) {
   if (cap != cudaStreamCaptureStatusNone) return false;
   cudaStreamSynchronize(ctx->stream);
   free_mixed(ctx);
-  bool ok = cudaMalloc(&ctx->mixed_sums, nf * 31 * sizeof(double)) == cudaSuccess &&
-            cudaMalloc(&ctx->mixed_count, 4 * sizeof(unsigned int)) == cudaSuccess;
+  bool ok = cudaMalloc(&ctx->mixed_count, 4 * sizeof(unsigned int)) == cudaSuccess;
   for (int k = 0; k < 2 && ok; ++k) {
     ok = cudaMalloc(&ctx->mixed_rows[k], nf * 36 * sizeof(float)) == cudaSuccess &&
          cudaMalloc(&ctx->mixed_rows64[k], nf * 36 * sizeof(double)) == cudaSuccess &&
@@ -66,6 +63,36 @@ bool ensure_mixed(lsmps_ctx* ctx, size_t nf) {
     return false;
   }
   ctx->mixed_cap = nf;
+  return true;
+}
+
+void free_moment_sums(lsmps_ctx* ctx) {
+  if (ctx->moment_sums) cudaFree(ctx->moment_sums);
+  ctx->moment_sums = nullptr;
+  ctx->moment_walled = nullptr;
+  ctx->moment_walls = nullptr;
+  ctx->moment_cap = 0;
+}
+
+bool ensure_moment_sums(lsmps_ctx* ctx, size_t nf) {
+  if (nf <= ctx->moment_cap) return true;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(ctx->stream, &cap);
+  if (cap != cudaStreamCaptureStatusNone) return false;
+  cudaStreamSynchronize(ctx->stream);
+  free_moment_sums(ctx);
+  // one allocation: the sums and both boundaries' wall terms, the list of
+  // particles with walls and its count
+  const size_t doubles = nf * (35 + 31 + 45);
+  if (cudaMalloc(&ctx->moment_sums, doubles * sizeof(double) + (nf + 1) * sizeof(int32_t)) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->moment_sums = nullptr;
+    return false;
+  }
+  ctx->moment_walls = reinterpret_cast<unsigned int*>(ctx->moment_sums + doubles);
+  ctx->moment_walled = reinterpret_cast<int32_t*>(ctx->moment_walls + 1);
+  cudaMemsetAsync(ctx->moment_walls, 0, sizeof(unsigned int), ctx->stream);
+  ctx->moment_cap = nf;
   return true;
 }
 
@@ -258,6 +285,7 @@ void lsmps_ctx_destroy(lsmps_ctx* ctx) {
   if (ctx->fluid_spos) cudaFree(ctx->fluid_spos);
   if (ctx->sorted_labels) cudaFree(ctx->sorted_labels);
   free_mixed(ctx);
+  free_moment_sums(ctx);
   free_adjoint(ctx);
   free_step_ops(ctx);
   if (ctx->d_status) cudaFree(ctx->d_status);
@@ -301,6 +329,8 @@ lsmps_status lsmps_ctx_reserve(lsmps_ctx* ctx, size_t fluid_capacity, size_t wal
   Scratch s(ctx);
   if (!s.reserve(need)) return fail(ctx, LSMPS_CUDA_ERROR, "scratch allocation failed");
   if (!ensure_packs(ctx, fluid_capacity, wall_capacity)) return fail(ctx, LSMPS_CUDA_ERROR, "pack allocation failed");
+  if (!ensure_moment_sums(ctx, fluid_capacity))
+    return fail(ctx, LSMPS_CUDA_ERROR, "moment sums allocation failed");
   if (ctx->precision == LSMPS_PRECISION_MIXED && !ensure_mixed(ctx, fluid_capacity))
     return fail(ctx, LSMPS_CUDA_ERROR, "mixed-form allocation failed");
   return LSMPS_OK;

@@ -4,16 +4,14 @@
 // build_matrix_cache_kernel (:254-309) and the cuSOLVER batched potrf +
 // potrs-per-identity-column inversion (:430-471).
 //
-// One thread owns one particle.  The moment sum is kept in registers as the
-// 45 (Type-A) or 55 (Type-B) entries of the lower triangle, each accumulated
-// as (w * b[r]) * b[c] in CSR row order like add_outer_product (:203-209).
-// The kinds that share the Type-A fluid sum (velocity Dirichlet, pressure
-// Neumann, fluid-only) are built from one pass over the fluid row: the
-// fluid sum is parked in shared memory and each kind adds its own wall term.
-// The inverse is computed in registers by the textbook Cholesky
-// factorisation (Golub & Van Loan, Alg. 4.2.1), the in-place inverse of the
-// triangular factor, and X = L^-T L^-1, then stored column-major and
-// symmetric like the reference's inverse_matrices.
+// Every entry of a moment matrix's fluid sum is one of 31 (Type-A) or 35
+// (Type-B) weighted monomials, the same for all kinds.  Two kernels:
+// plain_sums_kernel adds them up, several lanes to a particle, with the wall
+// terms of the particles that have walls; moment_finish_kernel assembles, regularises and inverts one particle and kind per thread: the
+// textbook Cholesky factorisation (Golub & Van Loan, Alg. 4.2.1) in registers,
+// the in-place inverse of the triangular factor, and X = L^-T L^-1, stored
+// column-major and symmetric like the reference's inverse_matrices.
+#include <algorithm>
 #include <cmath>
 #include <utility>
 
@@ -23,8 +21,6 @@
 
 namespace lsmps {
 namespace {
-
-constexpr int kMomentThreads = 64;
 
 __host__ __device__ constexpr int tri(int r, int c) { return r * (r + 1) / 2 + c; }
 
@@ -36,40 +32,6 @@ struct KindOut {
   int32_t* info;
   int32_t* count;
 };
-
-struct MomentArgs {
-  lsmps_fluid fluid;
-  lsmps_walls walls;
-  const index_t* fo;
-  const index_t* fi;
-  const index_t* wo;
-  const index_t* wi;
-  double re;
-  double inv_re;
-  double lambda;
-  double wall_scale;
-  KindOut k0;  // first kind (boundary given by the kernel's B0)
-  KindOut k1;  // second kind when the kernel's B1 >= 0
-  DeviceStatus* status;
-};
-
-// Type-A (N = 9) or Type-B (N = 10) monomial basis of basis_vector,
-// moment_matrix.cu:152-175.
-template <int N>
-__device__ __forceinline__ void basis(double dx, double dy, double dz, double inv_re, double b[N]) {
-  constexpr int o = N - 9;
-  const double sx = dx * inv_re, sy = dy * inv_re, sz = dz * inv_re;
-  if (o) b[0] = 1.0;
-  b[o + 0] = sx;
-  b[o + 1] = sy;
-  b[o + 2] = sz;
-  b[o + 3] = sx * sx;
-  b[o + 4] = sy * sy;
-  b[o + 5] = sz * sz;
-  b[o + 6] = sx * sy;
-  b[o + 7] = sy * sz;
-  b[o + 8] = sz * sx;
-}
 
 // wall_neumann_vector, moment_matrix.cu:177-201.
 template <int N>
@@ -86,16 +48,6 @@ __device__ __forceinline__ void neumann(double dx, double dy, double dz, double 
   q[o + 6] = (dy * nx + dx * ny) * inv_re;
   q[o + 7] = (dz * ny + dy * nz) * inv_re;
   q[o + 8] = (dx * nz + dz * nx) * inv_re;
-}
-
-template <int N>
-__device__ __forceinline__ void add_outer(double (&m)[N * (N + 1) / 2], const double v[N], double w) {
-#pragma unroll
-  for (int r = 0; r < N; ++r) {
-    const double wr = w * v[r];
-#pragma unroll
-    for (int c = 0; c <= r; ++c) m[tri(r, c)] = fma(wr, v[c], m[tri(r, c)]);
-  }
 }
 
 // Column J of the lower Cholesky factor, in place.  J is a template argument
@@ -152,147 +104,6 @@ __device__ __forceinline__ void invert_lower(double (&a)[N * (N + 1) / 2]) {
       for (int k = j; k < i; ++k) t = fma(a[tri(i, k)], a[tri(k, j)], t);
       a[tri(i, j)] = -t * dinv[i];
     }
-  }
-}
-
-template <int N>
-__device__ __forceinline__ void store_inverse(const double (&t)[N * (N + 1) / 2], double* __restrict__ out) {
-#pragma unroll
-  for (int c = 0; c < N; ++c) {
-#pragma unroll
-    for (int r = c; r < N; ++r) {
-      double x = 0.0;
-#pragma unroll
-      for (int k = r; k < N; ++k) x = fma(t[tri(k, r)], t[tri(k, c)], x);
-      out[r + c * N] = x;
-      if (r != c) out[c + r * N] = x;
-    }
-  }
-}
-
-// The inverse X = L^-T L^-1 from the inverted factor t, written by the
-// warp's active lanes together: in three passes of nine columns' 27 entries
-// each lane stages its particle's entries in shared memory (stage: 27 rows
-// of the warp's 32 lanes, `stride` doubles apart), then the warp writes them
-// particle by particle, 27 consecutive
-// doubles per store instruction, instead of 81 scattered 8-byte stores per
-// lane.  The active lanes are the lowest ones (lanes past the particle count
-// have left).  Same values as store_inverse (the same fused products in the
-// same order); NaN where the factorisation failed (ok = false).
-__device__ __forceinline__ void warp_store_inverse(const double (&t)[45], bool ok, double* out, double* stage,
-                                                   int stride, unsigned active) {
-  const int lane = threadIdx.x & (kWarp - 1);
-  const int nact = __popc(active);
-  const unsigned long long mine = reinterpret_cast<unsigned long long>(out);
-#pragma unroll
-  for (int pass = 0; pass < 3; ++pass) {
-#pragma unroll
-    for (int cc = 0; cc < 3; ++cc) {
-      const int c = 3 * pass + cc;
-#pragma unroll
-      for (int r = 0; r < 9; ++r) {
-        const int lo = r > c ? r : c;
-        double x = 0.0;
-#pragma unroll
-        for (int k = lo; k < 9; ++k) x = fma(t[tri(k, r)], t[tri(k, c)], x);
-        stage[(cc * 9 + r) * stride + lane] = ok ? x : __longlong_as_double(0x7ff8000000000000LL);
-      }
-    }
-    __syncwarp(active);
-    for (unsigned rem = active; rem; rem &= rem - 1) {
-      const int p = __ffs(rem) - 1;
-      double* op = reinterpret_cast<double*>(__shfl_sync(active, mine, p));
-      for (int e = lane; e < 27; e += nact) op[27 * pass + e] = stage[e * stride + p];
-    }
-    __syncwarp(active);
-  }
-}
-
-// Adds the wall term of boundary kind B (0 none, 1 Dirichlet sample,
-// 2 pressure Neumann) to m, regularises, inverts and stores one kind (with
-// stage, by the warp's active lanes together: warp_store_inverse).
-template <int N, int B>
-__device__ __forceinline__ void finish_kind(double (&m)[N * (N + 1) / 2], const MomentArgs& a, const KindOut& ko,
-                                            index_t i, double xi, double yi, double zi) {
-  double b[N];
-  if (B != 0) {
-    const index_t we = a.wo[i + 1];
-    for (index_t o = a.wo[i]; o < we; ++o) {
-      const index_t j = a.wi[o];
-      const double dx = a.walls.x[j] - xi, dy = a.walls.y[j] - yi, dz = a.walls.z[j] - zi;
-      const double d2 = dx * dx + dy * dy + dz * dz;
-      if (d2 <= 0.0) continue;
-      const double w = a.wall_scale * (1.0 - sqrt(d2) * a.inv_re);
-      if (w <= 0.0) continue;
-      if (B == 2) {
-        neumann<N>(dx, dy, dz, a.walls.normal_x[j], a.walls.normal_y[j], a.walls.normal_z[j], a.inv_re, b);
-      } else {
-        basis<N>(dx, dy, dz, a.inv_re, b);
-      }
-      add_outer<N>(m, b, w);
-    }
-  }
-  // trace and regularisation, moment_matrix.cu:297-308
-  double trace = 0.0;
-#pragma unroll
-  for (int r = 0; r < N; ++r) trace += m[tri(r, r)];
-  const double reg = a.lambda * (trace > 0.0 ? trace / static_cast<double>(N) : 1.0);
-#pragma unroll
-  for (int r = 0; r < N; ++r) m[tri(r, r)] += reg;
-  const int info = cholesky<N>(m);
-  double* out = ko.inverse + static_cast<size_t>(i) * N * N;
-  if (info == 0) {
-    invert_lower<N>(m);
-    store_inverse<N>(m, out);
-  } else {
-    for (int e = 0; e < N * N; ++e) out[e] = __longlong_as_double(0x7ff8000000000000LL);
-    atomicAdd(&a.status->non_spd, 1u);
-    raise_flag(a.status, kFlagNonSpd);
-  }
-  ko.trace[i] = trace;
-  ko.reg[i] = reg;
-  ko.info[i] = info;
-}
-
-// One or two kinds (B1 < 0: one) from one pass over the fluid row.
-template <int N, int B0, int B1>
-__global__ void __launch_bounds__(kMomentThreads) moment_kernel(MomentArgs a) {
-  constexpr int E = N * (N + 1) / 2;
-  extern __shared__ double s_fluid[];  // [E][kMomentThreads] when two kinds share the fluid sum
-  const index_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    if (a.k0.count) atomicAdd(a.k0.count, 1);
-    if (B1 >= 0 && a.k1.count) atomicAdd(a.k1.count, 1);
-  }
-  if (i >= static_cast<index_t>(a.fluid.count)) return;
-  const double* __restrict__ fx = a.fluid.x;
-  const double* __restrict__ fy = a.fluid.y;
-  const double* __restrict__ fz = a.fluid.z;
-  const double xi = fx[i], yi = fy[i], zi = fz[i];
-  double m[E];
-#pragma unroll
-  for (int e = 0; e < E; ++e) m[e] = 0.0;
-  double b[N];
-  const index_t fe = a.fo[i + 1];
-  for (index_t o = a.fo[i]; o < fe; ++o) {
-    const index_t j = a.fi[o];
-    const double dx = fx[j] - xi, dy = fy[j] - yi, dz = fz[j] - zi;
-    const double d2 = dx * dx + dy * dy + dz * dz;
-    if (d2 <= 0.0) continue;
-    const double w = 1.0 - sqrt(d2) * a.inv_re;
-    if (w <= 0.0) continue;
-    basis<N>(dx, dy, dz, a.inv_re, b);
-    add_outer<N>(m, b, w);
-  }
-  if (B1 >= 0) {
-#pragma unroll
-    for (int e = 0; e < E; ++e) s_fluid[e * kMomentThreads + threadIdx.x] = m[e];
-  }
-  finish_kind<N, B0>(m, a, a.k0, i, xi, yi, zi);
-  if (B1 >= 0) {
-#pragma unroll
-    for (int e = 0; e < E; ++e) m[e] = s_fluid[e * kMomentThreads + threadIdx.x];
-    finish_kind<N, (B1 < 0 ? 0 : B1)>(m, a, a.k1, i, xi, yi, zi);
   }
 }
 
@@ -365,8 +176,8 @@ __host__ __device__ constexpr int entry_slot(int r, int c) {
                        basis_exponent(r, 2) + basis_exponent(c, 2));
 }
 
-template <typename T>
-__device__ __forceinline__ void acc_monomials(T (&s)[kMonomials], T sx, T sy, T sz, T w) {
+template <typename T, int S>
+__device__ __forceinline__ void acc_monomials(T (&s)[S], T sx, T sy, T sz, T w) {
   const T qxx = sx * sx, qyy = sy * sy, qzz = sz * sz;
   const T qxy = sx * sy, qyz = sy * sz, qzx = sz * sx;
   const T wxx = w * qxx, wyy = w * qyy, wzz = w * qzz, wxy = w * qxy;
@@ -403,206 +214,369 @@ __device__ __forceinline__ void acc_monomials(T (&s)[kMonomials], T sx, T sy, T 
   s[30] = fma(wzz, qxy, s[30]);
 }
 
-struct MomentPackedArgs {
+// ---------------------------------------------------------------------------
+// Plain form.
+// ---------------------------------------------------------------------------
+constexpr int kMonomialsB = kMonomials + 4;  // Type-B: also the sums of w, w sx, w sy, w sz
+constexpr int kWallEntries = 45;             // lower triangle of sum w q q^T
+constexpr int kSumThreads = 128;
+constexpr int kWallThreads = kWarp;
+constexpr int kFinishThreads = kWarp;
+
+// The sum slot of entry (r, c) of an N x N matrix's fluid part.
+template <int N>
+__host__ __device__ constexpr int fluid_slot(int r, int c) {
+  if (N == 9) return entry_slot(r, c);
+  if (c == 0) {
+    return r == 0 ? kMonomials
+         : r <= 3 ? kMonomials + r
+                  : monomial_slot(basis_exponent(r - 1, 0), basis_exponent(r - 1, 1), basis_exponent(r - 1, 2));
+  }
+  return entry_slot(r - 1, c - 1);
+}
+
+struct SumArgs {
   index_t n;
-  const double4* fp;  // {x, y, z, -} fluid
-  const double4* wp;  // {x, y, z, -} walls
-  const double4* wn;  // {nx, ny, nz, -} walls
+  const double4* fp;
   const index_t* fo;
   const index_t* fi;
-  const index_t* wo;
-  const index_t* wi;
   double inv_re;
-  double lambda;
-  double wall_scale;
-  KindOut k0;
-  KindOut k1;
-  DeviceStatus* status;
+  double* sums;          // [kMonomials or kMonomialsB][n], by visiting position
   const int32_t* order;  // visiting order (lsmps_ctx::order) or NULL
   int sorted;            // fi and fp in cell-sorted positions (sorted_rows_of)
 };
 
-template <int B>
-__device__ __forceinline__ void finish_a(double (&s)[kMonomials], const MomentPackedArgs& a, const KindOut& ko,
-                                         index_t i, const double4& pi, double* stage = nullptr,
-                                         int stride = kWarp, unsigned active = 0u) {
-  const index_t wb = a.wo[i], we = a.wo[i + 1];
-  // The wall loops load the next wall's record(s) while this one is used,
-  // with the index one further ahead.
-  if (B == 1 && wb < we) {
-    double4 qn = ld4(a.wp, a.wi[wb]);
-    index_t jnn = wb + 1 < we ? a.wi[wb + 1] : 0;
-    for (index_t o = wb; o < we; ++o) {
+// The squared length of an offset in one fixed order of roundings: the sums'
+// last bits decide those of an ill-conditioned matrix's inverse (condition
+// number 1e9: the seventh digit), so they are not left to the compiler's choice
+// of products to fuse.
+__device__ __forceinline__ double length2(double dx, double dy, double dz) {
+  return fma(dz, dz, fma(dy, dy, dx * dx));
+}
+
+// ... and the one of the Neumann terms.
+__device__ __forceinline__ double length2_wall(double dx, double dy, double dz) {
+  return fma(dz, dz, fma(dx, dx, dy * dy));
+}
+
+// r_e-scaled offset and weight of one neighbour; all 0 where it has none.
+struct Scaled {
+  double x, y, z, w;
+};
+
+__device__ __forceinline__ Scaled scaled(const double4& q, const double4& pi, double inv_re) {
+  const double dx = q.x - pi.x, dy = q.y - pi.y, dz = q.z - pi.z;
+  const double d2 = length2(dx, dy, dz);
+  const double w = fma(-sqrt(d2), inv_re, 1.0);
+  if (d2 <= 0.0 || w <= 0.0) return Scaled{0.0, 0.0, 0.0, 0.0};
+  return Scaled{dx * inv_re, dy * inv_re, dz * inv_re, w};
+}
+
+// Lists the particle (visiting position t) when it has walls, for
+// wall_sums_kernel: walled[0 .. *walls), in no particular order.
+__device__ __forceinline__ void list_walled(bool mine, index_t t, index_t n, int32_t* walled, unsigned* walls) {
+  const int lane = threadIdx.x & (kWarp - 1);
+  const unsigned with = __ballot_sync(0xffffffffu, mine);
+  if (!with) return;
+  unsigned at = 0;
+  if (lane == 0) at = atomicAdd(walls, __popc(with));
+  at = __shfl_sync(0xffffffffu, at, 0) + __popc(with & ((1u << lane) - 1u));
+  if (mine && at < static_cast<unsigned>(n)) walled[at] = t;
+}
+
+// The fluid sums, G lanes to a particle: with two, one takes the even entries
+// and one the odd, then the two halves are added (LSMPS_KNOB_MOMENT_OCCUPANCY 2).
+// While one entry is accumulated, the next one's offset and weight are formed (a
+// chain of dependent FP64 operations through the square root) and the record
+// after it is loaded.  500,000 particles (54 M entries), B200: 0.38 ms with one
+// lane, 0.39 with two, FP64 pipe 56%, L1 wavefronts 47% (0.48 ms and 168
+// registers with the weight formed when its turn comes); 1,000 particles: 32 and
+// 21 us.  Tried for sets that do not fill the GPU: three lanes a particle, each
+// with a third of the monomials (the same additions): 27 us at 1,000 particles,
+// but 135 against 112 at 31,713.
+template <int G, bool TypeB>
+__global__ void __launch_bounds__(kSumThreads, 4) plain_sums_kernel(SumArgs a, const index_t* __restrict__ wo,
+                                                                    int32_t* __restrict__ walled,
+                                                                    unsigned* __restrict__ walls) {
+  constexpr int S = TypeB ? kMonomialsB : kMonomials;
+  const index_t t = static_cast<index_t>((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / G);
+  const int l = threadIdx.x & (G - 1);
+  const bool live = t < a.n;
+  const index_t i = live ? visit(a.order, t) : 0;
+  if (wo) list_walled(live && l == 0 && wo[i] < wo[i + 1], t, a.n, walled, walls);
+  double s[S];
+#pragma unroll
+  for (int e = 0; e < S; ++e) s[e] = 0.0;
+  if (live) {
+    // past the row's end a lane takes its own record, whose weight is 0
+    const index_t self = self_of(a.sorted, t, i);
+    const double4 pi = ld4(a.fp, self);
+    const index_t fe = a.fo[i + 1];
+    index_t o = a.fo[i] + l;
+    const index_t j0 = o < fe ? a.fi[o] : self, j1 = o + G < fe ? a.fi[o + G] : self;
+    index_t j2 = o + 2 * G < fe ? a.fi[o + 2 * G] : self;
+    double4 qn = ld4(a.fp, j1);
+    Scaled v = scaled(ld4(a.fp, j0), pi, a.inv_re);
+#pragma unroll 1
+    for (; o < fe; o += G) {
       const double4 q = qn;
-      if (o + 1 < we) {
-        qn = ld4(a.wp, jnn);
-        if (o + 2 < we) jnn = a.wi[o + 2];
+      qn = ld4(a.fp, j2);
+      if (o + 3 * G < fe) j2 = a.fi[o + 3 * G];
+      const Scaled next = scaled(q, pi, a.inv_re);
+      acc_monomials(s, v.x, v.y, v.z, v.w);
+      if (TypeB) {
+        s[kMonomials] += v.w;
+        s[kMonomials + 1] = fma(v.w, v.x, s[kMonomials + 1]);
+        s[kMonomials + 2] = fma(v.w, v.y, s[kMonomials + 2]);
+        s[kMonomials + 3] = fma(v.w, v.z, s[kMonomials + 3]);
       }
-      const double dx = q.x - pi.x, dy = q.y - pi.y, dz = q.z - pi.z;
-      const double d2 = dx * dx + dy * dy + dz * dz;
-      if (d2 <= 0.0) continue;
-      const double w = a.wall_scale * (1.0 - sqrt(d2) * a.inv_re);
-      if (w <= 0.0) continue;
-      acc_monomials(s, dx * a.inv_re, dy * a.inv_re, dz * a.inv_re, w);
+      v = next;
     }
   }
-  double m[45];
+  int base = 0, count = S;
+  lane_totals<S, G / 2>(s, base, count);
+  if (!live) return;
 #pragma unroll
-  for (int r = 0; r < 9; ++r) {
+  for (int k = 0; k < lane_totals_left(S, G / 2); ++k)
+    if (k < count) a.sums[static_cast<size_t>(base + k) * a.n + t] = s[k];
+}
+
+struct WallArgs {
+  index_t n;
+  const double4* fp;
+  const double4* wp;
+  const double4* wn;
+  const index_t* wo;
+  const index_t* wi;
+  double inv_re;
+  double wall_scale;
+  const double* sums;
+  double* velocity;  // [kMonomials][n] by visiting position, of the particles with walls
+  double* pressure;  // [kWallEntries][n]
+  const int32_t* order;
+  int sorted;
+  const int32_t* walled;
+  const unsigned* walls;
+};
+
+// The listed particles' sums with their wall terms, in row order, one thread to
+// a particle: the monomials with the Dirichlet samples, or the lower triangle of
+// the matrix with w q q^T.  A particle near a wall has 30 to 100 of them; walked
+// by the threads that invert the matrices, they set the pace of warps whose other
+// particles have none.  500,000 particles, 90,000 of them with walls: 0.12 ms
+// for both kinds; eight lanes a particle, which add in another order, take as
+// long, and looking for walls from every particle's lanes 0.27.
+template <bool Neumann>
+__device__ __forceinline__ void wall_sums(const WallArgs& a) {
+  const index_t many = static_cast<index_t>(*a.walls);
+  const size_t n = static_cast<size_t>(a.n);
+  for (index_t g = blockIdx.x * blockDim.x + threadIdx.x; g < many; g += gridDim.x * blockDim.x) {
+    const index_t t = a.walled[g];
+    const index_t i = visit(a.order, t);
+    const double4 pi = ld4(a.fp, self_of(a.sorted, t, i));
+    const index_t we = a.wo[i + 1];
+    index_t o = a.wo[i];
+    // As in plain_sums_kernel: the next wall's weight is formed while this one
+    // is accumulated, and the record after it loaded (past the row's end, the
+    // row's last wall again).
+    index_t j0 = a.wi[o], j1 = o + 1 < we ? a.wi[o + 1] : j0, j2 = o + 2 < we ? a.wi[o + 2] : j1;
+    double s[kMonomials];
 #pragma unroll
-    for (int c = 0; c <= r; ++c) m[tri(r, c)] = s[entry_slot(r, c)];
-  }
-  if (B == 2 && wb < we) {
-    double q9[9];
-    index_t jn = a.wi[wb];
-    index_t jnn = wb + 1 < we ? a.wi[wb + 1] : 0;
-    double4 qn = ld4(a.wp, jn), nn = ld4(a.wn, jn);
-    for (index_t o = wb; o < we; ++o) {
-      const double4 q = qn, nrm = nn;
-      if (o + 1 < we) {
-        jn = jnn;
-        qn = ld4(a.wp, jn);
-        nn = ld4(a.wn, jn);
-        if (o + 2 < we) jnn = a.wi[o + 2];
+    for (int e = 0; e < kMonomials; ++e) s[e] = a.sums[e * n + t];
+    if constexpr (!Neumann) {
+      double4 qn = ld4(a.wp, j1);
+      Scaled v = scaled(ld4(a.wp, j0), pi, a.inv_re);
+#pragma unroll 1
+      for (; o < we; ++o) {
+        const double4 q = qn;
+        qn = ld4(a.wp, j2);
+        if (o + 3 < we) j2 = a.wi[o + 3];
+        const Scaled next = scaled(q, pi, a.inv_re);
+        const double w = a.wall_scale * v.w;
+        if (w > 0.0) acc_monomials(s, v.x, v.y, v.z, w);
+        v = next;
       }
-      const double dx = q.x - pi.x, dy = q.y - pi.y, dz = q.z - pi.z;
-      const double d2 = dx * dx + dy * dy + dz * dz;
-      if (d2 <= 0.0) continue;
-      const double w = a.wall_scale * (1.0 - sqrt(d2) * a.inv_re);
-      if (w <= 0.0) continue;
-      neumann<9>(dx, dy, dz, nrm.x, nrm.y, nrm.z, a.inv_re, q9);
-      add_outer<9>(m, q9, w);
+#pragma unroll
+      for (int e = 0; e < kMonomials; ++e) a.velocity[e * n + t] = s[e];
+    } else {
+      double m[kWallEntries];
+#pragma unroll
+      for (int r = 0; r < 9; ++r) {
+#pragma unroll
+        for (int c = 0; c <= r; ++c) m[tri(r, c)] = s[entry_slot(r, c)];
+      }
+      double4 qn = ld4(a.wp, j0), nn = ld4(a.wn, j0);
+#pragma unroll 1
+      for (; o < we; ++o) {
+        const double4 q = qn, nrm = nn;
+        qn = ld4(a.wp, j1);
+        nn = ld4(a.wn, j1);
+        j1 = j2;
+        if (o + 3 < we) j2 = a.wi[o + 3];
+        const double dx = q.x - pi.x, dy = q.y - pi.y, dz = q.z - pi.z;
+        const double d2 = length2_wall(dx, dy, dz);
+        const double w = a.wall_scale * fma(-sqrt(d2), a.inv_re, 1.0);
+        if (d2 <= 0.0 || w <= 0.0) continue;
+        // neumann<9> with its roundings fixed
+        const double ir = a.inv_re;
+        const double q9[9] = {nrm.x, nrm.y, nrm.z, 2.0 * dx * nrm.x * ir, 2.0 * dy * nrm.y * ir, 2.0 * dz * nrm.z * ir,
+                              fma(dx, nrm.y, dy * nrm.x) * ir, fma(dy, nrm.z, dz * nrm.y) * ir, fma(dz, nrm.x, dx * nrm.z) * ir};
+#pragma unroll
+        for (int r = 0; r < 9; ++r) {
+          const double wr = w * q9[r];
+#pragma unroll
+          for (int c = 0; c <= r; ++c) m[tri(r, c)] = fma(wr, q9[c], m[tri(r, c)]);
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < kWallEntries; ++e) a.pressure[e * n + t] = m[e];
+    }
+  }
+}
+
+// blockIdx.y + first: 0 the Dirichlet samples, 1 the Neumann terms
+__global__ void __launch_bounds__(kWallThreads) wall_sums_kernel(WallArgs a, int first) {
+  if (blockIdx.y + first == 0)
+    wall_sums<false>(a);
+  else
+    wall_sums<true>(a);
+}
+
+struct FinishArgs {
+  index_t n;
+  const double* sums;
+  const double* velocity;
+  const double* pressure;
+  const index_t* wo;
+  double lambda;
+  KindOut k[3];
+  DeviceStatus* status;
+  const int32_t* order;
+  unsigned* walls;  // emptied for the next call's list
+};
+
+// X = L^-T L^-1 in place of the inverted factor (lower triangles): row r of X
+// needs rows >= r of the factor, and of row r itself each entry and, last, the
+// diagonal.
+template <int N>
+__device__ __forceinline__ void square_lower(double (&t)[N * (N + 1) / 2]) {
+#pragma unroll
+  for (int r = 0; r < N; ++r) {
+#pragma unroll
+    for (int c = 0; c <= r; ++c) {
+      double x = 0.0;
+#pragma unroll
+      for (int k = r; k < N; ++k) x = fma(t[tri(k, r)], t[tri(k, c)], x);
+      t[tri(r, c)] = x;
+    }
+  }
+}
+
+// The symmetric matrix x (lower triangle) of each active lane's particle i to
+// out + N^2 i, by the warp together: a few columns at a time, each lane stages
+// its entries in shared memory, then the warp writes them particle by particle,
+// consecutive doubles per store instruction, instead of N^2 scattered 8-byte
+// stores per lane.  The stage's rows are 33 doubles apart: at 32, all lanes of
+// the read-back meet in one bank.  The active lanes are the lowest ones (lanes
+// past the particle count have left).
+template <int N>
+__device__ __forceinline__ void warp_store_symmetric(const double (&x)[N * (N + 1) / 2], double* __restrict__ out,
+                                                     index_t i, double (*stage)[kWarp + 1], unsigned active) {
+  constexpr int C = N == 9 ? 3 : 2;  // columns a pass
+  static_assert(N % C == 0 && C * N <= kWarp, "whole passes of one store instruction a particle");
+  const int lane = threadIdx.x & (kWarp - 1);
+  const int many = __popc(active);
+#pragma unroll
+  for (int pass = 0; pass < N / C; ++pass) {
+#pragma unroll
+    for (int cc = 0; cc < C; ++cc) {
+      const int c = C * pass + cc;
+#pragma unroll
+      for (int r = 0; r < N; ++r) stage[cc * N + r][lane] = x[r > c ? tri(r, c) : tri(c, r)];
+    }
+    __syncwarp(active);
+    double* base = out + C * N * pass;
+    if (many == kWarp) {
+#pragma unroll 8
+      for (int p = 0; p < kWarp; ++p) {
+        const size_t at = static_cast<size_t>(__shfl_sync(0xffffffffu, i, p)) * (N * N);
+        if (lane < C * N) base[at + lane] = stage[lane][p];
+      }
+    } else {
+      for (int p = 0; p < many; ++p) {
+        const size_t at = static_cast<size_t>(__shfl_sync(active, i, p)) * (N * N);
+        for (int e = lane; e < C * N; e += many) base[at + e] = stage[e][p];
+      }
+    }
+    __syncwarp(active);
+  }
+}
+
+// One thread per particle and kind (blockIdx.y): the matrix from the fluid
+// sums and the particle's wall terms, trace and regularisation
+// (moment_matrix.cu:286-308), inverse.  One warp a block, so that a small set
+// spreads over the SMs.  500,000 particles, two kinds: 0.20 ms, of which the
+// 648-byte inverses take 0.10 at the copy rate (0.255 with every entry of X formed
+// twice and a pointer exchanged per store).  Sums, walls and this kernel together
+// take 0.71 ms where one kernel with two warps to 32 particles took 0.90, and
+// 75 us where it took 185 at 1,000 particles, with the same bits.
+template <int N>
+__global__ void __launch_bounds__(kFinishThreads, N == 9 ? 16 : 10) moment_finish_kernel(FinishArgs a) {
+  constexpr int o = N - 9;
+  __shared__ double s_stage[27][kWarp + 1];
+  const KindOut& ko = a.k[blockIdx.y];
+  const index_t t = blockIdx.x * kFinishThreads + threadIdx.x;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (ko.count) atomicAdd(ko.count, 1);
+    if (blockIdx.y == 0) *a.walls = 0u;
+  }
+  const unsigned active = __ballot_sync(0xffffffffu, t < a.n);
+  if (t >= a.n) return;
+  const index_t i = visit(a.order, t);
+  const size_t n = static_cast<size_t>(a.n);
+  const bool walls = ko.boundary != 0 && a.wo[i] < a.wo[i + 1];
+  double m[N * (N + 1) / 2];
+  if (N == 9 && walls && ko.boundary == 2) {
+#pragma unroll
+    for (int e = 0; e < 45; ++e) m[e] = a.pressure[e * n + t];
+  } else {
+    double s[N == 9 ? kMonomials : kMonomialsB];
+    const double* __restrict__ from = N == 9 && walls && ko.boundary == 1 ? a.velocity : a.sums;
+#pragma unroll
+    for (int e = 0; e < (N == 9 ? kMonomials : kMonomialsB); ++e) s[e] = from[e * n + t];
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+#pragma unroll
+      for (int c = 0; c <= r; ++c) m[tri(r, c)] = s[fluid_slot<N>(r, c)];
+    }
+    if (N == 10 && walls) {  // Type-B's q has no constant part: the 9 x 9 matrix
+#pragma unroll
+      for (int r = 0; r < 9; ++r) {
+#pragma unroll
+        for (int c = 0; c <= r; ++c) m[tri(r + o, c + o)] = a.pressure[tri(r, c) * n + t];
+      }
     }
   }
   double trace = 0.0;
 #pragma unroll
-  for (int r = 0; r < 9; ++r) trace += m[tri(r, r)];
-  const double reg = a.lambda * (trace > 0.0 ? trace / 9.0 : 1.0);
+  for (int r = 0; r < N; ++r) trace += m[tri(r, r)];
+  const double reg = a.lambda * (trace > 0.0 ? trace / static_cast<double>(N) : 1.0);
 #pragma unroll
-  for (int r = 0; r < 9; ++r) m[tri(r, r)] += reg;
-  const int info = cholesky<9>(m);
-  double* out = ko.inverse + static_cast<size_t>(i) * 81;
-  if (info == 0) invert_lower<9>(m);
-  if (stage) {
-    warp_store_inverse(m, info == 0, out, stage, stride, active);
-  } else if (info == 0) {
-    store_inverse<9>(m, out);
+  for (int r = 0; r < N; ++r) m[tri(r, r)] += reg;
+  const int info = cholesky<N>(m);
+  if (info == 0) {
+    invert_lower<N>(m);
+    square_lower<N>(m);
   } else {
-    for (int e = 0; e < 81; ++e) out[e] = __longlong_as_double(0x7ff8000000000000LL);
-  }
-  if (info != 0) {
+#pragma unroll
+    for (int e = 0; e < N * (N + 1) / 2; ++e) m[e] = __longlong_as_double(0x7ff8000000000000LL);
     atomicAdd(&a.status->non_spd, 1u);
     raise_flag(a.status, kFlagNonSpd);
   }
+  warp_store_symmetric<N>(m, ko.inverse, i, s_stage, active);
   ko.trace[i] = trace;
   ko.reg[i] = reg;
   ko.info[i] = info;
-}
-
-// Type-A kinds B0 (and B1 >= 0) from one pass over the fluid row.  MinBlocks
-// is the register budget variant (LSMPS_KNOB_MOMENT_OCCUPANCY).
-// The last kind's inverses are written through shared memory by the warp
-// (warp_store_inverse; the first of two kinds with scalar stores, its
-// shared memory still holding the second kind's sums).
-template <int B0, int B1, int MinBlocks>
-__global__ void __launch_bounds__(kMomentThreads, MinBlocks) moment_a_kernel(MomentPackedArgs a) {
-  // [kMonomials][kMomentThreads] when B1 >= 0, else [27][kMomentThreads]
-  extern __shared__ double s_mono[];
-  const index_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    if (a.k0.count) atomicAdd(a.k0.count, 1);
-    if (B1 >= 0 && a.k1.count) atomicAdd(a.k1.count, 1);
-  }
-  const unsigned active = __ballot_sync(0xffffffffu, t < a.n);
-  if (t >= a.n) return;
-  double* stage = s_mono + (threadIdx.x & ~(kWarp - 1));
-  const index_t i = visit(a.order, t);
-  const double4 pi = ld4(a.fp, self_of(a.sorted, t, i));
-  double s[kMonomials];
-#pragma unroll
-  for (int e = 0; e < kMonomials; ++e) s[e] = 0.0;
-  // The next neighbour's record is loaded while this one is accumulated.
-  const index_t fe = a.fo[i + 1];
-  index_t o = a.fo[i];
-  double4 qn = o < fe ? ld4(a.fp, a.fi[o]) : pi;
-  for (; o < fe; ++o) {
-    const double4 q = qn;
-    if (o + 1 < fe) qn = ld4(a.fp, a.fi[o + 1]);
-    const double dx = q.x - pi.x, dy = q.y - pi.y, dz = q.z - pi.z;
-    const double d2 = dx * dx + dy * dy + dz * dz;
-    if (d2 <= 0.0) continue;
-    const double w = 1.0 - sqrt(d2) * a.inv_re;
-    if (w <= 0.0) continue;
-    acc_monomials(s, dx * a.inv_re, dy * a.inv_re, dz * a.inv_re, w);
-  }
-  if (B1 >= 0) {
-#pragma unroll
-    for (int e = 0; e < kMonomials; ++e) s_mono[e * kMomentThreads + threadIdx.x] = s[e];
-  }
-  if (B1 < 0) {
-    finish_a<B0>(s, a, a.k0, i, pi, stage, kMomentThreads, active);
-    return;
-  }
-  finish_a<B0>(s, a, a.k0, i, pi);
-#pragma unroll
-  for (int e = 0; e < kMonomials; ++e) s[e] = s_mono[e * kMomentThreads + threadIdx.x];
-  finish_a<(B1 < 0 ? 0 : B1)>(s, a, a.k1, i, pi, stage, kMomentThreads, active);
-}
-
-// The velocity and pressure kinds with the two warps of a 64-thread block
-// sharing 32 particles: warp h sums the even (h = 0) or odd (h = 1) entries of
-// each row, the halves are exchanged through shared memory, then warp 0
-// finishes the velocity kind and warp 1 the pressure kind, so neither the
-// row sum nor the two factorisations run twice in one thread and no warp
-// diverges between the kinds (LSMPS_KNOB_MOMENT_OCCUPANCY variant 2).
-__global__ void __launch_bounds__(2 * kWarp, 8) moment_a_split_kernel(MomentPackedArgs a) {
-  __shared__ double s_half[2][kMonomials][kWarp];
-  const int lane = threadIdx.x & (kWarp - 1), half = threadIdx.x >> 5;
-  const index_t t = blockIdx.x * kWarp + lane;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    if (a.k0.count) atomicAdd(a.k0.count, 1);
-    if (a.k1.count) atomicAdd(a.k1.count, 1);
-  }
-  const bool live = t < a.n;
-  const index_t i = live ? visit(a.order, t) : 0;
-  const double4 pi = live ? ld4(a.fp, self_of(a.sorted, t, i)) : make_double4(0.0, 0.0, 0.0, 0.0);
-  double s[kMonomials];
-#pragma unroll
-  for (int e = 0; e < kMonomials; ++e) s[e] = 0.0;
-  if (live) {
-    const index_t fe = a.fo[i + 1];
-    index_t o = a.fo[i] + half;
-    double4 qn = o < fe ? ld4(a.fp, a.fi[o]) : pi;
-    index_t jnn = o + 2 < fe ? a.fi[o + 2] : i;  // the index after the next
-    for (; o < fe; o += 2) {
-      const double4 q = qn;
-      if (o + 2 < fe) {
-        qn = ld4(a.fp, jnn);
-        if (o + 4 < fe) jnn = a.fi[o + 4];
-      }
-      const double dx = q.x - pi.x, dy = q.y - pi.y, dz = q.z - pi.z;
-      const double d2 = dx * dx + dy * dy + dz * dz;
-      if (d2 <= 0.0) continue;
-      const double w = 1.0 - sqrt(d2) * a.inv_re;
-      if (w <= 0.0) continue;
-      acc_monomials(s, dx * a.inv_re, dy * a.inv_re, dz * a.inv_re, w);
-    }
-  }
-#pragma unroll
-  for (int e = 0; e < kMonomials; ++e) s_half[half][e][lane] = s[e];
-  __syncthreads();
-#pragma unroll
-  for (int e = 0; e < kMonomials; ++e) s[e] = s_half[0][e][lane] + s_half[1][e][lane];
-  // each warp then stages its kind's inverses in its half of s_half
-  __syncthreads();
-  const unsigned active = __ballot_sync(0xffffffffu, live);
-  if (!live) return;
-  double* stage = &s_half[half][0][0];
-  static_assert(kMonomials >= 27, "the stage holds 27 x 32 doubles");
-  if (half == 0)
-    finish_a<1>(s, a, a.k0, i, pi, stage, kWarp, active);
-  else
-    finish_a<2>(s, a, a.k1, i, pi, stage, kWarp, active);
 }
 
 // ---------------------------------------------------------------------------
@@ -614,7 +588,7 @@ __global__ void __launch_bounds__(2 * kWarp, 8) moment_a_split_kernel(MomentPack
 // and each is added into its sum with Kahan's compensated summation (an FP32
 // sum and an FP32 running compensation), so the summation adds no error
 // beyond O(n u^2) to the rounding of the terms themselves.  The totals
-// (sum minus compensation, in FP64) go to the context's mixed_sums array,
+// (sum minus compensation, in FP64) go to the context's moment_sums array,
 // monomial-major.
 //
 // Stage 2 (moment_rows_kernel, one thread per particle and kind): the kind's
@@ -632,19 +606,7 @@ __global__ void __launch_bounds__(2 * kWarp, 8) moment_a_split_kernel(MomentPack
 // With Full, all nine columns are solved and the full FP64 inverse is
 // written to the moment view (lsmps_prepare_moments in the mixed form).
 
-constexpr int kSumThreads = 128;
 constexpr int kRowThreads = 64;
-
-struct MixedSumArgs {
-  index_t n;
-  const double4* fp;
-  const index_t* fo;
-  const index_t* fi;
-  double inv_re;
-  double* sums;          // [kMonomials][n], by visiting position
-  const int32_t* order;  // visiting order (lsmps_ctx::order) or NULL
-  int sorted;            // fi and fp in cell-sorted positions (sorted_rows_of)
-};
 
 // Kahan step for the 31 weighted monomials of one neighbour (the same
 // products as acc_monomials).
@@ -706,7 +668,7 @@ __device__ __forceinline__ void monomial_pairs(f32x2 (&t)[16], float sx, float s
   t[15] = pack2(wzz * low_half(q1), 0.0f);                // wzz qxx
 }
 
-__global__ void __launch_bounds__(kSumThreads) moment_sums_kernel(MixedSumArgs a) {
+__global__ void __launch_bounds__(kSumThreads) moment_sums_kernel(SumArgs a) {
   const index_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= a.n) return;
   const index_t i = visit(a.order, t);
@@ -1182,7 +1144,7 @@ __global__ void __launch_bounds__(kRowThreads, 6) moment_rows_kernel(MixedRowArg
 // rows (Kahan-compensated FP32), the halves meet in shared memory as FP64
 // totals, then warp 0 finishes the velocity kind and warp 1 the pressure kind.
 template <bool Full>
-__global__ void __launch_bounds__(kRowThreads, 6) moment_mixed_split_kernel(MixedSumArgs sa, MixedRowArgs a) {
+__global__ void __launch_bounds__(kRowThreads, 6) moment_mixed_split_kernel(SumArgs sa, MixedRowArgs a) {
   static_assert(kRowThreads == 2 * kWarp, "two warps per block");
   __shared__ double s_m[45 * kRowThreads];
   __shared__ double s_half[2][kMonomials][kWarp];
@@ -1225,6 +1187,20 @@ __global__ void __launch_bounds__(kRowThreads, 6) moment_mixed_split_kernel(Mixe
   mixed_rows_of_particle<Full>(a, half, t, i, pi, s, s_m + threadIdx.x);
 }
 
+void launch_plain_sums(lsmps_ctx* ctx, const SumArgs& a, const index_t* wo, bool type_b) {
+  const bool halves = ctx->knob[LSMPS_KNOB_MOMENT_OCCUPANCY] == 2;
+  const auto queue = [&](const char* name, auto kernel) {
+    launch_named(ctx, name, kernel, dim3(div_up((halves ? 2LL : 1LL) * a.n, kSumThreads)), dim3(kSumThreads), 0, a, wo,
+                 ctx->moment_walled, ctx->moment_walls);
+  };
+  if (halves)
+    type_b ? queue("plain_sums_kernel<2, B>", plain_sums_kernel<2, true>)
+           : queue("plain_sums_kernel<2>", plain_sums_kernel<2, false>);
+  else
+    type_b ? queue("plain_sums_kernel<1, B>", plain_sums_kernel<1, true>)
+           : queue("plain_sums_kernel<1>", plain_sums_kernel<1, false>);
+}
+
 // make_matrix_request, moment_matrix.cu:494-538: boundary of each kind.
 int boundary_of(int kind) {
   switch (kind) {
@@ -1244,15 +1220,15 @@ int boundary_of(int kind) {
 lsmps_status launch_mixed(lsmps_ctx* ctx, index_t n, const lsmps_csr& fn, const lsmps_csr& wn,
                           const lsmps_params& p, const KindOut& kv, const KindOut& kp, bool full,
                           const lsmps_walls& walls) {
-  if (!ensure_mixed(ctx, static_cast<size_t>(n))) return fail(ctx, LSMPS_CUDA_ERROR, "mixed-form allocation failed");
+  if (!ensure_mixed(ctx, static_cast<size_t>(n)) || !ensure_moment_sums(ctx, static_cast<size_t>(n))) return fail(ctx, LSMPS_CUDA_ERROR, "mixed-form allocation failed");
   const double inv_re = 1.0 / p.support_radius;
   const index_t* srows = sorted_rows_of(ctx, fn, static_cast<size_t>(n));
   const index_t* fi = srows ? srows : fn.indices;
-  MixedSumArgs sa{n, ctx->pack_fluid[0], fn.offsets, fi, inv_re, ctx->mixed_sums, ctx->order, srows ? 1 : 0};
+  SumArgs sa{n, ctx->pack_fluid[0], fn.offsets, fi, inv_re, ctx->moment_sums, ctx->order, srows ? 1 : 0};
   const bool split = ctx->knob[LSMPS_KNOB_MOMENT_OCCUPANCY] == 2;
   MixedRowArgs ra{};
   ra.n = n;
-  ra.sums = ctx->mixed_sums;
+  ra.sums = ctx->moment_sums;
   ra.fp = ctx->pack_fluid[0];
   ra.wp = ctx->pack_wall[0];
   ra.wn = ctx->pack_wall[2];
@@ -1340,19 +1316,6 @@ lsmps_status prepare_moments_impl(lsmps_ctx* ctx, const lsmps_fluid& fluid, cons
   if (fluid.count > fn.particle_count || fluid.count > wn.particle_count)
     return fail(ctx, LSMPS_INVALID_ARGUMENT, "Moment matrix neighbor lists are smaller than fluid particle count");
   if (count < 0 || !kinds) return fail(ctx, LSMPS_INVALID_ARGUMENT, "moment kinds missing");
-  // Group the Type-A kinds (one launch) and the Type-B kinds (one launch each).
-  MomentArgs base{};
-  base.fluid = fluid;
-  base.walls = walls;
-  base.fo = fn.offsets;
-  base.fi = fn.indices;
-  base.wo = wn.offsets;
-  base.wi = wn.indices;
-  base.re = p.support_radius;
-  base.inv_re = 1.0 / p.support_radius;
-  base.lambda = p.lsmps_regularization;
-  base.wall_scale = p.lsmps_wall_weight_scale;
-  base.status = ctx->d_status;
   const index_t n = static_cast<index_t>(fluid.count);
   int velocity_a = -1, pressure_a = -1;
   for (int k = 0; k < count; ++k) {
@@ -1372,64 +1335,69 @@ lsmps_status prepare_moments_impl(lsmps_ctx* ctx, const lsmps_fluid& fluid, cons
     return KindOut{boundary_of(mk.kind), mk.inverse_matrices, mk.moment_trace, mk.regularization_added, mk.info,
                    mk.inversion_count};
   };
-  const dim3 grid(div_up(n, kMomentThreads)), block(kMomentThreads);
-  // single-kind launches: the warps' inverse staging (27 x kMomentThreads doubles)
-  constexpr size_t kStageBytes = sizeof(double) * 27 * kMomentThreads;
   if (!ensure_packs(ctx, fluid.count, walls.count)) return fail(ctx, LSMPS_CUDA_ERROR, "pack allocation failed");
   const index_t* srows = sorted_rows_of(ctx, fn, fluid.count);
   pack_fluid_positions(ctx, fluid, srows ? ctx->order : nullptr);
-  // (the mixed form packs the walls itself, after its fluid sums)
   const bool fused = velocity_a >= 0 && pressure_a >= 0;
-  if (!(fused && ctx->precision == LSMPS_PRECISION_MIXED)) {
-    pack_wall_positions(ctx, walls);
-    pack_wall_normals(ctx, walls);
-  }
-  MomentPackedArgs pa{n, ctx->pack_fluid[0], ctx->pack_wall[0], ctx->pack_wall[2], fn.offsets,
-                      srows ? srows : fn.indices, wn.offsets, wn.indices, base.inv_re, base.lambda,
-                      base.wall_scale, KindOut{}, KindOut{}, ctx->d_status, ctx->order, srows ? 1 : 0};
-  const bool capped = ctx->knob[LSMPS_KNOB_MOMENT_OCCUPANCY] == 1;
-  const bool split = ctx->knob[LSMPS_KNOB_MOMENT_OCCUPANCY] == 2;
-  if (fused && ctx->precision == LSMPS_PRECISION_MIXED) {
+  const bool mixed = fused && ctx->precision == LSMPS_PRECISION_MIXED;
+  if (mixed) {
     // Mixed form: FP32 assembly and factorisation with FP64 refinement; the
-    // full inverse is written (FP64) for the caller's views.
+    // full inverse is written (FP64) for the caller's views.  (It packs the
+    // walls itself, after its fluid sums.)
     lsmps_status st =
         launch_mixed(ctx, n, fn, wn, p, out_of(kinds[velocity_a]), out_of(kinds[pressure_a]), true, walls);
     if (st) return st;
-  } else if (fused) {
-    // The step's two kinds share the fluid sums: one pass over the rows.
-    MomentPackedArgs a = pa;
-    a.k0 = out_of(kinds[velocity_a]);
-    a.k1 = out_of(kinds[pressure_a]);
-    const size_t smem = sizeof(double) * kMonomials * kMomentThreads;
-    if (split)
-      launch_named(ctx, "moment_a_split_kernel", moment_a_split_kernel, dim3(div_up(n, kWarp)), dim3(2 * kWarp), 0, a);
-    else if (capped)
-      launch_named(ctx, "moment_a_kernel<V,P>", moment_a_kernel<1, 2, 8>, grid, block, smem, a);
-    else
-      launch_named(ctx, "moment_a_kernel<V,P>", moment_a_kernel<1, 2, 1>, grid, block, smem, a);
   }
+  // The other kinds share one pass over the rows.
+  FinishArgs a9{}, a10{};
+  int many9 = 0, many10 = 0;
+  bool dirichlet = false, neumann_terms = false;
+  const auto finish = [&](FinishArgs& a, int& many, auto kernel, const char* name) {
+    launch_named(ctx, name, kernel, dim3(div_up(n, kFinishThreads), many), dim3(kFinishThreads), 0, a);
+    many = 0;
+  };
   for (int k = 0; k < count; ++k) {
-    if (fused && (k == velocity_a || k == pressure_a)) continue;
-    MomentPackedArgs a = pa;
-    a.k0 = out_of(kinds[k]);
-    switch (kinds[k].kind) {
-      case LSMPS_MOMENT_VELOCITY_WALL_DIRICHLET_A:
-        launch_named(ctx, "moment_a_kernel<V>", moment_a_kernel<1, -1, 1>, grid, block, kStageBytes, a);
-        break;
-      case LSMPS_MOMENT_PRESSURE_WALL_NEUMANN_A:
-        launch_named(ctx, "moment_a_kernel<P>", moment_a_kernel<2, -1, 1>, grid, block, kStageBytes, a);
-        break;
-      case LSMPS_MOMENT_PRESSURE_WALL_NEUMANN_B: {
-        MomentArgs b = base;
-        b.k0 = a.k0;
-        launch_named(ctx, "moment_kernel<B>", moment_kernel<10, 2, -1>, grid, block, 0, b);
-        break;
-      }
-      default:
-        launch_named(ctx, "moment_a_kernel<F>", moment_a_kernel<0, -1, 1>, grid, block, kStageBytes, a);
-        break;
-    }
+    if (mixed && (k == velocity_a || k == pressure_a)) continue;
+    const int boundary = boundary_of(kinds[k].kind);
+    dirichlet |= boundary == 1;
+    neumann_terms |= boundary == 2;
+    ++(kinds[k].kind == LSMPS_MOMENT_PRESSURE_WALL_NEUMANN_B ? many10 : many9);
   }
+  if (many9 + many10 == 0) return check_launch(ctx, "moment matrices");
+  if (!ensure_moment_sums(ctx, fluid.count)) return fail(ctx, LSMPS_CUDA_ERROR, "moment sums allocation failed");
+  const size_t cap = ctx->moment_cap;
+  double* wall_velocity = ctx->moment_sums + cap * kMonomialsB;
+  double* wall_pressure = wall_velocity + cap * kMonomials;
+  const index_t* fi = srows ? srows : fn.indices;
+  const SumArgs sa{n, ctx->pack_fluid[0], fn.offsets, fi, 1.0 / p.support_radius, ctx->moment_sums, ctx->order,
+                   srows ? 1 : 0};
+  const bool with_walls = (dirichlet || neumann_terms) && walls.count > 0;
+  launch_plain_sums(ctx, sa, with_walls ? static_cast<const index_t*>(wn.offsets) : nullptr, many10 > 0);
+  if (with_walls) {
+    pack_wall_positions(ctx, walls);
+    pack_wall_normals(ctx, walls);
+    const WallArgs wa{n, ctx->pack_fluid[0], ctx->pack_wall[0], ctx->pack_wall[2], wn.offsets, wn.indices,
+                      1.0 / p.support_radius, p.lsmps_wall_weight_scale, ctx->moment_sums, wall_velocity, wall_pressure,
+                      ctx->order, srows ? 1 : 0, ctx->moment_walled, ctx->moment_walls};
+    const int blocks = std::min(div_up(n, kWallThreads), ctx->sm_count * 12);
+    launch(ctx, wall_sums_kernel, dim3(blocks, (dirichlet ? 1 : 0) + (neumann_terms ? 1 : 0)), dim3(kWallThreads), 0,
+           wa, dirichlet ? 0 : 1);
+  }
+  a9 = FinishArgs{n, ctx->moment_sums, wall_velocity, wall_pressure, wn.offsets, p.lsmps_regularization,
+                  {},  ctx->d_status,     ctx->order,    ctx->moment_walls};
+  a10 = a9;
+  many9 = many10 = 0;
+  for (int k = 0; k < count; ++k) {
+    if (mixed && (k == velocity_a || k == pressure_a)) continue;
+    if (kinds[k].kind == LSMPS_MOMENT_PRESSURE_WALL_NEUMANN_B)
+      a10.k[many10++] = out_of(kinds[k]);
+    else
+      a9.k[many9++] = out_of(kinds[k]);
+    if (many9 == 3) finish(a9, many9, moment_finish_kernel<9>, "moment_finish_kernel<9>");
+    if (many10 == 3) finish(a10, many10, moment_finish_kernel<10>, "moment_finish_kernel<10>");
+  }
+  if (many9) finish(a9, many9, moment_finish_kernel<9>, "moment_finish_kernel<9>");
+  if (many10) finish(a10, many10, moment_finish_kernel<10>, "moment_finish_kernel<10>");
   return check_launch(ctx, "moment matrices");
 }
 

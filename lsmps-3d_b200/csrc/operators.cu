@@ -50,35 +50,6 @@ __device__ __forceinline__ void basis_jt(const double s[3], const double beta[9]
   out[2] = beta[2] + 2.0 * s[2] * beta[5] + s[1] * beta[7] + s[0] * beta[8];
 }
 
-// Sums of N values over the warp, each exchange halving the values a lane
-// still carries: lane l ends with the totals of values base .. base + count - 1
-// (count 0, 1 or more) in v[0 ..].  N - 1 exchanges or so instead of the 5 N
-// of N separate butterflies.  The order of the additions is fixed.
-template <int N, int D = 16>
-__device__ __forceinline__ void warp_totals(double* v, int& base, int& count) {
-  if constexpr (D > 0) {
-    if constexpr (N == 1) {
-      v[0] += __shfl_xor_sync(0xffffffffu, v[0], D);
-      warp_totals<1, D / 2>(v, base, count);
-    } else {
-      constexpr int H = (N + 1) / 2;
-      const bool upper = (threadIdx.x & D) != 0;
-#pragma unroll
-      for (int k = 0; k < H; ++k) {
-        const double hi = k + H < N ? v[k + H] : 0.0;
-        const double keep = upper ? hi : v[k];
-        const double send = upper ? v[k] : hi;
-        v[k] = keep + __shfl_xor_sync(0xffffffffu, send, D);
-      }
-      base += upper ? H : 0;
-      const int rest = count - H;
-      count = upper ? (rest > 0 ? rest : 0) : (count < H ? count : H);
-      warp_totals<H, D / 2>(v, base, count);
-    }
-  }
-}
-
-
 __device__ __forceinline__ double opt(const double* p, index_t i) { return p ? p[i] : 0.0; }
 
 __device__ __forceinline__ bool dirichlet_row(const int32_t* label, index_t i) {
@@ -289,7 +260,7 @@ __global__ void __launch_bounds__(kAdjThreads, 5) operators_forward_kernel(Opera
     wall_rhs = group_sum<kWarp>(wall_rhs, 0xffffffffu);
   }
   int base = 0, count = 8;
-  warp_totals<8>(r, base, count);  // lane 4 k holds total k
+  lane_totals<8, 16>(r, base, count);  // lane 4 k holds total k
   const double t = r[0];
   const double diag = __shfl_sync(0xffffffffu, t, 28);
   if ((lane & 3) != 0) return;
@@ -407,7 +378,7 @@ __global__ void __launch_bounds__(kAdjThreads, 4) operators_backward_kernel(cons
       }
     }
     int base = 0, count = 27;
-    warp_totals<27, 8>(r, base, count);  // over the 16 lanes of a half: at most 2 left a lane
+    lane_totals<27, 8>(r, base, count);  // over the 16 lanes of a half: at most 2 left a lane
 #pragma unroll
     for (int k = 0; k < 2; ++k)
       if (k < count && 27 * half + base + k < 45) R[27 * half + base + k] = r[k];
@@ -603,7 +574,7 @@ __global__ void __launch_bounds__(kAdjThreads, 4) operators_backward_kernel(cons
   }
   if (!Atomic && a.j0 != 0) return;  // a later pass over the same rows
   int base = 0, count = 7;
-  warp_totals<7>(acc, base, count);
+  lane_totals<7, 16>(acc, base, count);
   // lanes that differ in the last two exchanges hold the same total
   if (count == 0 || (lane & 3) != 0) return;
   if (Atomic) {
@@ -682,7 +653,7 @@ __global__ void __launch_bounds__(kAdjThreads) operators_collect_kernel(Operator
     }
   }
   int base = 0, left = 7;
-  warp_totals<7>(acc, base, left);
+  lane_totals<7, 16>(acc, base, left);
   if (left == 0 || (lane & 3) != 0) return;
   double* out = base < 4 ? a.phibar[base] : a.xbar[base - 4];
   if (out) out[j] = acc[0] + a.own[8 * static_cast<size_t>(j) + base];

@@ -53,8 +53,12 @@ def kernel_bytes(nf: int, nw: int, kf: int, kw: int, c: int, s: int = 8) -> dict
     out = {}
     moment_kind_out = (81 * s + 2 * s + 4) * nf  # inverse, trace, regularisation, info
     moment_in = rows + pos_f + 2 * pos_w  # wall positions + normals
-    out["moment_a_kernel<V,P>"] = out["moment_a_split_kernel"] = moment_in + 2 * moment_kind_out
-    out["moment_a_kernel<V>"] = out["moment_a_kernel<P>"] = moment_in + moment_kind_out
+    # plain form: the fluid row's sums, the wall rows' terms (both kinds), two inverses
+    sums = 31 * s * nf
+    for g in (1, 2):
+        out[f"plain_sums_kernel<{g}>"] = 8 * (nf + 1) + 4 * kf + pos_f + sums
+    out["wall_sums_kernel"] = moment_in - 4 * kf + 2 * sums
+    out["moment_finish_kernel<9>"] = 2 * (sums + moment_kind_out)
     lap = rows + 2 * pos_f + 2 * pos_w + 3 * s * nf
     # the two mixed stages in one kernel (row halves on two warps)
     out["moment_mixed_split_kernel<false>"] = (4 * (nf + 1) + 4 * kf + pos_f + 2 * (4 * (nf + 1) + 4 * kw + 2 * pos_w)
