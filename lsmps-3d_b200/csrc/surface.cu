@@ -18,20 +18,42 @@ constexpr int kSurfaceThreads = 128;
 
 __device__ __forceinline__ double safe_rsqrt(double v) { return rsqrt(v > 1.0e-20 ? v : 1.0e-20); }
 
-// accumulate_neighbor_moments, surface_detection.cu:33-59
-__device__ __forceinline__ void accumulate(double dx, double dy, double dz, double re, double& nd, double& sx,
-                                           double& sy, double& sz, int& weighted) {
-  const double d2 = dx * dx + dy * dy + dz * dz;
-  if (d2 <= 0.0) return;
+// Squared lengths (of an offset; of the summed offsets) with the products fused
+// as the compiler fuses them in the reference's expressions, said outright so
+// that both label kernels give the same bits: the labels compare sums of these
+// with thresholds.
+__device__ __forceinline__ double length2(double x, double y, double z) { return fma(z, z, fma(x, x, y * y)); }
+__device__ __forceinline__ double squares(double x, double y, double z) { return fma(z, z, fma(y, y, x * x)); }
+
+// One neighbour's terms of accumulate_neighbor_moments
+// (surface_detection.cu:33-59): the weight w, w times the offset, and 1 / d; all
+// 0 (and uncounted) for one that has no weight.  The sums are n += w and
+// s_c += (w d_c) (1 / d), added in row order.
+struct Term {
+  double w, x, y, z, inv_d;
+  int counted;
+};
+
+__device__ __forceinline__ Term term_of(const double4& q, const double4& own, double re) {
+  const double dx = q.x - own.x, dy = q.y - own.y, dz = q.z - own.z;
+  const double d2 = length2(dx, dy, dz);
   const double d = sqrt(d2);
   const double w = lin_weight(d, re);
-  if (w <= 0.0) return;
-  const double inv_d = 1.0 / d;
-  nd += w;
-  sx += w * dx * inv_d;
-  sy += w * dy * inv_d;
-  sz += w * dz * inv_d;
-  ++weighted;
+  if (d2 <= 0.0 || w <= 0.0) return Term{0.0, 0.0, 0.0, 0.0, 0.0, 0};
+  return Term{w, w * dx, w * dy, w * dz, 1.0 / d, 1};
+}
+
+struct Moments {
+  double nd, sx, sy, sz;
+  int weighted;
+};
+
+__device__ __forceinline__ void add_term(Moments& m, const Term& t) {
+  m.nd += t.w;
+  m.sx = fma(t.x, t.inv_d, m.sx);
+  m.sy = fma(t.y, t.inv_d, m.sy);
+  m.sz = fma(t.z, t.inv_d, m.sz);
+  m.weighted += t.counted;
 }
 
 struct Basis3 {
@@ -39,8 +61,13 @@ struct Basis3 {
   double x[3], y[3], z[3];
 };
 
-// add_wall_basis_direction, surface_detection.cu:123-149
-__device__ __forceinline__ void add_direction(Basis3& b, double x, double y, double z, double thr) {
+// add_wall_basis_direction, surface_detection.cu:123-149: the remainder of a
+// direction against the basis, and whether it joins it.
+struct Remainder {
+  double x, y, z, len2;
+};
+
+__device__ __forceinline__ Remainder remainder_of(const Basis3& b, double x, double y, double z) {
   double rx = x, ry = y, rz = z;
   for (int k = 0; k < b.count; ++k) {
     const double proj = rx * b.x[k] + ry * b.y[k] + rz * b.z[k];
@@ -48,12 +75,14 @@ __device__ __forceinline__ void add_direction(Basis3& b, double x, double y, dou
     ry -= proj * b.y[k];
     rz -= proj * b.z[k];
   }
-  const double len2 = rx * rx + ry * ry + rz * rz;
-  if (len2 <= thr * thr || b.count >= 3) return;
-  const double inv = safe_rsqrt(len2);
-  b.x[b.count] = rx * inv;
-  b.y[b.count] = ry * inv;
-  b.z[b.count] = rz * inv;
+  return Remainder{rx, ry, rz, rx * rx + ry * ry + rz * rz};
+}
+
+__device__ __forceinline__ void join(Basis3& b, const Remainder& r) {
+  const double inv = safe_rsqrt(r.len2);
+  b.x[b.count] = r.x * inv;
+  b.y[b.count] = r.y * inv;
+  b.z[b.count] = r.z * inv;
   ++b.count;
 }
 
@@ -79,61 +108,42 @@ struct SurfaceArgs {
   int32_t* sorted_labels;
 };
 
-__global__ void __launch_bounds__(kSurfaceThreads) classify_kernel(SurfaceArgs a) {
-  const index_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= static_cast<index_t>(a.fluid.count)) return;
-  const index_t i = visit(a.order, t);
-  const index_t fb = a.fo[i], fe = a.fo[i + 1];
-  const index_t wb = a.wo[i], we = a.wo[i + 1];
-  const index_t fcount = fe - fb, wcount = we - wb;
+// build_wall_basis's direction of wall j (surface_detection.cu:151-197): its
+// inward normal reversed and normalised; false when the wall is out of reach or
+// has no normal.
+__device__ __forceinline__ bool wall_direction(const SurfaceArgs& a, const double4& own, index_t j, double& x, double& y,
+                                               double& z) {
+  const double4 q = ld4(a.wp, j);
+  const double dx = q.x - own.x, dy = q.y - own.y, dz = q.z - own.z;
+  const double d2 = dx * dx + dy * dy + dz * dz;
+  if (d2 <= 0.0) return false;
+  const double d = sqrt(d2);
+  if (lin_weight(d, a.p.support_radius) <= 0.0) return false;
+  const double4 nrm = ld4(a.wn, j);
+  const double nx = nrm.x, ny = nrm.y, nz = nrm.z;
+  const double nl2 = nx * nx + ny * ny + nz * nz;
+  if (nl2 <= 0.0) return false;
+  const double inv = safe_rsqrt(nl2);
+  x = -nx * inv;
+  y = -ny * inv;
+  z = -nz * inv;
+  return true;
+}
+
+// The label and the diagnostics of particle i (visiting position t) from its
+// sums and the basis of its walls' directions.
+__device__ __forceinline__ void label(const SurfaceArgs& a, index_t t, index_t i, index_t fcount, index_t wcount,
+                                      const Moments& m, const Basis3& basis) {
   const index_t cls = a.p.include_wall_neighbors ? fcount + wcount : fcount;
-  const double re = a.p.support_radius;
-  const double4 own = ld4(a.fp, self_of(a.sorted, t, i));
-  const double px = own.x, py = own.y, pz = own.z;
-  double nd = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
-  int weighted = 0;
-  // the next neighbour's record is loaded while this one is accumulated
-  double4 qn = ld4(a.fp, fb < fe ? a.fi[fb] : i);
-  index_t jnn = fb + 1 < fe ? a.fi[fb + 1] : i;  // the index after the next
-  for (index_t o = fb; o < fe; ++o) {
-    const double4 q = qn;
-    if (o + 1 < fe) {
-      qn = ld4(a.fp, jnn);
-      if (o + 2 < fe) jnn = a.fi[o + 2];
-    }
-    accumulate(q.x - px, q.y - py, q.z - pz, re, nd, sx, sy, sz, weighted);
-  }
-  if (a.p.include_wall_neighbors) {
-    for (index_t o = wb; o < we; ++o) {
-      const double4 q = ld4(a.wp, a.wi[o]);
-      accumulate(q.x - px, q.y - py, q.z - pz, re, nd, sx, sy, sz, weighted);
-    }
-  }
+  const double nd = m.nd, sx = m.sx, sy = m.sy, sz = m.sz;
+  const int weighted = m.weighted;
   double aniso = 0.0;
-  if (weighted > 0) aniso = sqrt(sx * sx + sy * sy + sz * sz) / static_cast<double>(weighted);
+  if (weighted > 0) aniso = sqrt(squares(sx, sy, sz)) / static_cast<double>(weighted);
   const double ratio = nd / a.n0;
   const double mx = -sx, my = -sy, mz = -sz;
-  const double ml2 = mx * mx + my * my + mz * mz;
+  const double ml2 = squares(mx, my, mz);
   double ax = mx, ay = my, az = mz;
   if (ml2 > 0.0 && a.p.include_wall_neighbors) {
-    // build_wall_basis, surface_detection.cu:151-197
-    Basis3 basis;
-    basis.count = 0;
-    for (index_t o = wb; o < we; ++o) {
-      const index_t j = a.wi[o];
-      const double4 q = ld4(a.wp, j);
-      const double dx = q.x - px, dy = q.y - py, dz = q.z - pz;
-      const double d2 = dx * dx + dy * dy + dz * dz;
-      if (d2 <= 0.0) continue;
-      const double d = sqrt(d2);
-      if (lin_weight(d, re) <= 0.0) continue;
-      const double4 nrm = ld4(a.wn, j);
-      const double nx = nrm.x, ny = nrm.y, nz = nrm.z;
-      const double nl2 = nx * nx + ny * ny + nz * nz;
-      if (nl2 <= 0.0) continue;
-      const double inv = safe_rsqrt(nl2);
-      add_direction(basis, -nx * inv, -ny * inv, -nz * inv, a.p.wall_normal_independence_threshold);
-    }
     for (int k = 0; k < basis.count; ++k) {
       const double proj = ax * basis.x[k] + ay * basis.y[k] + az * basis.z[k];
       if (proj > 0.0) {
@@ -177,6 +187,136 @@ __global__ void __launch_bounds__(kSurfaceThreads) classify_kernel(SurfaceArgs a
     if (d.surface_normal_y) d.surface_normal_y[i] = sny;
     if (d.surface_normal_z) d.surface_normal_z[i] = snz;
   }
+}
+
+// The row's terms added in order; the next record is loaded while this one is
+// used, with the index one further ahead.
+__device__ __forceinline__ void add_row(Moments& m, const double4* __restrict__ rec, const index_t* __restrict__ idx,
+                                        index_t b, index_t e, const double4& own, double re) {
+  double4 qn = b < e ? ld4(rec, idx[b]) : own;
+  index_t jn = b + 1 < e ? idx[b + 1] : -1;
+#pragma unroll 1
+  for (index_t o = b; o < e; ++o) {
+    const double4 q = qn;
+    qn = jn >= 0 ? ld4(rec, jn) : own;
+    jn = o + 2 < e ? idx[o + 2] : -1;
+    add_term(m, term_of(q, own, re));
+  }
+}
+
+// One thread per particle.  500,000 particles: 0.47 ms, FP64 pipe 42%, L1
+// wavefronts 58%, 161 instructions an entry, most of them the square root's and
+// the two divisions' (whose roundings the labels need).  Tried: two or four
+// entries' terms formed together (0.53 and 0.60 ms: 90 to 120 registers), eight
+// blocks per SM (0.51 ms).
+__global__ void __launch_bounds__(kSurfaceThreads) classify_kernel(SurfaceArgs a) {
+  const index_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= static_cast<index_t>(a.fluid.count)) return;
+  const index_t i = visit(a.order, t);
+  const index_t fb = a.fo[i], fe = a.fo[i + 1];
+  const index_t wb = a.wo[i], we = a.wo[i + 1];
+  const double re = a.p.support_radius;
+  const double4 own = ld4(a.fp, self_of(a.sorted, t, i));
+  Moments m{0.0, 0.0, 0.0, 0.0, 0};
+  add_row(m, a.fp, a.fi, fb, fe, own, re);
+  Basis3 basis;
+  basis.count = 0;
+  if (a.p.include_wall_neighbors) {
+    add_row(m, a.wp, a.wi, wb, we, own, re);
+    const double thr = a.p.wall_normal_independence_threshold;
+    for (index_t o = wb; o < we && basis.count < 3; ++o) {  // (a full basis takes no more)
+      double x, y, z;
+      if (!wall_direction(a, own, a.wi[o], x, y, z)) continue;
+      const Remainder r = remainder_of(basis, x, y, z);
+      if (!(r.len2 <= thr * thr)) join(basis, r);
+    }
+  }
+  label(a, t, i, fe - fb, we - wb, m, basis);
+}
+
+// The same labels, bit for bit, for sets that do not fill the GPU: kLabelLanes
+// lanes form the terms of as many entries at once; of each group, lanes 0..3 add
+// one of the four sums each, in row order.  A wall joins the basis by the
+// remainder against the walls that joined before it, so the lanes look for the
+// next one together: at most four passes over the walls.  1,000 particles: 18
+// against 176 us; 21,793: 51 against 179; 61,250: 110 against 160; 255,723: 393
+// against 357, the exchanges through shared memory then costing more than the
+// latency they hide.  The lines cross near 190,000 particles; below it by a third.
+constexpr int kLabelLanes = 16;
+constexpr index_t kLabelSmall = 131072;
+
+__global__ void __launch_bounds__(kSurfaceThreads) classify_small_kernel(SurfaceArgs a) {
+  constexpr int G = kLabelLanes, kGroups = kSurfaceThreads / G;
+  __shared__ double s_term[kGroups][5][G + 1];
+  const index_t t = (blockIdx.x * blockDim.x + threadIdx.x) / G;
+  const int l = threadIdx.x & (G - 1);
+  if (t >= static_cast<index_t>(a.fluid.count)) return;  // the whole group
+  const unsigned gm = group_mask<G>();
+  double(*term)[G + 1] = s_term[threadIdx.x / G];
+  const index_t i = visit(a.order, t);
+  const index_t fb = a.fo[i], fe = a.fo[i + 1];
+  const index_t wb = a.wo[i], we = a.wo[i + 1];
+  const double re = a.p.support_radius;
+  const double4 own = ld4(a.fp, self_of(a.sorted, t, i));
+  double sum = 0.0;  // lane 0: n; 1..3: s
+  int weighted = 0;
+  const auto add = [&](const double4* __restrict__ rec, const index_t* __restrict__ idx, index_t b, index_t e) {
+    double4 q = b + l < e ? ld4(rec, idx[b + l]) : own;
+    index_t jn = b + G + l < e ? idx[b + G + l] : -1;
+    for (index_t o = b; o < e; o += G) {
+      const Term v = term_of(q, own, re);  // (none past the row's end: own, at distance 0)
+      q = jn >= 0 ? ld4(rec, jn) : own;
+      jn = o + 2 * G + l < e ? idx[o + 2 * G + l] : -1;
+      weighted += v.counted;
+      term[0][l] = v.w;
+      term[1][l] = v.x;
+      term[2][l] = v.y;
+      term[3][l] = v.z;
+      term[4][l] = v.inv_d;
+      __syncwarp(gm);
+      if (l < 4) {
+#pragma unroll
+        for (int k = 0; k < G; ++k) sum = fma(term[l][k], l == 0 ? 1.0 : term[4][k], sum);
+      }
+      __syncwarp(gm);
+    }
+  };
+  add(a.fp, a.fi, fb, fe);
+  Basis3 basis;
+  basis.count = 0;
+  if (a.p.include_wall_neighbors) {
+    add(a.wp, a.wi, wb, we);
+    const double thr = a.p.wall_normal_independence_threshold;
+    index_t o = wb;
+    while (o < we && basis.count < 3) {
+      double x = 0.0, y = 0.0, z = 0.0;
+      Remainder r{0.0, 0.0, 0.0, 0.0};
+      bool joins = false;
+      if (o + l < we && wall_direction(a, own, a.wi[o + l], x, y, z)) {
+        r = remainder_of(basis, x, y, z);
+        joins = !(r.len2 <= thr * thr);
+      }
+      const unsigned any = __ballot_sync(gm, joins) & gm;
+      if (any == 0u) {
+        o += G;
+        continue;
+      }
+      const int first = __ffs(any) - 1;
+      const Remainder w{__shfl_sync(gm, r.x, first), __shfl_sync(gm, r.y, first), __shfl_sync(gm, r.z, first),
+                        __shfl_sync(gm, r.len2, first)};
+      join(basis, w);
+      o += (first & (G - 1)) + 1;
+    }
+  }
+  weighted = __reduce_add_sync(gm, weighted);
+  const int lead = (threadIdx.x & (kWarp - 1)) & ~(G - 1);
+  Moments m;
+  m.nd = __shfl_sync(gm, sum, lead);
+  m.sx = __shfl_sync(gm, sum, lead + 1);
+  m.sy = __shfl_sync(gm, sum, lead + 2);
+  m.sz = __shfl_sync(gm, sum, lead + 3);
+  m.weighted = weighted;
+  if (l == 0) label(a, t, i, fe - fb, we - wb, m, basis);
 }
 
 // expand_near_surface_kernel, surface_detection.cu:322-348.  Only Inner rows
@@ -401,7 +541,11 @@ lsmps_status classify_surface_impl(lsmps_ctx* ctx, const lsmps_fluid& fluid, con
   a.wn = ctx->pack_wall[2];
   a.order = ctx->order;
   const index_t n = static_cast<index_t>(fluid.count);
-  launch(ctx, classify_kernel, dim3(div_up(n, kSurfaceThreads)), dim3(kSurfaceThreads), 0, a);
+  if (n <= kLabelSmall)
+    launch(ctx, classify_small_kernel, dim3(div_up(static_cast<long long>(n) * kLabelLanes, kSurfaceThreads)),
+           dim3(kSurfaceThreads), 0, a);
+  else
+    launch(ctx, classify_kernel, dim3(div_up(n, kSurfaceThreads)), dim3(kSurfaceThreads), 0, a);
   if (p.near_surface_radius > 0.0) {
     launch(ctx, expand_kernel, dim3(div_up(static_cast<long long>(n) * kExpandLanes, kSurfaceThreads)),
            dim3(kSurfaceThreads), 0,
