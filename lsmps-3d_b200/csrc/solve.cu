@@ -13,14 +13,17 @@
 // Algorithm: GMRES(m) of Saad and Schultz (1986) with right preconditioning
 // (none, or Jacobi: M = diag(A)).  Arnoldi uses classical Gram-Schmidt with
 // one re-orthogonalisation (CGS2), so every projection is a batch of
-// independent dot products; the Hessenberg column, its Givens rotations and
-// the residual estimate |g_{j+1}| are kept on the host.  Each Arnoldi step is
-// one SpMV (G lanes per CSR row, the vector read through L2), two batched
-// dot-product passes and two update passes over the basis, and one 16-byte
-// read-back.  All reductions go through per-block partials summed in a fixed
-// order, so a solve is bitwise reproducible.
+// independent dot products.  An Arnoldi step is three kernels: the new basis
+// vector scaled, multiplied by A and projected (h = V^T w); the projection
+// taken off and the remainder projected again; that taken off, and the norm.
+// Each kernel's last block to finish adds the blocks' partial sums in a fixed
+// order, and that of the third extends the Hessenberg matrix by its column and
+// rotates it, so a solve is bitwise reproducible, nothing waits for the host
+// within a restart cycle, and a cycle that has converged lets its remaining
+// launches return at once.
+#include <algorithm>
 #include <cmath>
-#include <vector>
+#include <cstddef>
 
 #include "impl.cuh"
 
@@ -28,118 +31,374 @@ namespace lsmps {
 namespace {
 
 constexpr int kSolveThreads = 256;
-constexpr int kSpmvLanes = 8;
+constexpr int kSolveWarps = kSolveThreads / kWarp;
+constexpr int kRowLanes = 8;       // lanes per CSR row in products that end in dot products
+constexpr int kProductLanes = 16;  // ... in the products without
 constexpr int kMaxRestart = 64;
+// Rows up to which a product and its dot products are one kernel (measured at
+// product_dots_kernel).
+constexpr index_t kFusedRows = 100000;
 
-// y = A (s ∘ x) (s = NULL: y = A x); kSpmvLanes lanes per row.
+// The solve's scalars, in device memory.
+struct SolveState {
+  double beta, beta0, target;
+  double scale;  // 1 / norm of the vector that the next product takes
+  int iters;
+  int steps;      // of this cycle
+  int converged;  // the residual has reached the target
+  int stop;       // the rest of this cycle's launches return at once
+  unsigned tickets;
+  double h[kMaxRestart + 1];                       // first projection of the step
+  double h2[kMaxRestart + 1];                      // second projection
+  double H[kMaxRestart * (kMaxRestart + 1)];       // rotated Hessenberg columns
+  double cs[kMaxRestart], sn[kMaxRestart], g[kMaxRestart + 1];
+};
+
+struct SolveArgs {
+  index_t n;
+  const index_t* ro;
+  const index_t* ci;
+  const double* va;
+  const double* dinv;        // Jacobi: 1 / a_ii, or NULL
+  double* V;                 // [restart + 1][ldv]
+  size_t ldv;
+  double* w[2];  // the vector to be normalised next, and its product
+  double* x;
+  const double* b;
+  double* partial;  // [kMaxRestart + 1][gridDim.x]
+  SolveState* st;
+  volatile int* stopped;  // host memory: set with st->stop
+  int restart;
+  int max_iters;
+  double tolerance;
+  int relative;
+};
+
+// Lane l's share of row . (x, or dinv ∘ x): the entries l, l + G, ... of the row,
+// so that the lanes' gathers of x fall on neighbouring columns together, four
+// rounds of values and columns in flight.  500,000 rows of 109 entries, B200:
+// 122 us a product with 16 lanes (5.4 TB/s), 138 with 8, 137 with 32, 179 with 4:
+// bound by the load pipe's wavefronts (ncu at 8 lanes: 85%), of which the gathers
+// of x take most; rows of one warp that lie next to each other share the lines
+// of their values.  Tried: four consecutive entries a lane with 32-byte loads
+// (160 us: fewer loads, scattered gathers).
 template <int G>
-__global__ void __launch_bounds__(kSolveThreads)
-    spmv_kernel(index_t n, const index_t* __restrict__ ro, const index_t* __restrict__ ci,
-                const double* __restrict__ va, const double* __restrict__ x, const double* __restrict__ s,
-                double* __restrict__ y) {
-  const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const index_t row = static_cast<index_t>(t / G);
-  const int l = static_cast<int>(t % G);
-  if (row >= n) return;  // the whole group
+__device__ __forceinline__ double row_product(const SolveArgs& a, index_t row, int l, const double* __restrict__ x) {
+  constexpr int kRounds = 4;
+  const index_t e = a.ro[row + 1];
   double acc = 0.0;
-  const index_t e = ro[row + 1];
-  for (index_t k = ro[row] + l; k < e; k += G) {
-    const index_t c = ci[k];
-    acc += va[k] * (s ? s[c] * x[c] : x[c]);
+  for (index_t k = a.ro[row] + l; k < e; k += kRounds * G) {
+    index_t c[kRounds];
+    double v[kRounds];
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      const index_t at = k + r * G;
+      c[r] = at < e ? __ldcs(a.ci + at) : -1;
+      v[r] = at < e ? __ldcs(a.va + at) : 0.0;
+    }
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r)
+      if (c[r] >= 0) acc = fma(v[r], a.dinv ? a.dinv[c[r]] * x[c[r]] : x[c[r]], acc);
   }
-  acc = group_sum<G>(acc, group_mask<G>());
-  if (l == 0) y[row] = acc;
+  return group_sum<G>(acc, group_mask<G>());
 }
 
-// Per-block partial sums of a block-wide value, written to partial[blockIdx].
-__device__ __forceinline__ void block_partial(double v, double* partial_out) {
-  __shared__ double red[kSolveThreads / kWarp];
-  for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+// True in every thread of the last block to get here; the blocks' earlier
+// global writes are then visible to it.  No block waits for another.
+__device__ __forceinline__ bool last_block(SolveState* st) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(&st->tickets, 1u) == gridDim.x - 1;
+    if (last) st->tickets = 0u;
+  }
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+
+// Sum over the block's threads, in thread 0 (and every thread of warp 0).
+__device__ __forceinline__ double block_sum(double v) {
+  __shared__ double red[kSolveWarps];
+  v = group_sum<kWarp>(v, 0xffffffffu);
+  __syncthreads();
   if ((threadIdx.x & (kWarp - 1)) == 0) red[threadIdx.x / kWarp] = v;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double sum = 0.0;
-    for (int w = 0; w < kSolveThreads / kWarp; ++w) sum += red[w];
-    *partial_out = sum;
+  double sum = 0.0;
+  if (threadIdx.x < kWarp) {
+#pragma unroll
+    for (int w = 0; w < kSolveWarps; ++w) sum += red[w];
+  }
+  return sum;
+}
+
+// out[k] = the blocks' partials of k < count in order (the whole block).
+__device__ __forceinline__ void add_partials(const double* partial, int count, double* out) {
+  const int lane = threadIdx.x & (kWarp - 1);
+  for (int k = threadIdx.x / kWarp; k < count; k += kSolveWarps) {
+    double acc = 0.0;
+    for (int b = lane; b < static_cast<int>(gridDim.x); b += kWarp)
+      acc += __ldcg(partial + static_cast<size_t>(k) * gridDim.x + b);
+    acc = group_sum<kWarp>(acc, 0xffffffffu);
+    if (lane == 0) out[k] = acc;
+  }
+  __syncthreads();
+}
+
+// r = b - A x into w[0] and its norm (First: x = 0, so r = b): opens a cycle.
+template <bool First>
+__global__ void __launch_bounds__(kSolveThreads) residual_kernel(SolveArgs a, int report) {
+  constexpr int G = kProductLanes;
+  const int l = threadIdx.x & (G - 1);
+  const index_t rows = static_cast<index_t>(gridDim.x * (kSolveThreads / G));
+  double acc = 0.0;
+  SolveArgs plain = a;
+  plain.dinv = nullptr;
+  for (index_t row = static_cast<index_t>((blockIdx.x * kSolveThreads + threadIdx.x) / G); row < a.n; row += rows) {
+    double r = a.b[row];
+    if (First) {
+      if (l == 0) a.x[row] = 0.0;
+    } else {
+      r -= row_product<G>(plain, row, l, a.x);
+    }
+    if (l == 0) {
+      a.w[0][row] = r;
+      acc = fma(r, r, acc);
+    }
+  }
+  const double sum = block_sum(acc);
+  if (threadIdx.x == 0) a.partial[blockIdx.x] = sum;
+  SolveState* st = a.st;
+  if (!last_block(st)) return;
+  __shared__ double total;
+  add_partials(a.partial, 1, &total);
+  if (threadIdx.x != 0) return;
+  const double beta = sqrt(total);
+  if (report) {  // the solve's first residual
+    st->beta0 = beta;
+    st->target = a.relative ? a.tolerance * beta : a.tolerance;
+    st->iters = 0;
+  }
+  st->beta = beta;
+  st->scale = 1.0 / beta;
+  st->steps = 0;
+  st->g[0] = beta;
+  st->converged = beta <= st->target ? 1 : 0;
+  st->stop = st->converged || st->iters >= a.max_iters;
+}
+
+// Step j: v_j = scale w[j & 1] into the basis, w[(j + 1) & 1] = A v_j.
+__global__ void __launch_bounds__(kSolveThreads) product_kernel(SolveArgs a, int j) {
+  const SolveState* st = a.st;
+  if (st->stop) return;
+  const double scale = st->scale;
+  const index_t row = static_cast<index_t>((static_cast<long long>(blockIdx.x) * kSolveThreads + threadIdx.x) / kProductLanes);
+  const int l = threadIdx.x & (kProductLanes - 1);
+  if (row >= a.n) return;  // the whole group
+  const double* __restrict__ from = a.w[j & 1];
+  const double w = scale * row_product<kProductLanes>(a, row, l, from);
+  if (l == 0) {
+    a.V[static_cast<size_t>(j) * a.ldv + row] = scale * from[row];
+    a.w[(j + 1) & 1][row] = w;
   }
 }
 
-// partial[k * gridDim.x + bx] = sum over this block's slice of v_k[i] * w[i],
-// k = blockIdx.y.  V is [k][ldv].
-__global__ void __launch_bounds__(kSolveThreads)
-    dots_kernel(index_t n, const double* __restrict__ V, size_t ldv, const double* __restrict__ w,
-                double* __restrict__ partial) {
-  const double* v = V + blockIdx.y * ldv;
-  double acc = 0.0;
-  for (index_t i = blockIdx.x * kSolveThreads + threadIdx.x; i < n; i += gridDim.x * kSolveThreads)
-    acc += v[i] * w[i];
-  block_partial(acc, partial + static_cast<size_t>(blockIdx.y) * gridDim.x + blockIdx.x);
-}
-
-// out[k] (+)= sum of partial[k][0..nb) in order; one block per k.
-__global__ void __launch_bounds__(kSolveThreads)
-    reduce_kernel(const double* __restrict__ partial, int nb, double* __restrict__ out, int accumulate) {
-  double acc = 0.0;
-  for (int b = threadIdx.x; b < nb; b += kSolveThreads) acc += partial[static_cast<size_t>(blockIdx.x) * nb + b];
-  __shared__ double red[kSolveThreads / kWarp];
-  for (int d = 16; d > 0; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
-  if ((threadIdx.x & (kWarp - 1)) == 0) red[threadIdx.x / kWarp] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double sum = 0.0;
-    for (int w = 0; w < kSolveThreads / kWarp; ++w) sum += red[w];
-    out[blockIdx.x] = accumulate ? out[blockIdx.x] + sum : sum;
+// The same with the product's dot products with v_0 .. v_j, for systems whose
+// matrix stays in L2: a row's eight lanes take the basis vectors lane, lane + 8,
+// ..., and the four rows of a warp read whole sectors of them.  8,000 rows: 10
+// us against 7 + 5 in two kernels; 61,250: 31 against 23 + 8; 500,000: 181
+// against 138 + 14 (the vectors' loads hold up the row's).
+template <int Dots>
+__global__ void __launch_bounds__(kSolveThreads) product_dots_kernel(SolveArgs a, int j) {
+  SolveState* st = a.st;
+  if (st->stop) return;
+  const double scale = st->scale;
+  const int l = threadIdx.x & (kRowLanes - 1);
+  const double* __restrict__ from = a.w[j & 1];
+  double* __restrict__ to = a.w[(j + 1) & 1];
+  double* __restrict__ vj = a.V + static_cast<size_t>(j) * a.ldv;
+  const index_t rows = static_cast<index_t>(gridDim.x * (kSolveThreads / kRowLanes));
+  double acc[Dots];
+#pragma unroll
+  for (int d = 0; d < Dots; ++d) acc[d] = 0.0;
+  for (index_t row = static_cast<index_t>((blockIdx.x * kSolveThreads + threadIdx.x) / kRowLanes); row < a.n;
+       row += rows) {
+    const double own = scale * from[row];
+    double v[Dots];
+#pragma unroll
+    for (int d = 0; d < Dots; ++d) {
+      const int k = d * kRowLanes + l;
+      v[d] = k < j ? a.V[static_cast<size_t>(k) * a.ldv + row] : k == j ? own : 0.0;
+    }
+    const double w = scale * row_product<kRowLanes>(a, row, l, from);
+    if (l == 0) {
+      vj[row] = own;
+      to[row] = w;
+    }
+#pragma unroll
+    for (int d = 0; d < Dots; ++d) acc[d] = fma(v[d], w, acc[d]);
   }
+  // over the warp's four rows, then the block's warps
+  __shared__ double s_dot[kSolveWarps][kRowLanes * Dots];
+#pragma unroll
+  for (int d = 0; d < Dots; ++d) {
+    acc[d] += __shfl_xor_sync(0xffffffffu, acc[d], 8);
+    acc[d] += __shfl_xor_sync(0xffffffffu, acc[d], 16);
+    if ((threadIdx.x & (kWarp - 1)) < kRowLanes) s_dot[threadIdx.x / kWarp][d * kRowLanes + l] = acc[d];
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k <= j; k += kSolveThreads) {
+    double sum = 0.0;
+#pragma unroll
+    for (int w = 0; w < kSolveWarps; ++w) sum += s_dot[w][k];
+    a.partial[static_cast<size_t>(k) * gridDim.x + blockIdx.x] = sum;
+  }
+  if (!last_block(st)) return;
+  add_partials(a.partial, j + 1, st->h);
 }
 
-// w -= sum_{k<kc} h[k] v_k; partial[bx] = this block's sum of w^2.
-__global__ void __launch_bounds__(kSolveThreads)
-    update_kernel(index_t n, const double* __restrict__ V, size_t ldv, int kc, const double* __restrict__ h,
-                  double* __restrict__ w, double* __restrict__ partial) {
-  __shared__ double sh[kMaxRestart + 1];
-  for (int k = threadIdx.x; k < kc; k += kSolveThreads) sh[k] = h[k];
-  __syncthreads();
-  double acc = 0.0;
-  for (index_t i = blockIdx.x * kSolveThreads + threadIdx.x; i < n; i += gridDim.x * kSolveThreads) {
+// Update: w -= sum_k h[k] v_k, and the remainder's dot products with the same
+// vectors (their values are still in registers) into h2, the second projection
+// of CGS2; else w's dot products into h, the first.  K: the most vectors this
+// instance holds.
+template <int K, bool Update>
+__global__ void __launch_bounds__(kSolveThreads) project_kernel(SolveArgs a, int j) {
+  SolveState* st = a.st;
+  if (st->stop) return;
+  __shared__ double sh[K];
+  __shared__ double s_dot[kSolveWarps][K];
+  if (Update) {
+    for (int k = threadIdx.x; k < K; k += kSolveThreads) sh[k] = k <= j ? st->h[k] : 0.0;
+    __syncthreads();
+  }
+  double* __restrict__ w = a.w[(j + 1) & 1];
+  double acc[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) acc[k] = 0.0;
+  for (index_t i = blockIdx.x * kSolveThreads + threadIdx.x; i < a.n; i += gridDim.x * kSolveThreads) {
+    double v[K];
     double wi = w[i];
-    for (int k = 0; k < kc; ++k) wi -= sh[k] * V[k * ldv + i];
-    w[i] = wi;
-    acc += wi * wi;
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = k <= j ? a.V[static_cast<size_t>(k) * a.ldv + i] : 0.0;
+    if (Update) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) wi = fma(-sh[k], v[k], wi);
+      w[i] = wi;
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) acc[k] = fma(v[k], wi, acc[k]);
   }
-  block_partial(acc, partial + blockIdx.x);
-}
-
-// v = w * scale
-__global__ void __launch_bounds__(kSolveThreads)
-    scale_kernel(index_t n, const double* w, double scale, double* v) {  // v may alias w
-  for (index_t i = blockIdx.x * kSolveThreads + threadIdx.x; i < n; i += gridDim.x * kSolveThreads)
-    v[i] = w[i] * scale;
-}
-
-// x += s ∘ (sum_{k<kc} y[k] v_k)  (s = NULL: no scaling)
-__global__ void __launch_bounds__(kSolveThreads)
-    correct_kernel(index_t n, const double* __restrict__ V, size_t ldv, int kc, const double* __restrict__ y,
-                   const double* __restrict__ s, double* __restrict__ x) {
-  __shared__ double sy[kMaxRestart + 1];
-  for (int k = threadIdx.x; k < kc; k += kSolveThreads) sy[k] = y[k];
+  int base = 0, count = K;
+  lane_totals<K, 16>(acc, base, count);
+#pragma unroll
+  for (int k = 0; k < lane_totals_left(K, 16); ++k)
+    if (k < count) s_dot[threadIdx.x / kWarp][base + k] = acc[k];
   __syncthreads();
-  for (index_t i = blockIdx.x * kSolveThreads + threadIdx.x; i < n; i += gridDim.x * kSolveThreads) {
-    double u = 0.0;
-    for (int k = 0; k < kc; ++k) u += sy[k] * V[k * ldv + i];
-    x[i] += s ? s[i] * u : u;
+  for (int k = threadIdx.x; k <= j; k += kSolveThreads) {
+    double sum = 0.0;
+#pragma unroll
+    for (int q = 0; q < kSolveWarps; ++q) sum += s_dot[q][k];
+    a.partial[static_cast<size_t>(k) * gridDim.x + blockIdx.x] = sum;
   }
+  if (!last_block(st)) return;
+  add_partials(a.partial, j + 1, Update ? st->h2 : st->h);
 }
 
-// r = b - Ax (Ax in r on entry), v0 = r; partial[bx] = block sum of r^2.
-__global__ void __launch_bounds__(kSolveThreads)
-    residual_kernel(index_t n, const double* __restrict__ b, double* __restrict__ r, double* __restrict__ partial) {
+// w -= sum_k h2[k] v_k and its norm; the last block extends the Hessenberg
+// matrix by column j and applies the previous rotations and the one that zeroes
+// its subdiagonal.
+template <int K>
+__global__ void __launch_bounds__(kSolveThreads) extend_kernel(SolveArgs a, int j) {
+  SolveState* st = a.st;
+  if (st->stop) return;
+  __shared__ double sh[kMaxRestart + 1];
+  for (int k = threadIdx.x; k <= j; k += kSolveThreads) sh[k] = st->h2[k];
+  __syncthreads();
+  double* __restrict__ w = a.w[(j + 1) & 1];
   double acc = 0.0;
-  for (index_t i = blockIdx.x * kSolveThreads + threadIdx.x; i < n; i += gridDim.x * kSolveThreads) {
-    const double ri = b[i] - r[i];
-    r[i] = ri;
-    acc += ri * ri;
+  for (index_t i = blockIdx.x * kSolveThreads + threadIdx.x; i < a.n; i += gridDim.x * kSolveThreads) {
+    double wi = w[i], v[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = k <= j ? a.V[static_cast<size_t>(k) * a.ldv + i] : 0.0;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (k <= j) wi = fma(-sh[k], v[k], wi);
+    w[i] = wi;
+    acc = fma(wi, wi, acc);
   }
-  block_partial(acc, partial + blockIdx.x);
+  const double sum = block_sum(acc);
+  if (threadIdx.x == 0) a.partial[blockIdx.x] = sum;
+  if (!last_block(st)) return;
+  __shared__ double total, col[kMaxRestart + 1], cs[kMaxRestart], sn[kMaxRestart];
+  add_partials(a.partial, 1, &total);
+  for (int k = threadIdx.x; k <= j; k += kSolveThreads) {
+    col[k] = st->h[k] + sh[k];
+    if (k < j) {
+      cs[k] = st->cs[k];
+      sn[k] = st->sn[k];
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const double hnext = sqrt(total);
+    for (int k = 0; k < j; ++k) {
+      const double t = cs[k] * col[k] + sn[k] * col[k + 1];
+      col[k + 1] = -sn[k] * col[k] + cs[k] * col[k + 1];
+      col[k] = t;
+    }
+    const double den = hypot(col[j], hnext);
+    const double c = den > 0.0 ? col[j] / den : 1.0;
+    const double s = den > 0.0 ? hnext / den : 0.0;
+    col[j] = den;
+    st->cs[j] = c;
+    st->sn[j] = s;
+    const double g = st->g[j];
+    st->g[j + 1] = -s * g;
+    st->g[j] = c * g;
+    st->scale = 1.0 / hnext;
+    st->steps = j + 1;
+    st->iters += 1;
+    // hnext == 0: the Krylov space is invariant (the correction solves the
+    // system on it); the cycle stops there.
+    if (fabs(s * g) <= st->target || hnext == 0.0 || st->iters >= a.max_iters) {
+      st->stop = 1;
+      *a.stopped = 1;
+    }
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k <= j; k += kSolveThreads) st->H[static_cast<size_t>(j) * (kMaxRestart + 1) + k] = col[k];
+}
+
+// y = R^-1 g (back substitution on the rotated Hessenberg, by the first warp of
+// each block), x += M^-1 V y.
+__global__ void __launch_bounds__(kSolveThreads) correct_kernel(SolveArgs a) {
+  const SolveState* st = a.st;
+  __shared__ double sy[kMaxRestart];
+  const int m = st->steps;
+  if (threadIdx.x < kWarp) {
+    const int lane = threadIdx.x;
+    double t[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) t[q] = lane + q * kWarp < m ? st->g[lane + q * kWarp] : 0.0;
+    for (int k = m - 1; k >= 0; --k) {
+      const double* __restrict__ col = st->H + static_cast<size_t>(k) * (kMaxRestart + 1);
+      const double tk = __shfl_sync(0xffffffffu, k < kWarp ? t[0] : t[1], k & (kWarp - 1));
+      const double d = col[k];
+      const double y = d != 0.0 ? tk / d : 0.0;
+      if (lane == 0) sy[k] = y;
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        if (lane + q * kWarp < k) t[q] = fma(-col[lane + q * kWarp], y, t[q]);
+    }
+  }
+  __syncthreads();
+  for (index_t i = blockIdx.x * kSolveThreads + threadIdx.x; i < a.n; i += gridDim.x * kSolveThreads) {
+    double u = 0.0;
+#pragma unroll 8
+    for (int k = 0; k < m; ++k) u = fma(sy[k], a.V[static_cast<size_t>(k) * a.ldv + i], u);
+    a.x[i] += a.dinv ? a.dinv[i] * u : u;
+  }
 }
 
 // dinv[i] = 1 / a_ii (1 where the row has no non-zero diagonal entry).
@@ -160,49 +419,51 @@ __global__ void __launch_bounds__(kSolveThreads) clamp_kernel(index_t n, double*
   if (i < n && x[i] < 0.0) x[i] = 0.0;
 }
 
-__global__ void __launch_bounds__(kSolveThreads) zero_kernel(index_t n, double* __restrict__ x) {
-  const index_t i = blockIdx.x * kSolveThreads + threadIdx.x;
-  if (i < n) x[i] = 0.0;
+// Launch shapes: blocks of the streaming passes, of the row passes.
+struct SolveShape {
+  int stream, rows;
+  bool fused;  // the first projection in the product
+};
+
+void launch_residual(lsmps_ctx* ctx, const SolveArgs& a, bool zero, bool report, const SolveShape& g) {
+  const auto queue = [&](const char* name, auto kernel) {
+    launch_named(ctx, name, kernel, dim3(g.rows), dim3(kSolveThreads), 0, a, report ? 1 : 0);
+  };
+  zero ? queue("residual_kernel<first>", residual_kernel<true>) : queue("residual_kernel", residual_kernel<false>);
 }
 
-struct Solver {
-  lsmps_ctx* ctx;
-  index_t n;
-  int nb;  // blocks of the streaming passes
-  const lsmps_csr_matrix* A;
-  const double* dinv;  // NULL without preconditioner
-  double* V;
-  size_t ldv;
-  double* w;
-  double* partial;  // [kMaxRestart + 1][nb]
-  double* dev_h;    // [2 * (kMaxRestart + 1) + 1]: h (first pass), h (second pass), |w|^2
-  double* host;     // pinned mirror of dev_h
+// Step j's passes over the basis with the smallest instances that hold its
+// j + 1 vectors.
+template <int K>
+void launch_projections(lsmps_ctx* ctx, const SolveArgs& a, int j, const SolveShape& g) {
+  const dim3 grid(g.stream), block(kSolveThreads);
+  if (!g.fused) launch_named(ctx, "project_kernel<first>", project_kernel<K, false>, grid, block, 0, a, j);
+  launch_named(ctx, "project_kernel", project_kernel<K, true>, grid, block, 0, a, j);
+  launch_named(ctx, "extend_kernel", extend_kernel<K>, grid, block, 0, a, j);
+}
 
-  dim3 grid1() const { return dim3(nb); }
-
-  void spmv(const double* x, double* y, bool precondition) {
-    launch(ctx, spmv_kernel<kSpmvLanes>, dim3(div_up(static_cast<long long>(n) * kSpmvLanes, kSolveThreads)),
-           dim3(kSolveThreads), 0, n, static_cast<const index_t*>(A->row_offsets),
-           static_cast<const index_t*>(A->col_indices), static_cast<const double*>(A->values), x,
-           precondition ? dinv : static_cast<const double*>(nullptr), y);
-  }
-
-  // |r|^2 of r = b - A x into dev_h[0] (and r), synchronously.
-  bool residual(const double* b, const double* x, double* r, double& norm2) {
-    spmv(x, r, false);
-    launch(ctx, residual_kernel, grid1(), dim3(kSolveThreads), 0, n, b, r, partial);
-    launch(ctx, reduce_kernel, dim3(1), dim3(kSolveThreads), 0, static_cast<const double*>(partial), nb, dev_h, 0);
-    if (!read(1)) return false;
-    norm2 = host[0];
-    return true;
-  }
-
-  bool read(int count) {
-    if (cudaMemcpyAsync(host, dev_h, count * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess)
-      return false;
-    return cudaStreamSynchronize(ctx->stream) == cudaSuccess;
-  }
-};
+void launch_step(lsmps_ctx* ctx, const SolveArgs& a, int j, const SolveShape& g) {
+  const auto product = [&](auto kernel) {
+    launch_named(ctx, "product_dots_kernel", kernel, dim3(g.rows), dim3(kSolveThreads), 0, a, j);
+  };
+  if (!g.fused)
+    launch(ctx, product_kernel, dim3(div_up(static_cast<long long>(a.n) * kProductLanes, kSolveThreads)),
+           dim3(kSolveThreads), 0, a, j);
+  else if (j < 8)
+    product(product_dots_kernel<1>);
+  else if (j < 24)
+    product(product_dots_kernel<3>);
+  else
+    product(product_dots_kernel<kMaxRestart / kRowLanes>);
+  if (j < 8)
+    launch_projections<8>(ctx, a, j, g);
+  else if (j < 16)
+    launch_projections<16>(ctx, a, j, g);
+  else if (j < 24)
+    launch_projections<24>(ctx, a, j, g);
+  else
+    launch_projections<kMaxRestart>(ctx, a, j, g);
+}
 
 }  // namespace
 
@@ -237,123 +498,75 @@ lsmps_status solve_ppe_impl(lsmps_ctx* ctx, const lsmps_csr_matrix& A, const dou
 
   const index_t n = static_cast<index_t>(A.rows);
   const int m = opt.restart;
-  const int nb = static_cast<int>(std::min<long long>(div_up(static_cast<long long>(n), kSolveThreads),
-                                                      4LL * ctx->sm_count));
+  // Streaming passes: up to four blocks per SM; passes over the rows that end
+  // in a sum: eight.
+  SolveShape g;
+  g.stream = static_cast<int>(std::min<long long>(div_up(static_cast<long long>(n), kSolveThreads), 4LL * ctx->sm_count));
+  g.rows = static_cast<int>(
+      std::min<long long>(div_up(static_cast<long long>(n) * kRowLanes, kSolveThreads), 8LL * ctx->sm_count));
+  g.fused = n <= kFusedRows;
   const size_t ldv = (static_cast<size_t>(n) + 31) & ~size_t(31);
+  const size_t partials = static_cast<size_t>(kMaxRestart + 1) * std::max(g.stream, g.rows);
   Scratch scratch(ctx);
-  const size_t need = (static_cast<size_t>(m + 1) * ldv + 2 * ldv) * sizeof(double) +
-                      static_cast<size_t>(kMaxRestart + 1) * nb * sizeof(double) +
-                      (2 * (kMaxRestart + 1) + 8) * sizeof(double) + 16 * 256;
+  const size_t need = (static_cast<size_t>(m) * ldv + 3 * ldv) * sizeof(double) + partials * sizeof(double) +
+                      sizeof(SolveState) + 16 * 256;
   if (!scratch.reserve(need)) return fail(ctx, LSMPS_CUDA_ERROR, "scratch allocation failed");
-  Solver s{};
-  s.ctx = ctx;
-  s.n = n;
-  s.nb = nb;
-  s.A = &A;
-  s.ldv = ldv;
-  s.V = scratch.take<double>(static_cast<size_t>(m + 1) * ldv);
-  s.w = scratch.take<double>(ldv);
+  SolveArgs a{};
+  a.n = n;
+  a.ro = A.row_offsets;
+  a.ci = A.col_indices;
+  a.va = A.values;
+  a.V = scratch.take<double>(static_cast<size_t>(m) * ldv);
+  a.ldv = ldv;
+  a.w[0] = scratch.take<double>(ldv);
+  a.w[1] = scratch.take<double>(ldv);
   double* dinv = scratch.take<double>(ldv);
-  s.partial = scratch.take<double>(static_cast<size_t>(kMaxRestart + 1) * nb);
-  s.dev_h = scratch.take<double>(2 * (kMaxRestart + 1) + 8);
-  if (!s.V || !s.w || !dinv || !s.partial || !s.dev_h) return fail(ctx, LSMPS_CUDA_ERROR, "scratch exhausted");
-  static thread_local double* pinned = nullptr;
-  if (!pinned && cudaMallocHost(&pinned, (2 * (kMaxRestart + 1) + 8) * sizeof(double)) != cudaSuccess) {
+  a.partial = scratch.take<double>(partials);
+  a.st = scratch.take<SolveState>(1);
+  if (!a.V || !a.w[0] || !a.w[1] || !dinv || !a.partial || !a.st)
+    return fail(ctx, LSMPS_CUDA_ERROR, "scratch exhausted");
+  // pinned: the state's leading scalars read back after a cycle, and the flag
+  // that the device sets when a cycle stops early
+  struct Pinned {
+    SolveState state;
+    volatile int stopped;
+  };
+  static thread_local Pinned* pinned = nullptr;
+  if (!pinned && cudaMallocHost(&pinned, sizeof(Pinned)) != cudaSuccess) {
     pinned = nullptr;
     return fail(ctx, LSMPS_CUDA_ERROR, "pinned allocation failed");
   }
-  s.host = pinned;
-  const bool jacobi = opt.preconditioner == LSMPS_PRECONDITIONER_JACOBI;
-  if (jacobi) {
-    launch(ctx, jacobi_kernel, dim3(div_up(n, kSolveThreads)), dim3(kSolveThreads), 0, n,
-           static_cast<const index_t*>(A.row_offsets), static_cast<const index_t*>(A.col_indices),
-           static_cast<const double*>(A.values), dinv);
-    s.dinv = dinv;
+  a.stopped = &pinned->stopped;
+  a.x = x;
+  a.b = b;
+  a.restart = m;
+  a.max_iters = opt.max_iters;
+  a.tolerance = opt.tolerance;
+  a.relative = opt.convergence == LSMPS_CONVERGENCE_RELATIVE_INITIAL;
+  if (opt.preconditioner == LSMPS_PRECONDITIONER_JACOBI) {
+    launch(ctx, jacobi_kernel, dim3(div_up(n, kSolveThreads)), dim3(kSolveThreads), 0, n, a.ro, a.ci, a.va, dinv);
+    a.dinv = dinv;
   }
-  if (!opt.use_initial_guess) launch(ctx, zero_kernel, dim3(div_up(n, kSolveThreads)), dim3(kSolveThreads), 0, n, x);
-
-  // r0 = b - A x0 in V[0]
-  double beta2 = 0.0;
-  if (!s.residual(b, x, s.V, beta2)) return check_launch(ctx, "PPE solve");
-  const double beta0 = std::sqrt(beta2);
-  const double target = opt.convergence == LSMPS_CONVERGENCE_RELATIVE_INITIAL ? opt.tolerance * beta0 : opt.tolerance;
-  double beta = beta0;
-  int iters = 0;
-  bool converged = beta <= target;
-  std::vector<double> H(static_cast<size_t>(m + 1) * m), cs(m), sn(m), g(m + 1), y(m + 1);
-  while (!converged && iters < opt.max_iters) {
-    // V[0] = r / beta
-    launch(ctx, scale_kernel, s.grid1(), dim3(kSolveThreads), 0, n, static_cast<const double*>(s.V), 1.0 / beta, s.V);
-    std::fill(g.begin(), g.end(), 0.0);
-    g[0] = beta;
-    int j = 0;
-    for (; j < m && iters < opt.max_iters; ++j) {
-      double* vj = s.V + static_cast<size_t>(j) * ldv;
-      s.spmv(vj, s.w, jacobi);
-      const int kc = j + 1;
-      // CGS2: two passes of h = V^T w, w -= V h; the second pass also gives |w|^2.
-      for (int pass = 0; pass < 2; ++pass) {
-        double* hp = s.dev_h + pass * (kMaxRestart + 1);
-        launch(ctx, dots_kernel, dim3(nb, kc), dim3(kSolveThreads), 0, n, static_cast<const double*>(s.V), ldv,
-               static_cast<const double*>(s.w), s.partial);
-        launch(ctx, reduce_kernel, dim3(kc), dim3(kSolveThreads), 0, static_cast<const double*>(s.partial), nb, hp, 0);
-        launch(ctx, update_kernel, s.grid1(), dim3(kSolveThreads), 0, n, static_cast<const double*>(s.V), ldv, kc,
-               static_cast<const double*>(hp), s.w, s.partial);
-      }
-      launch(ctx, reduce_kernel, dim3(1), dim3(kSolveThreads), 0, static_cast<const double*>(s.partial), nb,
-             s.dev_h + 2 * (kMaxRestart + 1), 0);
-      if (cudaMemcpyAsync(s.host, s.dev_h, (2 * (kMaxRestart + 1) + 1) * sizeof(double), cudaMemcpyDeviceToHost,
-                          ctx->stream) != cudaSuccess ||
-          cudaStreamSynchronize(ctx->stream) != cudaSuccess)
-        return check_launch(ctx, "PPE solve");
-      ++iters;
-      double* col = &H[static_cast<size_t>(j) * (m + 1)];
-      for (int k = 0; k <= j; ++k) col[k] = s.host[k] + s.host[kMaxRestart + 1 + k];
-      const double hnext = std::sqrt(s.host[2 * (kMaxRestart + 1)]);
-      col[j + 1] = hnext;
-      // previous rotations, then the one that zeroes col[j + 1]
-      for (int k = 0; k < j; ++k) {
-        const double t = cs[k] * col[k] + sn[k] * col[k + 1];
-        col[k + 1] = -sn[k] * col[k] + cs[k] * col[k + 1];
-        col[k] = t;
-      }
-      const double den = std::hypot(col[j], col[j + 1]);
-      cs[j] = den > 0.0 ? col[j] / den : 1.0;
-      sn[j] = den > 0.0 ? col[j + 1] / den : 0.0;
-      col[j] = den;
-      col[j + 1] = 0.0;
-      g[j + 1] = -sn[j] * g[j];
-      g[j] = cs[j] * g[j];
-      const double estimate = std::fabs(g[j + 1]);
-      // hnext == 0: the Krylov space is invariant (the update below solves
-      // the system on it); stop the cycle there.
-      if (estimate <= target || hnext == 0.0) {
-        ++j;
-        break;
-      }
-      if (j + 1 < m && iters < opt.max_iters)
-        launch(ctx, scale_kernel, s.grid1(), dim3(kSolveThreads), 0, n, static_cast<const double*>(s.w),
-               1.0 / hnext, s.V + static_cast<size_t>(j + 1) * ldv);
-    }
-    // y = R^-1 g (back substitution on the rotated Hessenberg), x += M^-1 V y
-    for (int k = j - 1; k >= 0; --k) {
-      double t = g[k];
-      for (int c = k + 1; c < j; ++c) t -= H[static_cast<size_t>(c) * (m + 1) + k] * y[c];
-      const double d = H[static_cast<size_t>(k) * (m + 1) + k];
-      y[k] = d != 0.0 ? t / d : 0.0;
-    }
-    for (int k = 0; k < j; ++k) s.host[k] = y[k];
-    if (cudaMemcpyAsync(s.dev_h, s.host, j * sizeof(double), cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
-      return check_launch(ctx, "PPE solve");
-    launch(ctx, correct_kernel, s.grid1(), dim3(kSolveThreads), 0, n, static_cast<const double*>(s.V), ldv, j,
-           static_cast<const double*>(s.dev_h), static_cast<const double*>(s.dinv), x);
-    // true residual for the next cycle (and the report)
-    if (!s.residual(b, x, s.V, beta2)) return check_launch(ctx, "PPE solve");
-    beta = std::sqrt(beta2);
-    converged = beta <= target;
+  cudaMemsetAsync(&a.st->tickets, 0, sizeof(unsigned), ctx->stream);
+  launch_residual(ctx, a, !opt.use_initial_guess, true, g);
+  const SolveState& st = pinned->state;
+  const auto read = [&]() {
+    return cudaMemcpyAsync(&pinned->state, a.st, offsetof(SolveState, tickets), cudaMemcpyDeviceToHost, ctx->stream) ==
+               cudaSuccess &&
+           cudaStreamSynchronize(ctx->stream) == cudaSuccess;
+  };
+  // The first cycle is queued without waiting for the first residual: a system
+  // that starts converged lets its launches return at once.
+  for (;;) {
+    pinned->stopped = 0;
+    for (int j = 0; j < m && !pinned->stopped; ++j) launch_step(ctx, a, j, g);
+    launch(ctx, correct_kernel, dim3(g.stream), dim3(kSolveThreads), 0, a);
+    launch_residual(ctx, a, false, false, g);
+    if (!read()) return check_launch(ctx, "PPE solve");
+    if (st.converged || st.iters >= opt.max_iters) break;
   }
   if (opt.clamp_negative) launch(ctx, clamp_kernel, dim3(div_up(n, kSolveThreads)), dim3(kSolveThreads), 0, n, x);
-  if (report) *report = lsmps_solver_report{iters, converged ? 1 : 0, beta0, beta};
+  if (report) *report = lsmps_solver_report{st.iters, st.converged ? 1 : 0, st.beta0, st.beta};
   return check_launch(ctx, "PPE solve");
 }
 

@@ -117,10 +117,11 @@ def solve_kernel_bytes(rows: int, nnz: int, restart: int = 20, s: int = 8) -> di
     vec = s * rows
     avg_basis = (restart + 1) / 2.0
     return {
-        "spmv_kernel<kSpmvLanes>": 4 * (rows + 1) + (4 + s) * nnz + 2 * vec,
-        "dots_kernel": int(vec * (avg_basis + 1)),
-        "update_kernel": int(vec * (avg_basis + 2)),
-        "scale_kernel": 2 * vec,
+        "product_kernel": 4 * (rows + 1) + (4 + s) * nnz + 3 * vec,
+        "product_dots_kernel": 4 * (rows + 1) + (4 + s) * nnz + int(vec * (avg_basis + 2)),
+        "project_kernel<first>": int(vec * (avg_basis + 1)),
+        "project_kernel": int(vec * (avg_basis + 2)),
+        "extend_kernel": int(vec * (avg_basis + 2)),
         "correct_kernel": int(vec * (restart + 2)),
-        "residual_kernel": 2 * vec,
+        "residual_kernel": 4 * (rows + 1) + (4 + s) * nnz + 3 * vec,
     }
