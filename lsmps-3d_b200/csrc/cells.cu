@@ -1,18 +1,20 @@
-// cells.cu - cell list of one particle set: cell hash, stable LSD radix sort
-// of (cell id, particle index), cell ranges.  Replaces build_cell_list_impl of
-// src/neighbor/neighbor_search.cu:255-292, whose Thrust sort_by_key is a
-// stable radix sort; this sort is stable too, so the particles of a cell keep
-// ascending index order and cell_ids / sorted_indices / cell_begin / cell_end
-// are identical to the reference's.
+// cells.cu - cell lists of one or two particle sets: each set's particles by
+// cell, ascending index inside a cell, and every cell's range.  Replaces
+// build_cell_list_impl of src/neighbor/neighbor_search.cu:255-292, whose Thrust
+// sort_by_key of (cell id, particle index) is stable, so that cell_ids /
+// sorted_indices / cell_begin / cell_end are identical to the reference's.
 //
-// The sort is reduce-then-scan per 8-bit digit: a per-tile digit histogram,
-// one device-wide exclusive scan of the digit-major histogram table, and a
-// scatter that ranks each key stably inside its tile with warp match masks.
-// No block waits on another block.
+// A counting sort, both sets in the same launches: every particle takes a
+// number in its cell (in no particular order), the cells' counts are scanned
+// into ranges, the particles are put there by number, and each cell's few
+// particles are then ordered by index.  No block waits on another.  The
+// radix-sort kernels at the end of the kernels' list are those of the
+// allocation-free entry point (cells_noalloc.cu).
 #include <climits>
 #include <cmath>
 
 #include "cells.cuh"
+#include "scan.cuh"
 
 namespace lsmps {
 namespace {
@@ -54,33 +56,6 @@ __global__ void hash_kernel(const double* __restrict__ x, const double* __restri
       const index_t iz = cell_coord(z[t], grid.origin[2], grid.cell_size, grid.dims[2], bad);
       if (bad) raise_flag(status, kFlagNonFinite);
       keys[t] = (iz * grid.dims[1] + iy) * grid.dims[0] + ix;  // flatten_cell, :32-34
-      vals[t] = t;
-    }
-  }
-}
-
-// hash_kernel for a merged batch: particle t belongs to the box whose range
-// of this set holds it (field 1: fluid, 2: walls) and is hashed on that box's
-// grid (cell size shared), offset by the box's first global cell.
-__global__ void hash_boxes_kernel(const double* __restrict__ x, const double* __restrict__ y,
-                                  const double* __restrict__ z, index_t n, const BoxGrid* __restrict__ boxes,
-                                  int nbox, int field, double cell_size, index_t* __restrict__ keys,
-                                  index_t* __restrict__ vals, index_t* __restrict__ cell_begin,
-                                  index_t* __restrict__ cell_end, index_t ncell, DeviceStatus* __restrict__ status) {
-  const index_t total = n > ncell ? n : ncell;
-  for (index_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    if (t < ncell) {
-      cell_begin[t] = -1;
-      cell_end[t] = -1;
-    }
-    if (t < n) {
-      const BoxGrid& g = boxes[box_of(boxes, nbox, t, field)];
-      bool bad = false;
-      const index_t ix = cell_coord(x[t], g.origin[0], cell_size, g.dims[0], bad);
-      const index_t iy = cell_coord(y[t], g.origin[1], cell_size, g.dims[1], bad);
-      const index_t iz = cell_coord(z[t], g.origin[2], cell_size, g.dims[2], bad);
-      if (bad) raise_flag(status, kFlagNonFinite);
-      keys[t] = g.cell_base + (iz * g.dims[1] + iy) * g.dims[0] + ix;
       vals[t] = t;
     }
   }
@@ -165,6 +140,158 @@ __global__ void ranges_kernel(const index_t* __restrict__ keys, index_t n, index
   }
 }
 
+namespace {
+
+constexpr int kCellThreads = 256;
+
+// One or two sets as one index range: set s's particles at first[s] .., its
+// cells' counts at s * ncell ...
+struct CellArgs {
+  CellSet set[2];
+  int sets;
+  index_t first1;  // particles of set 0
+  index_t total;   // of both
+  lsmps_grid grid;
+  index_t ncell;
+  const BoxGrid* boxes;
+  int nbox;
+  index_t* key;     // [total] cell of each particle
+  index_t* number;  // [total] its number in the cell
+  index_t* count;   // [sets * ncell] particles per cell, then the cells' first positions
+  index_t* placed;  // [total] particles by cell, unordered inside a cell
+  DeviceStatus* status;
+};
+
+// assign_cells_kernel (neighbor_search.cu:61-73) of both sets, with the count
+// of every cell.  In a merged batch a particle is hashed on the grid of the box
+// whose range of its set holds it.
+__global__ void __launch_bounds__(kCellThreads) cell_count_kernel(CellArgs a) {
+  for (index_t p = blockIdx.x * kCellThreads + threadIdx.x; p < a.total; p += gridDim.x * kCellThreads) {
+    const int s = p >= a.first1 ? 1 : 0;
+    const CellSet& set = a.set[s];
+    const index_t t = p - (s ? a.first1 : 0);
+    double o[3] = {a.grid.origin[0], a.grid.origin[1], a.grid.origin[2]};
+    index_t d[3] = {a.grid.dims[0], a.grid.dims[1], a.grid.dims[2]}, base = 0;
+    if (a.boxes) {
+      const BoxGrid& g = a.boxes[box_of(a.boxes, a.nbox, t, set.box_field)];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        o[k] = g.origin[k];
+        d[k] = g.dims[k];
+      }
+      base = g.cell_base;
+    }
+    bool bad = false;
+    const index_t ix = cell_coord(set.x[t], o[0], a.grid.cell_size, d[0], bad);
+    const index_t iy = cell_coord(set.y[t], o[1], a.grid.cell_size, d[1], bad);
+    const index_t iz = cell_coord(set.z[t], o[2], a.grid.cell_size, d[2], bad);
+    if (bad) raise_flag(a.status, kFlagNonFinite);
+    const index_t key = base + (iz * d[1] + iy) * d[0] + ix;  // flatten_cell, :32-34
+    a.key[p] = key;
+    a.number[p] = atomicAdd(&a.count[static_cast<size_t>(s) * a.ncell + key], 1);
+  }
+}
+
+// Cell c's range from its count and the sum of the counts before it (both
+// sets' cells in one scan; set 1's positions start at 0 again).
+__device__ __forceinline__ void store_range(const CellArgs& a, size_t c, long long before, index_t count) {
+  const int s = c >= static_cast<size_t>(a.ncell) ? 1 : 0;
+  const index_t first = static_cast<index_t>(before - (s ? a.first1 : 0));
+  const size_t at = c - (s ? static_cast<size_t>(a.ncell) : 0);
+  a.count[c] = first;
+  a.set[s].begin[at] = count ? first : -1;
+  a.set[s].end[at] = count ? first + count : -1;
+}
+
+__global__ void __launch_bounds__(kSmallScanThreads) cell_ranges_small_kernel(CellArgs a) {
+  scan_small(
+      a.sets * a.ncell, [&](int i) { return a.count[i]; },
+      [&](int i, long long before, index_t v) { store_range(a, i, before, v); });
+}
+
+__global__ void __launch_bounds__(kScanThreads) cell_totals_kernel(CellArgs a, long long* __restrict__ partials) {
+  const long long t = tile_sum(static_cast<size_t>(a.sets) * a.ncell, [&](size_t i) { return a.count[i]; });
+  if (threadIdx.x == 0) partials[blockIdx.x] = t;
+}
+
+__global__ void __launch_bounds__(kScanThreads) cell_ranges_kernel(CellArgs a, const long long* __restrict__ partials,
+                                                                  int scanned) {
+  scan_tile(
+      static_cast<size_t>(a.sets) * a.ncell, before_tile(partials, scanned != 0), [&](size_t i) { return a.count[i]; },
+      [&](size_t i, long long before, index_t v) { store_range(a, i, before, v); });
+}
+
+__global__ void __launch_bounds__(kCellThreads) cell_place_kernel(CellArgs a) {
+  for (index_t p = blockIdx.x * kCellThreads + threadIdx.x; p < a.total; p += gridDim.x * kCellThreads) {
+    const int s = p >= a.first1 ? 1 : 0;
+    const index_t first = s ? a.first1 : 0;
+    a.placed[first + a.count[static_cast<size_t>(s) * a.ncell + a.key[p]] + a.number[p]] = p - first;
+  }
+}
+
+// A cell of more particles than this is ordered by a walk over the whole set
+// instead of by comparing its particles with one another.
+constexpr index_t kManyInCell = 1024;
+
+// Orders the particles of cell c of set s by index (one warp), writes its
+// stretch of the sorted list and, where asked for, the sorted positions.
+__device__ __forceinline__ void order_cell(const CellArgs& a, const CellSet& set, index_t first, index_t n, index_t c,
+                                           index_t b, index_t e) {
+  const int lane = threadIdx.x & (kWarp - 1);
+  const index_t* __restrict__ placed = a.placed + first;
+  const auto put = [&](index_t at, index_t i) {
+    set.sorted[at] = i;
+    set.ids[at] = c;
+    if (set.pos) set.pos[at] = make_double4(set.x[i], set.y[i], set.z[i], 0.0);
+  };
+  const index_t many = e - b;
+  if (many <= kWarp) {
+    const index_t v = lane < many ? placed[b + lane] : INT_MAX;
+    index_t rank = 0;
+    for (index_t k = 0; k < many; ++k) rank += __shfl_sync(0xffffffffu, v, k) < v ? 1 : 0;
+    if (lane < many) put(b + rank, v);
+  } else if (many <= kManyInCell) {
+    for (index_t k = b + lane; k < e; k += kWarp) {
+      const index_t v = placed[k];
+      index_t rank = 0;
+      for (index_t q = b; q < e; ++q) rank += placed[q] < v ? 1 : 0;
+      put(b + rank, v);
+    }
+  } else {
+    index_t at = b;
+    for (index_t k = 0; k < n; k += kWarp) {
+      const bool mine = k + lane < n && a.key[first + k + lane] == c;
+      const unsigned in = __ballot_sync(0xffffffffu, mine);
+      if (mine) put(at + __popc(in & ((1u << lane) - 1u)), k + lane);
+      at += __popc(in);
+    }
+  }
+}
+
+// Each warp orders the non-empty ones of `span` (1 .. 32) consecutive cells.
+__global__ void __launch_bounds__(kCellThreads) cell_order_kernel(CellArgs a, int span) {
+  const int lane = threadIdx.x & (kWarp - 1);
+  const long long cells = static_cast<long long>(a.sets) * a.ncell;
+  const long long warps = static_cast<long long>(gridDim.x) * (kCellThreads / kWarp);
+  for (long long g = static_cast<long long>(blockIdx.x) * (kCellThreads / kWarp) + threadIdx.x / kWarp;
+       g * span < cells; g += warps) {
+    const long long c = g * span + lane;
+    const bool mine = lane < span && c < cells;
+    const int s = c >= a.ncell ? 1 : 0;
+    const index_t at = static_cast<index_t>(c - (s ? a.ncell : 0));
+    const index_t b = mine ? a.set[s].begin[at] : -1, e = mine ? a.set[s].end[at] : -1;
+    for (unsigned rem = __ballot_sync(0xffffffffu, b >= 0); rem; rem &= rem - 1) {
+      const int k = __ffs(rem) - 1;
+      const int sk = __shfl_sync(0xffffffffu, s, k);
+      const index_t ck = __shfl_sync(0xffffffffu, at, k), bk = __shfl_sync(0xffffffffu, b, k),
+                    ek = __shfl_sync(0xffffffffu, e, k);
+      order_cell(a, a.set[sk], sk ? a.first1 : 0, sk ? a.total - a.first1 : a.first1, ck, bk, ek);
+    }
+  }
+}
+
+}  // namespace
+
 int key_bits(long long ncell) {
   int bits = 0;
   while ((1LL << bits) < ncell) ++bits;
@@ -180,18 +307,12 @@ lsmps_status validate_grid(lsmps_ctx* ctx, const lsmps_grid& grid) {
 }
 
 size_t cell_list_scratch_bytes(size_t n, size_t ncell) {
-  (void)ncell;
-  const size_t tiles = (n + kSortTile - 1) / kSortTile + 1;
-  // ping-pong keys and values, the histogram table, and one scan per pass
-  return 2 * (n * sizeof(index_t) + 256) + tiles * kRadixBins * sizeof(index_t) + 256 +
-         4 * scan_scratch_bytes(tiles * kRadixBins) + 4096;
+  // keys, numbers and placed particles; the cells' counts; their scan
+  return 3 * (n * sizeof(index_t) + 256) + ncell * sizeof(index_t) + scan_scratch_bytes(ncell) + 4096;
 }
 
-lsmps_status build_cell_list_impl(lsmps_ctx* ctx, Scratch& scratch, const double* x, const double* y,
-                                  const double* z, size_t count, const lsmps_grid& grid,
-                                  const lsmps_cells& cells, const BoxGrid* boxes, int box_field) {
-  lsmps_status st = validate_grid(ctx, grid);
-  if (st) return st;
+lsmps_status check_cell_set(lsmps_ctx* ctx, const CellSet& set, size_t count, const lsmps_grid& grid,
+                            const lsmps_cells& cells) {
   const long long ncell = static_cast<long long>(grid.dims[0]) * grid.dims[1] * grid.dims[2];
   if (static_cast<size_t>(ncell) != cells.cell_count)
     return fail(ctx, LSMPS_INVALID_ARGUMENT, "Cell list capacity does not match grid cell count");
@@ -199,44 +320,72 @@ lsmps_status build_cell_list_impl(lsmps_ctx* ctx, Scratch& scratch, const double
     return fail(ctx, LSMPS_INVALID_ARGUMENT, "Cell list particle capacity is smaller than particle count");
   if (count > static_cast<size_t>(INT_MAX))
     return fail(ctx, LSMPS_INDEX_OVERFLOW, "Particle count exceeds 32-bit index capacity");
-  if (!cells.cell_begin || !cells.cell_end || (count && (!cells.cell_ids || !cells.sorted_indices || !x || !y || !z)))
+  if (!cells.cell_begin || !cells.cell_end ||
+      (count && (!cells.cell_ids || !cells.sorted_indices || !set.x || !set.y || !set.z)))
     return fail(ctx, LSMPS_INVALID_ARGUMENT, "cell list buffers missing");
-  const index_t n = static_cast<index_t>(count);
-  const int passes = (key_bits(ncell) + kRadixBits - 1) / kRadixBits;
-  const int tiles = n ? div_up(n, kSortTile) : 0;
-  index_t* alt_keys = scratch.take<index_t>(n + 1);
-  index_t* alt_vals = scratch.take<index_t>(n + 1);
-  index_t* hist = scratch.take<index_t>(static_cast<size_t>(tiles) * kRadixBins + 1);
-  if (!alt_keys || !alt_vals || !hist) return fail(ctx, LSMPS_CUDA_ERROR, "cell list scratch exhausted");
-  // Ping-pong so that the last pass lands in the caller's arrays.
-  index_t* k0 = (passes & 1) ? alt_keys : cells.cell_ids;
-  index_t* v0 = (passes & 1) ? alt_vals : cells.sorted_indices;
-  index_t* k1 = (passes & 1) ? cells.cell_ids : alt_keys;
-  index_t* v1 = (passes & 1) ? cells.sorted_indices : alt_vals;
-  const long long work = n > ncell ? n : ncell;
-  const int hash_blocks = static_cast<int>(std::min<long long>(div_up(work, 256), ctx->sm_count * 8LL));
-  if (boxes)
-    launch(ctx, hash_boxes_kernel, dim3(hash_blocks), dim3(256), 0, x, y, z, n, boxes, ctx->nbox, box_field,
-           grid.cell_size, k0, v0, cells.cell_begin, cells.cell_end, static_cast<index_t>(ncell), ctx->d_status);
-  else
-    launch(ctx, hash_kernel, dim3(hash_blocks), dim3(256), 0, x, y, z, n, grid, k0, v0, cells.cell_begin,
-           cells.cell_end, static_cast<index_t>(ncell), ctx->d_status);
-  if (n == 0) return check_launch(ctx, "cell hash");
-  for (int p = 0; p < passes; ++p) {
-    const int shift = p * kRadixBits;
-    launch(ctx, radix_hist_kernel, dim3(tiles), dim3(kSortThreads), 0, static_cast<const index_t*>(k0), n, shift,
-           hist, tiles);
-    st = exclusive_scan_i32(ctx, scratch, hist, hist, static_cast<size_t>(tiles) * kRadixBins, nullptr, nullptr);
-    if (st) return st;
-    launch(ctx, radix_scatter_kernel, dim3(tiles), dim3(kSortThreads), 0, static_cast<const index_t*>(k0),
-           static_cast<const index_t*>(v0), k1, v1, n, shift, static_cast<const index_t*>(hist), tiles);
-    std::swap(k0, k1);
-    std::swap(v0, v1);
+  return LSMPS_OK;
+}
+
+lsmps_status build_cell_lists_impl(lsmps_ctx* ctx, Scratch& scratch, CellSet* sets, const size_t* counts,
+                                   const lsmps_cells* const* cells, int many, const lsmps_grid& grid,
+                                   const BoxGrid* boxes) {
+  lsmps_status st = validate_grid(ctx, grid);
+  for (int s = 0; s < many && !st; ++s) st = check_cell_set(ctx, sets[s], counts[s], grid, *cells[s]);
+  if (st) return st;
+  // both sets' particles in one index range: one after the other where that
+  // would pass 32 bits
+  if (many == 2 && counts[0] + counts[1] > static_cast<size_t>(INT_MAX)) {
+    for (int s = 0; s < 2 && !st; ++s)
+      st = build_cell_lists_impl(ctx, scratch, sets + s, counts + s, cells + s, 1, grid, boxes);
+    return st;
   }
-  const int range_blocks = static_cast<int>(std::min<long long>(div_up(n, 256), ctx->sm_count * 8LL));
-  launch(ctx, ranges_kernel, dim3(range_blocks), dim3(256), 0, static_cast<const index_t*>(cells.cell_ids), n,
-         cells.cell_begin, cells.cell_end);
-  return check_launch(ctx, "cell list");
+  CellArgs a{};
+  a.sets = many;
+  a.grid = grid;
+  a.ncell = static_cast<index_t>(static_cast<long long>(grid.dims[0]) * grid.dims[1] * grid.dims[2]);
+  a.boxes = boxes;
+  a.nbox = ctx->nbox;
+  a.first1 = static_cast<index_t>(counts[0]);
+  a.total = a.first1 + (many == 2 ? static_cast<index_t>(counts[1]) : 0);
+  a.status = ctx->d_status;
+  for (int s = 0; s < many; ++s) {
+    a.set[s] = sets[s];
+    a.set[s].ids = cells[s]->cell_ids;
+    a.set[s].sorted = cells[s]->sorted_indices;
+    a.set[s].begin = cells[s]->cell_begin;
+    a.set[s].end = cells[s]->cell_end;
+  }
+  const size_t m = static_cast<size_t>(many) * a.ncell;
+  a.key = scratch.take<index_t>(static_cast<size_t>(a.total) + 1);
+  a.number = scratch.take<index_t>(static_cast<size_t>(a.total) + 1);
+  a.placed = scratch.take<index_t>(static_cast<size_t>(a.total) + 1);
+  a.count = scratch.take<index_t>(m + 1);
+  const int tiles = div_up(static_cast<long long>(m), kScanTile);
+  long long* partials = scratch.take<long long>(tiles + 1);
+  if (!a.key || !a.number || !a.placed || !a.count || !partials)
+    return fail(ctx, LSMPS_CUDA_ERROR, "cell list scratch exhausted");
+  if (cudaMemsetAsync(a.count, 0, m * sizeof(index_t), ctx->stream) != cudaSuccess)
+    return check_launch(ctx, "cell counts");
+  const int blocks = static_cast<int>(
+      std::min<long long>(div_up(static_cast<long long>(a.total), kCellThreads), ctx->sm_count * 8LL));
+  if (a.total) launch(ctx, cell_count_kernel, dim3(blocks), dim3(kCellThreads), 0, a);
+  if (m <= static_cast<size_t>(kSmallScan)) {
+    launch(ctx, cell_ranges_small_kernel, dim3(1), dim3(kSmallScanThreads), 0, a);
+  } else {
+    launch(ctx, cell_totals_kernel, dim3(tiles), dim3(kScanThreads), 0, a, partials);
+    if (tiles > kDirectTiles) launch(ctx, scan_partials_kernel, dim3(1), dim3(1024), 0, partials, tiles);
+    launch(ctx, cell_ranges_kernel, dim3(tiles), dim3(kScanThreads), 0, a, static_cast<const long long*>(partials),
+           tiles > kDirectTiles ? 1 : 0);
+  }
+  if (a.total == 0) return check_launch(ctx, "cell lists");
+  launch(ctx, cell_place_kernel, dim3(blocks), dim3(kCellThreads), 0, a);
+  // cells per warp: few enough to give every SM 32 warps, up to 32
+  const long long span = std::min<long long>(
+      32, std::max<long long>(1, static_cast<long long>(m) / (ctx->sm_count * 32LL)));
+  const int order_blocks = static_cast<int>(std::min<long long>(
+      div_up(div_up(static_cast<long long>(m), static_cast<int>(span)), kCellThreads / kWarp), ctx->sm_count * 32LL));
+  launch(ctx, cell_order_kernel, dim3(order_blocks), dim3(kCellThreads), 0, a, static_cast<int>(span));
+  return check_launch(ctx, "cell lists");
 }
 
 }  // namespace lsmps
@@ -251,6 +400,10 @@ extern "C" lsmps_status lsmps_build_cell_list(lsmps_ctx* ctx, const double* x, c
   Scratch scratch(ctx);
   if (!scratch.reserve(cell_list_scratch_bytes(count, cells->cell_count)))
     return fail(ctx, LSMPS_CUDA_ERROR, "scratch allocation failed");
-  st = build_cell_list_impl(ctx, scratch, x, y, z, count, *grid, *cells);
+  CellSet set{};
+  set.x = x;
+  set.y = y;
+  set.z = z;
+  st = build_cell_lists_impl(ctx, scratch, &set, &count, &cells, 1, *grid, nullptr);
   return end_call(ctx, st);
 }

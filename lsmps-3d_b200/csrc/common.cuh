@@ -444,14 +444,27 @@ lsmps_status exclusive_scan_i32(lsmps_ctx* ctx, Scratch& scratch, const index_t*
 // Cell-list build shared by lsmps_build_cell_list and the neighbour search
 // (cells.cu).
 size_t cell_list_scratch_bytes(size_t n, size_t ncell);
-// boxes (a merged batch's device table, ctx->nbox entries): hash each
-// particle on its box's grid (box_field 1: fluid ranges, 2: wall ranges);
-// grid then only supplies the cell size and the total cell count
-// (dims product).
-lsmps_status build_cell_list_impl(lsmps_ctx* ctx, Scratch& scratch, const double* x, const double* y,
-                                  const double* z, size_t count, const lsmps_grid& grid,
-                                  const lsmps_cells& cells, const BoxGrid* boxes = nullptr,
-                                  int box_field = 0);
+// One set of particles to list by cell: the caller fills in the positions, where
+// the positions in sorted order go (or NULL) and, for a merged batch, which of a
+// box's ranges the set is (1: fluid, 2: walls); the rest is the cell list's.
+struct CellSet {
+  const double* x;
+  const double* y;
+  const double* z;
+  double4* pos;
+  int box_field;
+  index_t* ids;
+  index_t* sorted;
+  index_t* begin;
+  index_t* end;
+};
+// The cell lists of one or two sets (counts[s] particles each) on one grid.
+// boxes (a merged batch's device table, ctx->nbox entries): hash each particle
+// on its box's grid; grid then only supplies the cell size and the total cell
+// count (dims product).
+lsmps_status build_cell_lists_impl(lsmps_ctx* ctx, Scratch& scratch, CellSet* sets, const size_t* counts,
+                                   const lsmps_cells* const* cells, int many, const lsmps_grid& grid,
+                                   const BoxGrid* boxes);
 lsmps_status validate_grid(lsmps_ctx* ctx, const lsmps_grid& grid);
 
 }  // namespace lsmps

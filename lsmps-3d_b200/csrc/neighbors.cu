@@ -122,16 +122,6 @@ __device__ __forceinline__ CellFrame frame_of(const CsrArgs& a, index_t c) {
   return f;
 }
 
-// src_pos[k] = {x, y, z, 0} of particle sorted[k].
-__global__ void sorted_positions_kernel(const double* __restrict__ x, const double* __restrict__ y,
-                                        const double* __restrict__ z, const index_t* __restrict__ sorted, index_t n,
-                                        double4* __restrict__ out) {
-  for (index_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    const index_t j = sorted[k];
-    out[k] = make_double4(x[j], y[j], z[j], 0.0);
-  }
-}
-
 __device__ __forceinline__ bool within_radius(double ax, double ay, double az, double bx, double by, double bz,
                                               double r2) {
   const double dx = ax - bx;
@@ -666,7 +656,7 @@ __global__ void __launch_bounds__(kCsrThreads) csr_write_kernel(CsrArgs a) {
 lsmps_status one_neighbor_list(lsmps_ctx* ctx, Scratch& scratch, const lsmps_fluid& fluid, const double* sx,
                                const double* sy, const double* sz, const lsmps_cells& home, const lsmps_cells& src,
                                const lsmps_grid& grid, double radius, bool exclude_self, const lsmps_csr& out,
-                               size_t n_src, unsigned* bits, double4* src_pos, index_t* spos) {
+                               size_t n_src, unsigned* bits, const double4* src_pos, index_t* spos) {
   if (fluid.count > out.particle_count || !out.offsets)
     return fail(ctx, LSMPS_INVALID_ARGUMENT, "Neighbor list particle capacity is smaller than fluid count");
   const size_t n = fluid.count;
@@ -709,12 +699,6 @@ lsmps_status one_neighbor_list(lsmps_ctx* ctx, Scratch& scratch, const lsmps_flu
   // sorted entries; its particle_count is only a capacity)
   if (n_src > src.particle_count)
     return fail(ctx, LSMPS_INVALID_ARGUMENT, "Cell list particle capacity is smaller than particle count");
-  if (n_src > 0) {
-    const int pb = static_cast<int>(std::min<long long>(div_up(static_cast<long long>(n_src), 256),
-                                                        static_cast<long long>(ctx->sm_count) * 8));
-    launch(ctx, sorted_positions_kernel, dim3(pb), dim3(256), 0, sx, sy, sz,
-           static_cast<const index_t*>(src.sorted_indices), static_cast<index_t>(n_src), src_pos);
-  }
   const int count_blocks = static_cast<int>(
       std::min<long long>(div_up(static_cast<long long>(a.ncell), kCountWarps), static_cast<long long>(ctx->sm_count) * 20));
   if (n && ctx->csr_cell_blocks)
@@ -733,9 +717,9 @@ lsmps_status one_neighbor_list(lsmps_ctx* ctx, Scratch& scratch, const lsmps_flu
 }  // namespace
 
 size_t neighbor_scratch_bytes(size_t n_fluid, size_t n_wall, size_t ncell) {
-  const size_t nmax = n_fluid > n_wall ? n_fluid : n_wall;
-  return 2 * cell_list_scratch_bytes(nmax, ncell) + 2 * scan_scratch_bytes(n_fluid + 1) +
-         n_fluid * kMaskWords * sizeof(unsigned) + nmax * sizeof(double4) + 4096;
+  return cell_list_scratch_bytes(n_fluid + n_wall, 2 * ncell) + cell_list_scratch_bytes(0, ncell) +
+         2 * scan_scratch_bytes(n_fluid + 1) + n_fluid * kMaskWords * sizeof(unsigned) +
+         (n_fluid + n_wall) * sizeof(double4) + 8192;
 }
 
 lsmps_status build_neighbor_lists_impl(lsmps_ctx* ctx, Scratch& scratch, const lsmps_fluid& fluid,
@@ -746,17 +730,28 @@ lsmps_status build_neighbor_lists_impl(lsmps_ctx* ctx, Scratch& scratch, const l
   if (radius > p.grid.cell_size)
     return fail(ctx, LSMPS_INVALID_ARGUMENT, "Neighbor search currently requires radius <= cell_size");
   unsigned* bits = scratch.take<unsigned>(fluid.count * kMaskWords + 1);
-  double4* src_pos = scratch.take<double4>(std::max(fluid.count, walls.count) + 1);
-  if (!bits || !src_pos) return fail(ctx, LSMPS_CUDA_ERROR, "neighbour scratch exhausted");
+  double4* fluid_pos = scratch.take<double4>(fluid.count + 1);
+  double4* wall_pos = scratch.take<double4>(walls.count + 1);
+  if (!bits || !fluid_pos || !wall_pos) return fail(ctx, LSMPS_CUDA_ERROR, "neighbour scratch exhausted");
   ctx->built_order = nullptr;
-  lsmps_status st =
-      build_cell_list_impl(ctx, scratch, fluid.x, fluid.y, fluid.z, fluid.count, p.grid, fc, ctx->boxes, 1);
+  CellSet sets[2]{};
+  sets[0].x = fluid.x;
+  sets[0].y = fluid.y;
+  sets[0].z = fluid.z;
+  sets[0].pos = fluid_pos;
+  sets[0].box_field = 1;
+  sets[1].x = walls.x;
+  sets[1].y = walls.y;
+  sets[1].z = walls.z;
+  sets[1].pos = wall_pos;
+  sets[1].box_field = 2;
+  const size_t counts[2] = {fluid.count, walls.count};
+  const lsmps_cells* lists[2] = {&fc, &wc};
+  lsmps_status st = build_cell_lists_impl(ctx, scratch, sets, counts, lists, 2, p.grid, ctx->boxes);
   if (!st) {
     ctx->built_order = fc.sorted_indices;
     ctx->built_order_count = fluid.count;
   }
-  if (!st)
-    st = build_cell_list_impl(ctx, scratch, walls.x, walls.y, walls.z, walls.count, p.grid, wc, ctx->boxes, 2);
   // The fluid table's cell-sorted rows go to the context's own array, where
   // they stay for the next step's gathers.
   ctx->spos_table = nullptr;
@@ -766,7 +761,7 @@ lsmps_status build_neighbor_lists_impl(lsmps_ctx* ctx, Scratch& scratch, const l
   // the two tables run one after the other on the stream and share the masks
   if (!st)
     st = one_neighbor_list(ctx, scratch, fluid, fluid.x, fluid.y, fluid.z, fc, fc, p.grid, radius, true, fn,
-                           fluid.count, bits, src_pos, spos);
+                           fluid.count, bits, fluid_pos, spos);
   if (!st && spos) {
     ctx->spos_table = fn.offsets;
     ctx->spos_order = fc.sorted_indices;
@@ -774,7 +769,7 @@ lsmps_status build_neighbor_lists_impl(lsmps_ctx* ctx, Scratch& scratch, const l
   }
   if (!st)
     st = one_neighbor_list(ctx, scratch, fluid, walls.x, walls.y, walls.z, fc, wc, p.grid, radius, false, wn,
-                           walls.count, bits, src_pos, nullptr);
+                           walls.count, bits, wall_pos, nullptr);
   return st;
 }
 
