@@ -284,11 +284,6 @@ struct lsmps_ctx {
   bool step_packs = false;
   unsigned packs_ready = 0;
   const int32_t* packs_fluid_order = nullptr;
-  // CSR count pass shape: false = warp per home cell, lane per home particle
-  // (the fastest on a GPU the build has to itself); true = block per home
-  // cell, warp per two home particles, which leaves the streams of a batched
-  // graph running beside it faster (set for batch worker contexts).
-  bool csr_cell_blocks = false;
   // 32-byte neighbour records (packed.cuh): two fluid and three wall arrays.
   double4* pack_fluid[2] = {nullptr, nullptr};
   double4* pack_wall[3] = {nullptr, nullptr, nullptr};
@@ -440,6 +435,14 @@ struct StageRange {
 size_t scan_scratch_bytes(size_t n);
 lsmps_status exclusive_scan_i32(lsmps_ctx* ctx, Scratch& scratch, const index_t* in, index_t* out, size_t n,
                                 unsigned long long* total, index_t* total_i32);
+// One or two sets of n counts in the same launches.
+struct ScanSet {
+  const index_t* in;
+  index_t* out;
+  unsigned long long* total;
+  index_t* total_i32;
+};
+lsmps_status exclusive_scans_i32(lsmps_ctx* ctx, Scratch& scratch, const ScanSet* sets, int count, size_t n);
 
 // Cell-list build shared by lsmps_build_cell_list and the neighbour search
 // (cells.cu).
