@@ -69,6 +69,7 @@ MergedArgs merged_args(const MergedBatch& mb) {
 __device__ __forceinline__ int box_fluid(const MergedArgs& a, index_t t) { return box_of(a.grids, a.nbox, t, 1); }
 
 __global__ void gather_kernel(MergedArgs a) {
+  wait_for_previous();
   const index_t stride = gridDim.x * blockDim.x;
   for (index_t t = blockIdx.x * blockDim.x + threadIdx.x; t < a.nf; t += stride) {
     const BoxIO& b = a.io[box_fluid(a, t)];
@@ -112,6 +113,7 @@ __device__ __forceinline__ void copy3(const lsmps_vector& src, const lsmps_vecto
 // moment traces; the first particle of a box advances the box's inversion
 // counters (one per kind and step, as a solo step does).
 __global__ void scatter_particles_kernel(MergedArgs a) {
+  wait_for_previous();
   const index_t stride = gridDim.x * blockDim.x;
   const lsmps_step_state& m = a.m;
   for (index_t t = blockIdx.x * blockDim.x + threadIdx.x; t < a.nf; t += stride) {
@@ -166,6 +168,7 @@ __global__ void scatter_particles_kernel(MergedArgs a) {
 }
 
 __global__ void scatter_walls_kernel(MergedArgs a) {
+  wait_for_previous();
   const index_t stride = gridDim.x * blockDim.x;
   for (index_t t = blockIdx.x * blockDim.x + threadIdx.x; t < a.nw; t += stride) {
     const BoxIO& b = a.io[box_of(a.grids, a.nbox, t, 2)];
@@ -181,6 +184,7 @@ __global__ void scatter_walls_kernel(MergedArgs a) {
 __device__ __forceinline__ index_t shift_or_empty(index_t v, index_t base) { return v < 0 ? -1 : v - base; }
 
 __global__ void scatter_cells_kernel(MergedArgs a) {
+  wait_for_previous();
   const index_t stride = gridDim.x * blockDim.x;
   for (index_t c = blockIdx.x * blockDim.x + threadIdx.x; c < a.nc; c += stride) {
     const BoxIO& b = a.io[box_of(a.grids, a.nbox, c, 0)];
@@ -305,6 +309,7 @@ __device__ void scatter_table(const MergedArgs& a, const index_t* offsets, const
 // the cursor walks past it because its first row starts where the next
 // box's does.
 __global__ void scatter_entries_kernel(MergedArgs a) {
+  wait_for_previous();
   // the rebuilt totals, held to the merged capacities (beyond them the
   // rebuild wrote nothing and has raised the capacity flag)
   const index_t kf = static_cast<index_t>(min(static_cast<unsigned long long>(a.m.fluid_neighbors.offsets[a.nf]),
@@ -318,6 +323,7 @@ __global__ void scatter_entries_kernel(MergedArgs a) {
 
 // Plain form: the 81-entry inverses of both kinds.
 __global__ void scatter_inverse_kernel(MergedArgs a) {
+  wait_for_previous();
   const long long total = 81LL * a.nf;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long v = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; v < total; v += stride) {

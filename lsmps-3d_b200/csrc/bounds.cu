@@ -21,6 +21,7 @@ namespace {
 
 __global__ void csr_check_kernel(const index_t* __restrict__ offsets, const index_t* __restrict__ indices, index_t n,
                                  unsigned long long capacity, long long n_src, DeviceStatus* __restrict__ status) {
+  wait_for_previous();
   for (index_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const index_t b = offsets[i], e = offsets[i + 1];
     if (b < 0 || e < b || static_cast<unsigned long long>(e) > capacity || (i == 0 && b != 0)) {

@@ -43,6 +43,7 @@ __global__ void hash_kernel(const double* __restrict__ x, const double* __restri
                             index_t* __restrict__ keys, index_t* __restrict__ vals,
                             index_t* __restrict__ cell_begin, index_t* __restrict__ cell_end, index_t ncell,
                             DeviceStatus* __restrict__ status) {
+  wait_for_previous();
   const index_t total = n > ncell ? n : ncell;
   for (index_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
     if (t < ncell) {
@@ -65,6 +66,7 @@ __global__ void hash_kernel(const double* __restrict__ x, const double* __restri
 __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const index_t* __restrict__ keys, index_t n,
                                                                   int shift, index_t* __restrict__ hist,
                                                                   int tiles) {
+  wait_for_previous();
   __shared__ unsigned int bins[kRadixBins];
   bins[threadIdx.x] = 0;
   __syncthreads();
@@ -85,6 +87,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(const index_t*
 __global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(
     const index_t* __restrict__ keys_in, const index_t* __restrict__ vals_in, index_t* __restrict__ keys_out,
     index_t* __restrict__ vals_out, index_t n, int shift, const index_t* __restrict__ hist_scanned, int tiles) {
+  wait_for_previous();
   __shared__ unsigned int base[kRadixBins];
   __shared__ unsigned int warp_count[kSortWarps][kRadixBins];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -133,6 +136,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(
 // build_cell_ranges_kernel, neighbor_search.cu:85-98.
 __global__ void ranges_kernel(const index_t* __restrict__ keys, index_t n, index_t* __restrict__ cell_begin,
                               index_t* __restrict__ cell_end) {
+  wait_for_previous();
   for (index_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
     const index_t c = keys[p];
     if (p == 0 || keys[p - 1] != c) cell_begin[c] = p;
@@ -166,6 +170,7 @@ struct CellArgs {
 // of every cell.  In a merged batch a particle is hashed on the grid of the box
 // whose range of its set holds it.
 __global__ void __launch_bounds__(kCellThreads) cell_count_kernel(CellArgs a) {
+  wait_for_previous();
   for (index_t p = blockIdx.x * kCellThreads + threadIdx.x; p < a.total; p += gridDim.x * kCellThreads) {
     const int s = p >= a.first1 ? 1 : 0;
     const CellSet& set = a.set[s];
@@ -204,24 +209,28 @@ __device__ __forceinline__ void store_range(const CellArgs& a, size_t c, long lo
 }
 
 __global__ void __launch_bounds__(kSmallScanThreads) cell_ranges_small_kernel(CellArgs a) {
+  wait_for_previous();
   scan_small(
       a.sets * a.ncell, [&](int i) { return a.count[i]; },
       [&](int i, long long before, index_t v) { store_range(a, i, before, v); });
 }
 
 __global__ void __launch_bounds__(kScanThreads) cell_totals_kernel(CellArgs a, long long* __restrict__ partials) {
+  wait_for_previous();
   const long long t = tile_sum(static_cast<size_t>(a.sets) * a.ncell, [&](size_t i) { return a.count[i]; });
   if (threadIdx.x == 0) partials[blockIdx.x] = t;
 }
 
 __global__ void __launch_bounds__(kScanThreads) cell_ranges_kernel(CellArgs a, const long long* __restrict__ partials,
                                                                   int scanned) {
+  wait_for_previous();
   scan_tile(
       static_cast<size_t>(a.sets) * a.ncell, before_tile(partials, scanned != 0), [&](size_t i) { return a.count[i]; },
       [&](size_t i, long long before, index_t v) { store_range(a, i, before, v); });
 }
 
 __global__ void __launch_bounds__(kCellThreads) cell_place_kernel(CellArgs a) {
+  wait_for_previous();
   for (index_t p = blockIdx.x * kCellThreads + threadIdx.x; p < a.total; p += gridDim.x * kCellThreads) {
     const int s = p >= a.first1 ? 1 : 0;
     const index_t first = s ? a.first1 : 0;
@@ -270,6 +279,7 @@ __device__ __forceinline__ void order_cell(const CellArgs& a, const CellSet& set
 
 // Each warp orders the non-empty ones of `span` (1 .. 32) consecutive cells.
 __global__ void __launch_bounds__(kCellThreads) cell_order_kernel(CellArgs a, int span) {
+  wait_for_previous();
   const int lane = threadIdx.x & (kWarp - 1);
   const long long cells = static_cast<long long>(a.sets) * a.ncell;
   const long long warps = static_cast<long long>(gridDim.x) * (kCellThreads / kWarp);

@@ -48,6 +48,7 @@ constexpr int kScanThreads = 1024;
 // Exclusive scan of the histogram table in one block: each thread owns a
 // contiguous run of entries (at most kHistEntries / kScanThreads = 32).
 __global__ void __launch_bounds__(kScanThreads) hist_scan_kernel(index_t* __restrict__ hist, int entries) {
+  wait_for_previous();
   __shared__ index_t warp_total[kScanThreads / kWarp];
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x >> 5;
   const int per = (entries + kScanThreads - 1) / kScanThreads;

@@ -24,6 +24,7 @@ __device__ __forceinline__ bool is_surface(const int32_t* type, index_t i) {
 
 // clamp_fluid_pressure_kernel, pressure_correction.cu:188-198
 __global__ void clamp_kernel(index_t n, double* pressure, double* fluid_pressure) {
+  wait_for_previous();
   for (index_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double p = pressure[i];
     const double c = p < 0.0 ? 0.0 : p;
@@ -54,6 +55,7 @@ __global__ void __launch_bounds__(kThreads) gradient_kernel(GatherArgs a, const 
                                                             const double* __restrict__ pinv, double re,
                                                             double wall_scale, double* gx, double* gy,
                                                             double* gz) {
+  wait_for_previous();
   const index_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= static_cast<index_t>(a.fluid.count)) return;
   if (is_splash(a.fluid.surface_type, i)) {
@@ -110,6 +112,7 @@ __global__ void __launch_bounds__(kThreads) gradient_kernel(GatherArgs a, const 
 // compute_particle_shifting_kernel, pressure_correction.cu:278-367
 __global__ void __launch_bounds__(kThreads) shifting_kernel(GatherArgs a, double* sx_out, double* sy_out,
                                                             double* sz_out) {
+  wait_for_previous();
   const index_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= static_cast<index_t>(a.fluid.count)) return;
   if (a.p.ps_displacement_scale <= 0.0 || is_splash(a.fluid.surface_type, i)) {
@@ -183,6 +186,7 @@ __global__ void update_kernel(lsmps_fluid f, const double* __restrict__ tx, cons
                               const double* __restrict__ gx, const double* __restrict__ gy,
                               const double* __restrict__ gz, const double* __restrict__ sx,
                               const double* __restrict__ sy, const double* __restrict__ sz) {
+  wait_for_previous();
   const double dt = dtp ? *dtp : dt_host;
   for (index_t i = blockIdx.x * blockDim.x + threadIdx.x; i < static_cast<index_t>(f.count);
        i += gridDim.x * blockDim.x) {
@@ -210,6 +214,7 @@ __global__ void __launch_bounds__(kThreads) anti_penetration_kernel(lsmps_fluid 
                                                                     const index_t* __restrict__ wo,
                                                                     const index_t* __restrict__ wi,
                                                                     double clearance) {
+  wait_for_previous();
   const index_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= static_cast<index_t>(f.count)) return;
   const index_t we = wo[i + 1];
@@ -254,6 +259,7 @@ __global__ void __launch_bounds__(kThreads) smooth_kernel(index_t n, const doubl
                                                           const index_t* __restrict__ fi, double re, double strength,
                                                           double* ox, double* oy, double* oz,
                                                           const int32_t* __restrict__ order, int sorted) {
+  wait_for_previous();
   // G lanes per particle (lane l takes entries l, l + G, ...); the group
   // leaves or continues as a whole.
   const index_t t = (blockIdx.x * blockDim.x + threadIdx.x) / G;
@@ -318,6 +324,7 @@ __global__ void __launch_bounds__(kThreads) smooth_kernel(index_t n, const doubl
 // copy_smoothed_velocity_kernel, pressure_correction.cu:506-515
 __global__ void copy_kernel(index_t n, const double* __restrict__ sx, const double* __restrict__ sy,
                             const double* __restrict__ sz, double* vx, double* vy, double* vz) {
+  wait_for_previous();
   for (index_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     vx[i] = sx[i];
     vy[i] = sy[i];
@@ -668,6 +675,7 @@ __device__ __forceinline__ void gradient_shifting_of(const GatherArgs& a, const 
 
 template <bool Mixed, int G>
 __global__ void __launch_bounds__(kThreads, 6) gradient_shifting_kernel(GatherArgs a, GradShiftOut out) {
+  wait_for_previous();
   const long long tt = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   const index_t t = static_cast<index_t>(tt / G);
   const int l = static_cast<int>(tt % G);
@@ -680,6 +688,7 @@ __global__ void __launch_bounds__(kThreads, 6) gradient_shifting_kernel(GatherAr
 // G>, FP64 arithmetic); lane groups stride over the list.
 template <int G>
 __global__ void __launch_bounds__(kThreads, 6) gradient_shifting_list_kernel(GatherArgs a, GradShiftOut out) {
+  wait_for_previous();
   const index_t groups = static_cast<index_t>(gridDim.x * blockDim.x / G);
   const int l = threadIdx.x & (G - 1);
   const index_t count = static_cast<index_t>(*out.prows.count);
@@ -701,6 +710,7 @@ __global__ void __launch_bounds__(kThreads, 6) gradient_shifting_list_kernel(Gat
 // pressure rows took the FP64 route are left to gradient_shifting_list_kernel.
 template <int G>
 __global__ void __launch_bounds__(kThreads, 6) gradient32_kernel(GatherArgs a, GradShiftOut out) {
+  wait_for_previous();
   const long long tt = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   const index_t t = static_cast<index_t>(tt / G);
   const int l = static_cast<int>(tt % G);
@@ -874,6 +884,7 @@ __global__ void __launch_bounds__(kThreads) update_anti_penetration_kernel(
     const double* __restrict__ dtp, double density, const double* __restrict__ gx, const double* __restrict__ gy, const double* __restrict__ gz,
     const double* __restrict__ sx, const double* __restrict__ sy, const double* __restrict__ sz, double clearance,
     const double4* __restrict__ wp, const double4* __restrict__ wn) {
+  wait_for_previous();
   const index_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= static_cast<index_t>(f.count)) return;
   const double dt = dtp ? *dtp : dt_host;

@@ -298,6 +298,7 @@ template <int G, bool TypeB>
 __global__ void __launch_bounds__(kSumThreads, 4) plain_sums_kernel(SumArgs a, const index_t* __restrict__ wo,
                                                                     int32_t* __restrict__ walled,
                                                                     unsigned* __restrict__ walls) {
+  wait_for_previous();
   constexpr int S = TypeB ? kMonomialsB : kMonomials;
   const index_t t = static_cast<index_t>((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / G);
   const int l = threadIdx.x & (G - 1);
@@ -436,6 +437,7 @@ __device__ __forceinline__ void wall_sums(const WallArgs& a) {
 
 // blockIdx.y + first: 0 the Dirichlet samples, 1 the Neumann terms
 __global__ void __launch_bounds__(kWallThreads) wall_sums_kernel(WallArgs a, int first) {
+  wait_for_previous();
   if (blockIdx.y + first == 0)
     wall_sums<false>(a);
   else
@@ -522,6 +524,7 @@ __device__ __forceinline__ void warp_store_symmetric(const double (&x)[N * (N + 
 // 75 us where it took 185 at 1,000 particles, with the same bits.
 template <int N>
 __global__ void __launch_bounds__(kFinishThreads, N == 9 ? 16 : 10) moment_finish_kernel(FinishArgs a) {
+  wait_for_previous();
   constexpr int o = N - 9;
   __shared__ double s_stage[27][kWarp + 1];
   const KindOut& ko = a.k[blockIdx.y];
@@ -669,6 +672,7 @@ __device__ __forceinline__ void monomial_pairs(f32x2 (&t)[16], float sx, float s
 }
 
 __global__ void __launch_bounds__(kSumThreads) moment_sums_kernel(SumArgs a) {
+  wait_for_previous();
   const index_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= a.n) return;
   const index_t i = visit(a.order, t);
@@ -1126,6 +1130,7 @@ __device__ __forceinline__ void mixed_rows_of_particle(const MixedRowArgs& a, in
 
 template <bool Full>
 __global__ void __launch_bounds__(kRowThreads, 6) moment_rows_kernel(MixedRowArgs a) {
+  wait_for_previous();
   __shared__ double s_m[45 * kRowThreads];
   const int kind = blockIdx.y;
   const index_t t = blockIdx.x * kRowThreads + threadIdx.x;
@@ -1145,6 +1150,7 @@ __global__ void __launch_bounds__(kRowThreads, 6) moment_rows_kernel(MixedRowArg
 // totals, then warp 0 finishes the velocity kind and warp 1 the pressure kind.
 template <bool Full>
 __global__ void __launch_bounds__(kRowThreads, 6) moment_mixed_split_kernel(SumArgs sa, MixedRowArgs a) {
+  wait_for_previous();
   static_assert(kRowThreads == 2 * kWarp, "two warps per block");
   __shared__ double s_m[45 * kRowThreads];
   __shared__ double s_half[2][kMonomials][kWarp];

@@ -273,6 +273,7 @@ __device__ __forceinline__ void stage_runs(const SourceRuns& runs, Load load, St
 // the home cell) and is cleared after the tests (the reference skips j == i).
 // The masks meet in shared memory and leave it as whole lines.
 __global__ void __launch_bounds__(kCountThreads) csr_count_kernel(const __grid_constant__ CsrTables tables) {
+  wait_for_previous();
   __shared__ float4 sxy[kStageCap / 2];  // pair p: {x_2p, x_2p+1, y_2p, y_2p+1}
   __shared__ float2 sz[kStageCap / 2];   // pair p: {z_2p, z_2p+1}
   __shared__ unsigned far[kMaskWords];   // per chunk: candidates outside the window
@@ -428,6 +429,7 @@ __global__ void __launch_bounds__(kCountThreads) csr_count_kernel(const __grid_c
 // warp stores whole rows, 32 consecutive entries at a time.  Rows come out in the
 // reference's order.
 __global__ void __launch_bounds__(kCsrThreads) csr_write_kernel(const __grid_constant__ CsrTables tables) {
+  wait_for_previous();
   __shared__ index_t s_idx[kStageCap];
   __shared__ index_t s_sp[kStageCap];  // the candidates' sorted positions
   __shared__ SourceRuns runs;

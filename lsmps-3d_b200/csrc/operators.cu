@@ -150,6 +150,7 @@ __device__ __noinline__ void stage_row_again(const OperatorArgs& a, const double
 // 0.88 with one thread a particle, which wrote its row slot by slot).
 template <bool Walls>
 __global__ void __launch_bounds__(kAdjThreads, 5) operators_forward_kernel(OperatorArgs a) {
+  wait_for_previous();
   // per warp: the Laplacian row of the scalar's (pressure's) inverse, its rows
   // 0..2, rows 0..2 of the velocity's and, with walls, its Laplacian row
   __shared__ __align__(16) double s_row[kAdjWarps][8][10];
@@ -302,6 +303,7 @@ __global__ void __launch_bounds__(kAdjThreads, 5) operators_forward_kernel(Opera
 // 1.24 ms for the stash and 1.3 ms for a transpose of the table.
 template <bool Walls, bool Atomic>
 __global__ void __launch_bounds__(kAdjThreads, 4) operators_backward_kernel(const __grid_constant__ OperatorArgs a) {
+  wait_for_previous();
   extern __shared__ __align__(16) unsigned char s_rows[];  // a StagedRow per warp
   __shared__ double s_r[kAdjWarps][82];      // 45 sums, the 36 cotangents of y
   __shared__ double2 s_st[kAdjWarps][5][9];  // {Rbar, y} of the four fields, {hhat, l}
@@ -592,6 +594,7 @@ __global__ void __launch_bounds__(kAdjThreads, 4) operators_backward_kernel(cons
 // up to 128 at a time.  A row of 108 costs the ranking about 900 warp
 // instructions, half of what the 64-byte records' own transfer takes.
 __global__ void __launch_bounds__(kAdjThreads) operators_collect_kernel(OperatorArgs a) {
+  wait_for_previous();
   constexpr int kWindow = 128, kPer = kWindow / kWarp;
   __shared__ __align__(16) int s_id[kAdjWarps][kWindow];
   __shared__ int s_at[kAdjWarps][kWindow];
@@ -664,6 +667,7 @@ __global__ void __launch_bounds__(kAdjThreads) operators_collect_kernel(Operator
 __global__ void __launch_bounds__(kAdjThreads) incoming_count_kernel(const index_t* __restrict__ fo,
                                                                      const index_t* __restrict__ fi, index_t n,
                                                                      index_t* __restrict__ count) {
+  wait_for_previous();
   const index_t i = static_cast<index_t>((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / 8);
   if (i >= n) return;
   const index_t ne = fo[i + 1];

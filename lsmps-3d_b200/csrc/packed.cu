@@ -6,6 +6,7 @@ namespace lsmps {
 __global__ void pack4_kernel(const double* __restrict__ a, const double* __restrict__ b,
                              const double* __restrict__ c, const double* __restrict__ d, index_t n,
                              double4* __restrict__ out, const index_t* __restrict__ order) {
+  wait_for_previous();
   for (index_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const index_t j = order ? order[i] : i;
     out[i] = make_double4(a[j], b[j], c[j], d ? d[j] : 0.0);
@@ -15,6 +16,7 @@ __global__ void pack4_kernel(const double* __restrict__ a, const double* __restr
 __global__ void pack4_label_kernel(const double* __restrict__ a, const double* __restrict__ b,
                                    const double* __restrict__ c, const int32_t* __restrict__ label, index_t n,
                                    double4* __restrict__ out, const index_t* __restrict__ order) {
+  wait_for_previous();
   for (index_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const index_t j = order ? order[i] : i;
     out[i] = make_double4(a[j], b[j], c[j], label ? static_cast<double>(label[j]) : 0.0);

@@ -140,6 +140,7 @@ __device__ __forceinline__ double coeff_row(const double* __restrict__ inv, cons
 }
 
 __global__ void __launch_bounds__(kThreads) ppe_kernel(PpeArgs a) {
+  wait_for_previous();
   const index_t i = blockIdx.x * blockDim.x + threadIdx.x;
   const index_t n = static_cast<index_t>(a.fluid.count);
   if (i >= n) return;
@@ -355,6 +356,7 @@ __device__ __forceinline__ void ppe_row(const PpeArgs& a, index_t i, index_t vt,
 
 template <int G, bool Mixed>
 __global__ void __launch_bounds__(kThreads, 4) ppe_lanes_kernel(PpeArgs a) {
+  wait_for_previous();
   const index_t t = (blockIdx.x * blockDim.x + threadIdx.x) / G;
   const int l = threadIdx.x & (G - 1);
   // Whole groups leave together, so the shuffles see full groups.
@@ -497,6 +499,7 @@ __device__ __forceinline__ void ppe_row32(const PpeArgs& a, index_t i, index_t v
 
 template <int G>
 __global__ void __launch_bounds__(kThreads, 7) ppe32_kernel(PpeArgs a) {
+  wait_for_previous();
   const index_t t = (blockIdx.x * blockDim.x + threadIdx.x) / G;
   const int l = threadIdx.x & (G - 1);
   if (t >= static_cast<index_t>(a.fluid.count)) return;
@@ -510,6 +513,7 @@ __global__ void __launch_bounds__(kThreads, 7) ppe32_kernel(PpeArgs a) {
 // stride over the lists.
 template <int G>
 __global__ void __launch_bounds__(kThreads, 4) ppe_list_kernel(PpeArgs a) {
+  wait_for_previous();
   const index_t groups = static_cast<index_t>(gridDim.x * blockDim.x / G);
   const index_t g0 = static_cast<index_t>((blockIdx.x * blockDim.x + threadIdx.x) / G);
   const int l = threadIdx.x & (G - 1);

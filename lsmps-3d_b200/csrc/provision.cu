@@ -138,6 +138,7 @@ __device__ __forceinline__ void laplacian_of(const LaplacianArgs& a, const Mixed
 
 template <bool Mixed, int G>
 __global__ void __launch_bounds__(kThreads, 5) laplacian_kernel(LaplacianArgs a, MixedRows rows) {
+  wait_for_previous();
   const index_t t = (blockIdx.x * blockDim.x + threadIdx.x) / G;
   const int l = threadIdx.x & (G - 1);
   if (t >= a.n) return;  // the whole group
@@ -152,6 +153,7 @@ __global__ void __launch_bounds__(kThreads, 5) laplacian_kernel(LaplacianArgs a,
 // velocity rows took the FP64 route are left to laplacian_list_kernel.
 template <int G>
 __global__ void __launch_bounds__(kThreads, 7) laplacian32_kernel(LaplacianArgs a, MixedRows rows) {
+  wait_for_previous();
   const index_t t = (blockIdx.x * blockDim.x + threadIdx.x) / G;
   const int l = threadIdx.x & (G - 1);
   if (t >= a.n) return;  // the whole group
@@ -227,6 +229,7 @@ __global__ void __launch_bounds__(kThreads, 7) laplacian32_kernel(LaplacianArgs 
 // laplacian_of<true, G>); lane groups stride over the list.
 template <int G>
 __global__ void __launch_bounds__(kThreads, 5) laplacian_list_kernel(LaplacianArgs a, MixedRows rows) {
+  wait_for_previous();
   const index_t groups = static_cast<index_t>(gridDim.x * blockDim.x / G);
   const int l = threadIdx.x & (G - 1);
   const index_t count = static_cast<index_t>(*rows.count);
@@ -241,6 +244,7 @@ __global__ void __launch_bounds__(kThreads, 5) laplacian_list_kernel(LaplacianAr
 __global__ void combine_kernel(lsmps_fluid f, lsmps_params p, const double* __restrict__ lx,
                                const double* __restrict__ ly, const double* __restrict__ lz, double* tx, double* ty,
                                double* tz, const double* __restrict__ dtp) {
+  wait_for_previous();
   const double dt = dtp ? *dtp : p.time_step;
   for (index_t i = blockIdx.x * blockDim.x + threadIdx.x; i < static_cast<index_t>(f.count);
        i += gridDim.x * blockDim.x) {
@@ -255,6 +259,7 @@ __global__ void combine_kernel(lsmps_fluid f, lsmps_params p, const double* __re
 // combine_explicit_wall_velocity_kernel, explicit_update.cu:272-284
 __global__ void wall_combine_kernel(lsmps_walls w, lsmps_params p, double* tx, double* ty, double* tz,
                                     const double* __restrict__ dtp) {
+  wait_for_previous();
   const double dt = dtp ? *dtp : p.time_step;
   for (index_t i = blockIdx.x * blockDim.x + threadIdx.x; i < static_cast<index_t>(w.count);
        i += gridDim.x * blockDim.x) {

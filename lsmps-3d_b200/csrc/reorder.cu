@@ -26,11 +26,13 @@ constexpr int kThreads = 256;
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
     gather_kernel(const T* __restrict__ src, const index_t* __restrict__ order, index_t n, T* __restrict__ dst) {
+  wait_for_previous();
   for (index_t k = blockIdx.x * kThreads + threadIdx.x; k < n; k += gridDim.x * kThreads) dst[k] = src[order[k]];
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads) copy_back_kernel(const T* __restrict__ src, index_t n, T* __restrict__ dst) {
+  wait_for_previous();
   for (index_t k = blockIdx.x * kThreads + threadIdx.x; k < n; k += gridDim.x * kThreads) dst[k] = src[k];
 }
 

@@ -11,6 +11,7 @@
 namespace lsmps {
 
 __global__ void __launch_bounds__(1024) scan_partials_kernel(long long* __restrict__ partials, int count) {
+  wait_for_previous();
   __shared__ long long warp_sum[32];
   __shared__ long long carry;
   if (threadIdx.x == 0) carry = 0;
@@ -53,6 +54,7 @@ struct ScanSets {
 
 __global__ void __launch_bounds__(kSmallScanThreads) scan_small_kernel(const __grid_constant__ ScanSets sets, int n,
                                                                        DeviceStatus* status) {
+  wait_for_previous();
   const ScanSet& a = sets.t[blockIdx.y];
   const long long sum =
       scan_small(n, [&](int i) { return a.in[i]; },
@@ -62,6 +64,7 @@ __global__ void __launch_bounds__(kSmallScanThreads) scan_small_kernel(const __g
 
 __global__ void __launch_bounds__(kScanThreads) scan_reduce_kernel(const __grid_constant__ ScanSets sets, size_t n,
                                                                    long long* __restrict__ partials) {
+  wait_for_previous();
   const ScanSet& a = sets.t[blockIdx.y];
   const long long t = tile_sum(n, [&](size_t i) { return a.in[i]; });
   if (threadIdx.x == 0) partials[static_cast<size_t>(blockIdx.y) * gridDim.x + blockIdx.x] = t;
@@ -70,6 +73,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_reduce_kernel(const __grid_
 __global__ void __launch_bounds__(kScanThreads) scan_down_kernel(const __grid_constant__ ScanSets sets, size_t n,
                                                                  const long long* __restrict__ partials, int scanned,
                                                                  DeviceStatus* status) {
+  wait_for_previous();
   const ScanSet& a = sets.t[blockIdx.y];
   const long long end =
       scan_tile(n, before_tile(partials + static_cast<size_t>(blockIdx.y) * gridDim.x, scanned != 0),

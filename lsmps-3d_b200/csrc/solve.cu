@@ -149,6 +149,7 @@ __device__ __forceinline__ void add_partials(const double* partial, int count, d
 // r = b - A x into w[0] and its norm (First: x = 0, so r = b): opens a cycle.
 template <bool First>
 __global__ void __launch_bounds__(kSolveThreads) residual_kernel(SolveArgs a, int report) {
+  wait_for_previous();
   constexpr int G = kProductLanes;
   const int l = threadIdx.x & (G - 1);
   const index_t rows = static_cast<index_t>(gridDim.x * (kSolveThreads / G));
@@ -190,6 +191,7 @@ __global__ void __launch_bounds__(kSolveThreads) residual_kernel(SolveArgs a, in
 
 // Step j: v_j = scale w[j & 1] into the basis, w[(j + 1) & 1] = A v_j.
 __global__ void __launch_bounds__(kSolveThreads) product_kernel(SolveArgs a, int j) {
+  wait_for_previous();
   const SolveState* st = a.st;
   if (st->stop) return;
   const double scale = st->scale;
@@ -211,6 +213,7 @@ __global__ void __launch_bounds__(kSolveThreads) product_kernel(SolveArgs a, int
 // against 138 + 14 (the vectors' loads hold up the row's).
 template <int Dots>
 __global__ void __launch_bounds__(kSolveThreads) product_dots_kernel(SolveArgs a, int j) {
+  wait_for_previous();
   SolveState* st = a.st;
   if (st->stop) return;
   const double scale = st->scale;
@@ -264,6 +267,7 @@ __global__ void __launch_bounds__(kSolveThreads) product_dots_kernel(SolveArgs a
 // instance holds.
 template <int K, bool Update>
 __global__ void __launch_bounds__(kSolveThreads) project_kernel(SolveArgs a, int j) {
+  wait_for_previous();
   SolveState* st = a.st;
   if (st->stop) return;
   __shared__ double sh[K];
@@ -310,6 +314,7 @@ __global__ void __launch_bounds__(kSolveThreads) project_kernel(SolveArgs a, int
 // its subdiagonal.
 template <int K>
 __global__ void __launch_bounds__(kSolveThreads) extend_kernel(SolveArgs a, int j) {
+  wait_for_previous();
   SolveState* st = a.st;
   if (st->stop) return;
   __shared__ double sh[kMaxRestart + 1];
@@ -373,6 +378,7 @@ __global__ void __launch_bounds__(kSolveThreads) extend_kernel(SolveArgs a, int 
 // y = R^-1 g (back substitution on the rotated Hessenberg, by the first warp of
 // each block), x += M^-1 V y.
 __global__ void __launch_bounds__(kSolveThreads) correct_kernel(SolveArgs a) {
+  wait_for_previous();
   const SolveState* st = a.st;
   __shared__ double sy[kMaxRestart];
   const int m = st->steps;
@@ -405,6 +411,7 @@ __global__ void __launch_bounds__(kSolveThreads) correct_kernel(SolveArgs a) {
 __global__ void __launch_bounds__(kSolveThreads)
     jacobi_kernel(index_t n, const index_t* __restrict__ ro, const index_t* __restrict__ ci,
                   const double* __restrict__ va, double* __restrict__ dinv) {
+  wait_for_previous();
   const index_t i = blockIdx.x * kSolveThreads + threadIdx.x;
   if (i >= n) return;
   double d = 0.0;
@@ -415,6 +422,7 @@ __global__ void __launch_bounds__(kSolveThreads)
 
 // clamp_pressure_kernel, ppe_matrix.cu:373-379
 __global__ void __launch_bounds__(kSolveThreads) clamp_kernel(index_t n, double* __restrict__ x) {
+  wait_for_previous();
   const index_t i = blockIdx.x * kSolveThreads + threadIdx.x;
   if (i < n && x[i] < 0.0) x[i] = 0.0;
 }

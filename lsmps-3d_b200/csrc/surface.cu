@@ -210,6 +210,7 @@ __device__ __forceinline__ void add_row(Moments& m, const double4* __restrict__ 
 // entries' terms formed together (0.53 and 0.60 ms: 90 to 120 registers), eight
 // blocks per SM (0.51 ms).
 __global__ void __launch_bounds__(kSurfaceThreads) classify_kernel(SurfaceArgs a) {
+  wait_for_previous();
   const index_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= static_cast<index_t>(a.fluid.count)) return;
   const index_t i = visit(a.order, t);
@@ -246,6 +247,7 @@ constexpr int kLabelLanes = 16;
 constexpr index_t kLabelSmall = 131072;
 
 __global__ void __launch_bounds__(kSurfaceThreads) classify_small_kernel(SurfaceArgs a) {
+  wait_for_previous();
   constexpr int G = kLabelLanes, kGroups = kSurfaceThreads / G;
   __shared__ double s_term[kGroups][5][G + 1];
   const index_t t = (blockIdx.x * blockDim.x + threadIdx.x) / G;
@@ -334,6 +336,7 @@ __global__ void __launch_bounds__(kSurfaceThreads) expand_kernel(const double4* 
                                                                  const index_t* __restrict__ fi, double r2,
                                                                  const int32_t* __restrict__ order,
                                                                  const int32_t* __restrict__ sorted_labels) {
+  wait_for_previous();
   const index_t t = (blockIdx.x * blockDim.x + threadIdx.x) / kExpandLanes;
   const int l = threadIdx.x & (kExpandLanes - 1);
   if (t >= n) return;  // the whole group
@@ -424,6 +427,7 @@ __global__ void __launch_bounds__(kSurfaceThreads)
                          const index_t* __restrict__ fo, const index_t* __restrict__ fi,
                          const index_t* __restrict__ wo, const index_t* __restrict__ wi, int include_walls,
                          double re2, double cone, int32_t* open_count, double* open_fraction) {
+  wait_for_previous();
   const index_t i = (blockIdx.x * blockDim.x + threadIdx.x) / kLightLanes;
   const int l = threadIdx.x & (kLightLanes - 1);
   if (i >= n) return;  // the whole group

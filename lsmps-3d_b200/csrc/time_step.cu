@@ -31,6 +31,7 @@ __device__ __forceinline__ double warp_max(double v) {
 
 // partial[bx] = the largest finite |u| in this block's slice (0 if none).
 __global__ void __launch_bounds__(kThreads) max_speed_kernel(lsmps_fluid f, double* __restrict__ partial) {
+  wait_for_previous();
   double m = 0.0;
   for (index_t i = blockIdx.x * kThreads + threadIdx.x; i < static_cast<index_t>(f.count);
        i += gridDim.x * kThreads) {
@@ -51,6 +52,7 @@ __global__ void __launch_bounds__(kThreads) max_speed_kernel(lsmps_fluid f, doub
 // The maximum over the partials, then SimulationTimeManager::advance.
 __global__ void __launch_bounds__(kThreads)
     advance_kernel(const double* __restrict__ partial, int nb, lsmps_time_limits lim, lsmps_time_state* st) {
+  wait_for_previous();
   double m = 0.0;
   for (int b = threadIdx.x; b < nb; b += kThreads) m = fmax(m, partial[b]);
   __shared__ double red[kThreads / kWarp];
