@@ -342,6 +342,127 @@ __global__ void __launch_bounds__(kSumThreads, 4) plain_sums_kernel(SumArgs a, c
     if (k < count) a.sums[static_cast<size_t>(base + k) * a.n + t] = s[k];
 }
 
+// Sums in parts, for sets that leave most of the GPU idle with a thread to a
+// particle: a block of kPartWarps warps takes 32 particles, a lane each.  In a
+// round every warp forms the offset and weight of another entry of its lanes'
+// rows (the long chain through the square root), the block shares them, and every
+// warp adds all of the round's entries, in row order, to its own part of the sums:
+// the same additions as one thread makes, so the same bits.  The products behind
+// the additions are made once per part and the rounds meet at a barrier, so the
+// work is two to five times that of a thread per particle: it pays while the
+// blocks have SMs to themselves.  Event times of the sums and of the wall terms,
+// thread per particle -> parts (about 4.5 us of each are the events'): 1,000
+// particles 35.6 -> 18.9 and 39.0 -> 26.8 us, 2,016: 40.2 -> 18.9 and 39.5 -> 33.0,
+// 4,096: 41.1 -> 19.0 and 43.7 -> 41.8, 8,000: 39.7 -> 23.2 and 39.9 -> 47.5,
+// 13,824: 43.6 -> 31.3, 20,480: 42.3 -> 49.5; hence the two lines.  Four warps a
+// block: 22.9 and 29.3 at 1,000, 28.1 and 45.5 at 13,824.
+constexpr int kPartWarps = 8;
+constexpr int kPartThreads = kPartWarps * kWarp;
+constexpr index_t kPartSums = 12288;  // the largest set summed in parts
+constexpr index_t kPartWalls = 2048;  // and its wall terms
+
+// The sums' slots first .. first + Count - 1 with one more entry.
+template <int First, int Count, int S>
+__device__ __forceinline__ void acc_part(double (&s)[Count], const Scaled& v) {
+  double all[S];
+#pragma unroll
+  for (int e = 0; e < S; ++e) all[e] = e >= First && e < First + Count ? s[e >= First && e < First + Count ? e - First : 0] : 0.0;
+  acc_monomials(all, v.x, v.y, v.z, v.w);
+  if (S > kMonomials) {
+    all[S - 4] += v.w;
+    all[S - 3] = fma(v.w, v.x, all[S - 3]);
+    all[S - 2] = fma(v.w, v.y, all[S - 2]);
+    all[S - 1] = fma(v.w, v.z, all[S - 1]);
+  }
+#pragma unroll
+  for (int e = 0; e < Count; ++e)
+    if (First + e < S) s[e] = all[First + e < S ? First + e : 0];
+}
+
+// f(integral_constant<int, warp>) for this thread's warp.
+template <int... P, typename F>
+__device__ __forceinline__ void by_warp(std::integer_sequence<int, P...>, F f) {
+  const int w = threadIdx.x / kWarp;
+  ((w == P ? f(std::integral_constant<int, P>{}) : void()), ...);
+}
+
+// The block's barrier, met by each warp in its own part's code.
+__device__ __forceinline__ void part_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kPartThreads) : "memory"); }
+
+// A round's shared values: [parity][entry of the round][component][particle].
+template <int Values>
+using PartStage = double[2][kPartWarps][Values][kWarp];
+
+// Walks the rows o .. e of the block's 32 particles (a lane's row; the same in all
+// warps): form(record and entry loads of a lane's entry, or of `none` past its end)
+// gives the values that the block shares, add(p) takes those of a round's entry p.
+// Rows' indices are loaded two rounds ahead, records one.
+template <int Values, typename Load, typename Form, typename Add>
+__device__ __forceinline__ void walk_in_parts(PartStage<Values>& stage, const index_t* __restrict__ indices, index_t o,
+                                              index_t e, index_t none, Load load, Form form, Add add) {
+  const int lane = threadIdx.x & (kWarp - 1), w = threadIdx.x / kWarp;
+  const int rounds = __reduce_max_sync(0xffffffffu, (e - o + kPartWarps - 1) / kPartWarps);
+  const auto index = [&](int r) {
+    const index_t at = o + r * kPartWarps + w;
+    return at < e ? indices[at] : none;
+  };
+  if (rounds == 0) return;
+  index_t j1 = index(1);
+  auto first = load(index(0));
+  auto next = load(j1);
+  index_t j2 = index(2);
+  double v[Values];
+  form(first, w < e - o, v);
+  for (int r = 0; r < rounds; ++r) {
+#pragma unroll
+    for (int k = 0; k < Values; ++k) stage[r & 1][w][k][lane] = v[k];
+    part_barrier();  // (two buffers: who writes the other one has passed this)
+    const auto now = next;
+    next = load(j2);
+    j2 = index(r + 3);
+    form(now, o + (r + 1) * kPartWarps + w < e, v);
+    add(stage[r & 1]);
+  }
+}
+
+template <bool TypeB>
+__global__ void __launch_bounds__(kPartThreads) plain_sums_parts_kernel(SumArgs a, const index_t* __restrict__ wo,
+                                                                        int32_t* __restrict__ walled,
+                                                                        unsigned* __restrict__ walls) {
+  wait_for_previous();
+  constexpr int S = TypeB ? kMonomialsB : kMonomials;
+  constexpr int kCount = (S + kPartWarps - 1) / kPartWarps;
+  __shared__ PartStage<4> stage;
+  const int lane = threadIdx.x & (kWarp - 1);
+  const index_t t = static_cast<index_t>(blockIdx.x) * kWarp + lane;
+  const bool live = t < a.n;
+  const index_t i = live ? visit(a.order, t) : 0;
+  if (wo && threadIdx.x < kWarp) list_walled(live && wo[i] < wo[i + 1], t, a.n, walled, walls);
+  const index_t self = live ? self_of(a.sorted, t, i) : 0;
+  const double4 pi = ld4(a.fp, self);
+  double s[kCount];
+#pragma unroll
+  for (int e = 0; e < kCount; ++e) s[e] = 0.0;
+  by_warp(std::make_integer_sequence<int, kPartWarps>{}, [&](auto part) {
+    constexpr int kFirst = decltype(part)::value * kCount;
+    walk_in_parts<4>(
+        stage, a.fi, live ? a.fo[i] : 0, live ? a.fo[i + 1] : 0, self, [&](index_t j) { return ld4(a.fp, j); },
+        [&](const double4& q, bool, double (&v)[4]) {
+          const Scaled f = scaled(q, pi, a.inv_re);
+          v[0] = f.x, v[1] = f.y, v[2] = f.z, v[3] = f.w;
+        },
+        [&](const double (&round)[kPartWarps][4][kWarp]) {
+#pragma unroll 2
+          for (int p = 0; p < kPartWarps; ++p)
+            acc_part<kFirst, kCount, S>(s, Scaled{round[p][0][lane], round[p][1][lane], round[p][2][lane], round[p][3][lane]});
+        });
+    if (!live) return;
+#pragma unroll
+    for (int e = 0; e < kCount; ++e)
+      if (kFirst + e < S) a.sums[static_cast<size_t>(kFirst + e) * a.n + t] = s[e];
+  });
+}
+
 struct WallArgs {
   index_t n;
   const double4* fp;
@@ -359,6 +480,21 @@ struct WallArgs {
   const int32_t* walled;
   const unsigned* walls;
 };
+
+// neumann<9> with its roundings fixed.
+template <int N>
+__device__ __forceinline__ void neumann_vector(double dx, double dy, double dz, const double4& nrm, double ir,
+                                               double (&q)[N]) {
+  q[0] = nrm.x;
+  q[1] = nrm.y;
+  q[2] = nrm.z;
+  q[3] = 2.0 * dx * nrm.x * ir;
+  q[4] = 2.0 * dy * nrm.y * ir;
+  q[5] = 2.0 * dz * nrm.z * ir;
+  q[6] = fma(dx, nrm.y, dy * nrm.x) * ir;
+  q[7] = fma(dy, nrm.z, dz * nrm.y) * ir;
+  q[8] = fma(dz, nrm.x, dx * nrm.z) * ir;
+}
 
 // The listed particles' sums with their wall terms, in row order, one thread to
 // a particle: the monomials with the Dirichlet samples, or the lower triangle of
@@ -418,10 +554,8 @@ __device__ __forceinline__ void wall_sums(const WallArgs& a) {
         const double d2 = length2_wall(dx, dy, dz);
         const double w = a.wall_scale * fma(-sqrt(d2), a.inv_re, 1.0);
         if (d2 <= 0.0 || w <= 0.0) continue;
-        // neumann<9> with its roundings fixed
-        const double ir = a.inv_re;
-        const double q9[9] = {nrm.x, nrm.y, nrm.z, 2.0 * dx * nrm.x * ir, 2.0 * dy * nrm.y * ir, 2.0 * dz * nrm.z * ir,
-                              fma(dx, nrm.y, dy * nrm.x) * ir, fma(dy, nrm.z, dz * nrm.y) * ir, fma(dz, nrm.x, dx * nrm.z) * ir};
+        double q9[9];
+        neumann_vector(dx, dy, dz, nrm, a.inv_re, q9);
 #pragma unroll
         for (int r = 0; r < 9; ++r) {
           const double wr = w * q9[r];
@@ -442,6 +576,115 @@ __global__ void __launch_bounds__(kWallThreads) wall_sums_kernel(WallArgs a, int
     wall_sums<false>(a);
   else
     wall_sums<true>(a);
+}
+
+// The lower triangle's entries first .. first + Count - 1, in the order of tri().
+template <int First, int Count>
+__device__ __forceinline__ void acc_wall_part(double (&m)[Count], double w, const double (&q9)[9]) {
+#pragma unroll
+  for (int r = 0; r < 9; ++r) {
+    const double wr = w * q9[r];
+#pragma unroll
+    for (int c = 0; c <= r; ++c) {
+      constexpr int kLast = First + Count;
+      if (tri(r, c) >= First && tri(r, c) < kLast) {
+        const int e = tri(r, c) - First;
+        m[e] = fma(wr, q9[c], m[e]);
+      }
+    }
+  }
+}
+
+// Entry e of the lower triangle's fluid part.
+__host__ __device__ constexpr int triangle_slot(int e) {
+  int r = 0;
+  while (e > r) e -= ++r;
+  return entry_slot(r, e);
+}
+
+// wall_sums_kernel in parts; blockIdx.y + first as there.
+__global__ void __launch_bounds__(kPartThreads) wall_sums_parts_kernel(WallArgs a, int first) {
+  wait_for_previous();
+  __shared__ PartStage<10> stage;
+  const int lane = threadIdx.x & (kWarp - 1);
+  const index_t many = static_cast<index_t>(*a.walls);
+  const size_t n = static_cast<size_t>(a.n);
+  const bool neumann = blockIdx.y + first != 0;
+  for (index_t g0 = static_cast<index_t>(blockIdx.x) * kWarp; g0 < many; g0 += static_cast<index_t>(gridDim.x) * kWarp) {
+    const bool live = g0 + lane < many;
+    const index_t t = a.walled[live ? g0 + lane : g0];
+    const index_t i = visit(a.order, t);
+    const double4 pi = ld4(a.fp, self_of(a.sorted, t, i));
+    const index_t o = a.wo[i], e = live ? a.wo[i + 1] : o;
+    const index_t none = a.wi[o];
+    by_warp(std::make_integer_sequence<int, kPartWarps>{}, [&](auto part) {
+      if (!neumann) {
+        constexpr int kCount = (kMonomials + kPartWarps - 1) / kPartWarps;
+        constexpr int kFirst = decltype(part)::value * kCount;
+        double s[kCount];
+#pragma unroll
+        for (int k = 0; k < kCount; ++k) s[k] = kFirst + k < kMonomials ? a.sums[(kFirst + k) * n + t] : 0.0;
+        walk_in_parts<10>(
+            stage, a.wi, o, e, none, [&](index_t j) { return ld4(a.wp, j); },
+            [&](const double4& q, bool in, double (&v)[10]) {
+              const Scaled f = scaled(q, pi, a.inv_re);
+              const double w = a.wall_scale * f.w;
+              const bool counts = in && w > 0.0;
+              v[0] = counts ? f.x : 0.0, v[1] = counts ? f.y : 0.0, v[2] = counts ? f.z : 0.0, v[3] = counts ? w : 0.0;
+            },
+            [&](const double (&round)[kPartWarps][10][kWarp]) {
+#pragma unroll 2
+              for (int p = 0; p < kPartWarps; ++p)
+                acc_part<kFirst, kCount, kMonomials>(
+                    s, Scaled{round[p][0][lane], round[p][1][lane], round[p][2][lane], round[p][3][lane]});
+            });
+        if (live) {
+#pragma unroll
+          for (int k = 0; k < kCount; ++k)
+            if (kFirst + k < kMonomials) a.velocity[(kFirst + k) * n + t] = s[k];
+        }
+      } else {
+        constexpr int kCount = (kWallEntries + kPartWarps - 1) / kPartWarps;
+        constexpr int kFirst = decltype(part)::value * kCount;
+        double m[kCount];
+#pragma unroll
+        for (int k = 0; k < kCount; ++k)
+          m[k] = kFirst + k < kWallEntries ? a.sums[triangle_slot(kFirst + k < kWallEntries ? kFirst + k : 0) * n + t] : 0.0;
+        struct Wall {
+          double4 q, n;
+        };
+        walk_in_parts<10>(
+            stage, a.wi, o, e, none, [&](index_t j) { return Wall{ld4(a.wp, j), ld4(a.wn, j)}; },
+            [&](const Wall& wall, bool in, double (&v)[10]) {
+              const double dx = wall.q.x - pi.x, dy = wall.q.y - pi.y, dz = wall.q.z - pi.z;
+              const double d2 = length2_wall(dx, dy, dz);
+              const double w = a.wall_scale * fma(-sqrt(d2), a.inv_re, 1.0);
+              const bool counts = in && !(d2 <= 0.0 || w <= 0.0);
+              neumann_vector(dx, dy, dz, wall.n, a.inv_re, v);
+              v[9] = w;
+              if (!counts) {
+#pragma unroll
+                for (int k = 0; k < 10; ++k) v[k] = 0.0;
+              }
+            },
+            [&](const double (&round)[kPartWarps][10][kWarp]) {
+#pragma unroll 2
+              for (int p = 0; p < kPartWarps; ++p) {
+                double q9[9];
+#pragma unroll
+                for (int k = 0; k < 9; ++k) q9[k] = round[p][k][lane];
+                acc_wall_part<kFirst, kCount>(m, round[p][9][lane], q9);
+              }
+            });
+        if (live) {
+#pragma unroll
+          for (int k = 0; k < kCount; ++k)
+            if (kFirst + k < kWallEntries) a.pressure[(kFirst + k) * n + t] = m[k];
+        }
+      }
+    });
+    __syncthreads();  // the stage's last round has been read
+  }
 }
 
 struct FinishArgs {
@@ -1195,6 +1438,15 @@ __global__ void __launch_bounds__(kRowThreads, 6) moment_mixed_split_kernel(SumA
 
 void launch_plain_sums(lsmps_ctx* ctx, const SumArgs& a, const index_t* wo, bool type_b) {
   const bool halves = ctx->knob[LSMPS_KNOB_MOMENT_OCCUPANCY] == 2;
+  if (!halves && a.n <= kPartSums) {
+    const auto parts = [&](const char* name, auto kernel) {
+      launch_named(ctx, name, kernel, dim3(div_up(a.n, kWarp)), dim3(kPartThreads), 0, a, wo, ctx->moment_walled,
+                   ctx->moment_walls);
+    };
+    type_b ? parts("plain_sums_parts_kernel<B>", plain_sums_parts_kernel<true>)
+           : parts("plain_sums_parts_kernel", plain_sums_parts_kernel<false>);
+    return;
+  }
   const auto queue = [&](const char* name, auto kernel) {
     launch_named(ctx, name, kernel, dim3(div_up((halves ? 2LL : 1LL) * a.n, kSumThreads)), dim3(kSumThreads), 0, a, wo,
                  ctx->moment_walled, ctx->moment_walls);
@@ -1385,9 +1637,14 @@ lsmps_status prepare_moments_impl(lsmps_ctx* ctx, const lsmps_fluid& fluid, cons
     const WallArgs wa{n, ctx->pack_fluid[0], ctx->pack_wall[0], ctx->pack_wall[2], wn.offsets, wn.indices,
                       1.0 / p.support_radius, p.lsmps_wall_weight_scale, ctx->moment_sums, wall_velocity, wall_pressure,
                       ctx->order, srows ? 1 : 0, ctx->moment_walled, ctx->moment_walls};
-    const int blocks = std::min(div_up(n, kWallThreads), ctx->sm_count * 12);
-    launch(ctx, wall_sums_kernel, dim3(blocks, (dirichlet ? 1 : 0) + (neumann_terms ? 1 : 0)), dim3(kWallThreads), 0,
-           wa, dirichlet ? 0 : 1);
+    const int kinds_on = (dirichlet ? 1 : 0) + (neumann_terms ? 1 : 0);
+    const int groups = div_up(n, kWarp);
+    if (n <= kPartWalls)
+      launch(ctx, wall_sums_parts_kernel, dim3(std::min(groups, ctx->sm_count * 4), kinds_on), dim3(kPartThreads), 0, wa,
+             dirichlet ? 0 : 1);
+    else
+      launch(ctx, wall_sums_kernel, dim3(std::min(groups, ctx->sm_count * 12), kinds_on), dim3(kWallThreads), 0, wa,
+             dirichlet ? 0 : 1);
   }
   a9 = FinishArgs{n, ctx->moment_sums, wall_velocity, wall_pressure, wn.offsets, p.lsmps_regularization,
                   {},  ctx->d_status,     ctx->order,    ctx->moment_walls};
