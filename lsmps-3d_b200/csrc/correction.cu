@@ -874,67 +874,162 @@ __global__ void __launch_bounds__(kThreads, 6) gradient32_kernel(GatherArgs a, G
   }
 }
 
-// update_velocity_position_kernel followed by anti_penetration_kernel for the
-// same particle: the anti-penetration pass reads only the particle's own
-// updated state and the walls, so running it right after the update in the
-// same thread gives the same result as the two reference kernels.
-__global__ void __launch_bounds__(kThreads) update_anti_penetration_kernel(
-    lsmps_fluid f, const index_t* __restrict__ wo, const index_t* __restrict__ wi,
-    const double* __restrict__ tx, const double* __restrict__ ty, const double* __restrict__ tz, double dt_host,
-    const double* __restrict__ dtp, double density, const double* __restrict__ gx, const double* __restrict__ gy, const double* __restrict__ gz,
-    const double* __restrict__ sx, const double* __restrict__ sy, const double* __restrict__ sz, double clearance,
-    const double4* __restrict__ wp, const double4* __restrict__ wn) {
-  wait_for_previous();
-  const index_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= static_cast<index_t>(f.count)) return;
-  const double dt = dtp ? *dtp : dt_host;
-  const bool splash = is_splash(f.surface_type, i);
-  const double ox = f.vx[i], oy = f.vy[i], oz = f.vz[i];
-  double vx = tx[i], vy = ty[i], vz = tz[i];
-  if (!splash) {
-    const double ps = dt / density;
-    vx -= ps * gx[i];
-    vy -= ps * gy[i];
-    vz -= ps * gz[i];
+struct UpdateArgs {
+  lsmps_fluid f;
+  const index_t* wo;
+  const index_t* wi;
+  const double *tx, *ty, *tz;  // u*
+  double dt_host;
+  const double* dtp;
+  double density;
+  const double *gx, *gy, *gz;  // pressure gradient
+  const double *sx, *sy, *sz;  // shifting
+  double clearance;
+  const double4* wp;  // wall records {x, y, z, -} and {nx, ny, nz, -}
+  const double4* wn;
+};
+
+// Position and velocity of one particle.
+struct Moving {
+  double x, y, z, vx, vy, vz;
+};
+
+__device__ __forceinline__ void store(const lsmps_fluid& f, index_t i, const Moving& m) {
+  f.x[i] = m.x;
+  f.y[i] = m.y;
+  f.z[i] = m.z;
+  f.vx[i] = m.vx;
+  f.vy[i] = m.vy;
+  f.vz[i] = m.vz;
+}
+
+// One wall, `sd` away: the particle out to the clearance, its velocity towards the
+// wall taken off.
+__device__ __forceinline__ void push(Moving& m, double c, double nx, double ny, double nz) {
+  m.x += c * nx;
+  m.y += c * ny;
+  m.z += c * nz;
+  const double nv = m.vx * nx + m.vy * ny + m.vz * nz;
+  if (nv < 0.0) {
+    m.vx -= nv * nx;
+    m.vy -= nv * ny;
+    m.vz -= nv * nz;
   }
-  double x = f.x[i], y = f.y[i], z = f.z[i];
-  x += 0.5 * dt * (ox + vx) + sx[i];
-  y += 0.5 * dt * (oy + vy) + sy[i];
-  z += 0.5 * dt * (oz + vz) + sz[i];
-  if (clearance > 0.0 && wo[i] < wo[i + 1]) {
-    // the wall records {x, y, z, -} and {nx, ny, nz, -}, the next wall's
-    // loaded while this one is applied (in row order)
-    const index_t wb = wo[i], we = wo[i + 1];
-    index_t jn = wi[wb];
-    double4 qn = ld4(wp, jn), nn = ld4(wn, jn);
-    for (index_t o = wb; o < we; ++o) {
-      const double4 q = qn, nrm = nn;
-      if (o + 1 < we) {
-        jn = wi[o + 1];
-        qn = ld4(wp, jn);
-        nn = ld4(wn, jn);
-      }
-      const double nx = nrm.x, ny = nrm.y, nz = nrm.z;
-      const double sd = (x - q.x) * nx + (y - q.y) * ny + (z - q.z) * nz;
-      if (sd >= clearance) continue;
-      const double c = clearance - sd;
-      x += c * nx;
-      y += c * ny;
-      z += c * nz;
-      const double nv = vx * nx + vy * ny + vz * nz;
-      if (nv < 0.0) {
-        vx -= nv * nx;
-        vy -= nv * ny;
-        vz -= nv * nz;
-      }
+}
+
+__device__ __forceinline__ double wall_distance(const Moving& m, const double4& q, const double4& nrm) {
+  return (m.x - q.x) * nrm.x + (m.y - q.y) * nrm.y + (m.z - q.z) * nrm.z;
+}
+
+// The walls wb .. we of one particle in row order, by its own thread, the next
+// wall's records loaded while this one is applied.
+__device__ __forceinline__ void push_from_walls_alone(const UpdateArgs& a, index_t wb, index_t we, Moving& m) {
+  index_t jn = a.wi[wb];
+  double4 qn = ld4(a.wp, jn), nn = ld4(a.wn, jn);
+  for (index_t o = wb; o < we; ++o) {
+    const double4 q = qn, nrm = nn;
+    if (o + 1 < we) {
+      jn = a.wi[o + 1];
+      qn = ld4(a.wp, jn);
+      nn = ld4(a.wn, jn);
+    }
+    const double sd = wall_distance(m, q, nrm);
+    if (sd >= a.clearance) continue;
+    push(m, a.clearance - sd, nrm.x, nrm.y, nrm.z);
+  }
+}
+
+// The same by a group of kWallLanes lanes: each lane tests one wall against the present state; the first
+// that is too close is applied and the walls after it are tested again.  Few are,
+// so most of a row passes eight walls at a time, with the next eight's records
+// loaded meanwhile.
+constexpr int kWallLanes = 8;
+
+__device__ __forceinline__ void push_from_walls(const UpdateArgs& a, index_t wb, index_t we, Moving& m) {
+  const unsigned mask = group_mask<kWallLanes>();
+  const int l = threadIdx.x & (kWallLanes - 1);
+  const int first_lane = (threadIdx.x & (kWarp - 1)) & ~(kWallLanes - 1);
+  const index_t none = a.wi[wb];
+  index_t jn = wb + l < we ? a.wi[wb + l] : none;
+  double4 qn = ld4(a.wp, jn), nn = ld4(a.wn, jn);
+  jn = wb + kWallLanes + l < we ? a.wi[wb + kWallLanes + l] : none;
+  for (index_t o = wb; o < we; o += kWallLanes) {
+    const double4 q = qn, nrm = nn;
+    qn = ld4(a.wp, jn);
+    nn = ld4(a.wn, jn);
+    jn = o + 2 * kWallLanes + l < we ? a.wi[o + 2 * kWallLanes + l] : none;
+    for (int from = 0;;) {
+      const double sd = wall_distance(m, q, nrm);
+      const bool close = l >= from && o + l < we && !(sd >= a.clearance);
+      const unsigned hits = __ballot_sync(mask, close) >> first_lane & ((1u << kWallLanes) - 1u);
+      if (!hits) break;
+      const int k = __ffs(hits) - 1;
+      const double nx = __shfl_sync(mask, nrm.x, k, kWallLanes), ny = __shfl_sync(mask, nrm.y, k, kWallLanes),
+                   nz = __shfl_sync(mask, nrm.z, k, kWallLanes);
+      push(m, a.clearance - __shfl_sync(mask, sd, k, kWallLanes), nx, ny, nz);
+      from = k + 1;
     }
   }
-  f.x[i] = x;
-  f.y[i] = y;
-  f.z[i] = z;
-  f.vx[i] = vx;
-  f.vy[i] = vy;
-  f.vz[i] = vz;
+}
+
+// update_velocity_position_kernel followed by anti_penetration_kernel for the
+// same particle: the anti-penetration pass reads only the particle's own
+// updated state and the walls, so running it right after the update gives the
+// same result as the two reference kernels.
+constexpr int kUpdateThreads = 128;
+
+__device__ __forceinline__ Moving moved(const UpdateArgs& a, index_t i) {
+  const lsmps_fluid& f = a.f;
+  const double dt = a.dtp ? *a.dtp : a.dt_host;
+  const bool splash = is_splash(f.surface_type, i);
+  const double ox = f.vx[i], oy = f.vy[i], oz = f.vz[i];
+  double vx = a.tx[i], vy = a.ty[i], vz = a.tz[i];
+  if (!splash) {
+    const double ps = dt / a.density;
+    vx -= ps * a.gx[i];
+    vy -= ps * a.gy[i];
+    vz -= ps * a.gz[i];
+  }
+  double x = f.x[i], y = f.y[i], z = f.z[i];
+  x += 0.5 * dt * (ox + vx) + a.sx[i];
+  y += 0.5 * dt * (oy + vy) + a.sy[i];
+  z += 0.5 * dt * (oz + vz) + a.sz[i];
+  return Moving{x, y, z, vx, vy, vz};
+}
+
+__global__ void __launch_bounds__(kThreads) update_anti_penetration_kernel(const __grid_constant__ UpdateArgs a) {
+  wait_for_previous();
+  const index_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= static_cast<index_t>(a.f.count)) return;
+  Moving m = moved(a, i);
+  if (a.clearance > 0.0 && a.wo[i] < a.wo[i + 1]) push_from_walls_alone(a, a.wo[i], a.wo[i + 1], m);
+  store(a.f, i, m);
+}
+
+// For sets of at most kSmallUpdate particles, where the latency of index, record
+// and test per wall is what it takes: a block moves as many particles as it has
+// lane groups, a thread each, and then takes those of them with walls a group
+// each.  Event times: 1,000 particles 31 -> 13 us, 21,793: 33 -> 16, 61,250: 41 ->
+// 25; 500,000: 72 against 120, 2,000,000: 143 against 400 (blocks of 128 particles
+// there: 82 and 150).
+constexpr size_t kSmallUpdate = 131072;
+constexpr int kUpdateGroups = kUpdateThreads / kWallLanes;
+
+__global__ void __launch_bounds__(kUpdateThreads) update_anti_penetration_small_kernel(
+    const __grid_constant__ UpdateArgs a) {
+  wait_for_previous();
+  __shared__ Moving s_moving[kUpdateGroups];
+  const index_t i0 = static_cast<index_t>(blockIdx.x) * kUpdateGroups;
+  const index_t n = static_cast<index_t>(a.f.count);
+  const index_t mine = i0 + threadIdx.x;
+  if (threadIdx.x < kUpdateGroups && mine < n) s_moving[threadIdx.x] = moved(a, mine);
+  __syncthreads();
+  const int g = threadIdx.x / kWallLanes;
+  const index_t i = i0 + g;
+  if (i >= n) return;  // the whole group
+  Moving m = s_moving[g];
+  if (a.clearance > 0.0 && a.wo[i] < a.wo[i + 1]) push_from_walls(a, a.wo[i], a.wo[i + 1], m);
+  if ((threadIdx.x & (kWallLanes - 1)) == 0) store(a.f, i, m);
 }
 
 // gradient_shifting_kernel with the context's lane count (LSMPS_KNOB_GATHER_LANES).
@@ -1036,14 +1131,15 @@ lsmps_status pressure_correction_impl(lsmps_ctx* ctx, const lsmps_fluid& f, cons
   if (f.count == 0) return LSMPS_OK;
   st = gradient_shifting_stage(ctx, f, w, fn, wn, pressure, p, pm, g, s, mixed);
   if (st) return st;
-  const int blocks = div_up(static_cast<long long>(f.count), kThreads);
-  launch(ctx, update_anti_penetration_kernel, dim3(blocks), dim3(kThreads), 0, f,
-         static_cast<const index_t*>(wn.offsets), static_cast<const index_t*>(wn.indices),
-         static_cast<const double*>(t.vx), static_cast<const double*>(t.vy), static_cast<const double*>(t.vz),
-         p.time_step, ctx->device_dt, p.density, static_cast<const double*>(g.x), static_cast<const double*>(g.y),
-         static_cast<const double*>(g.z), static_cast<const double*>(s.x), static_cast<const double*>(s.y),
-         static_cast<const double*>(s.z), p.wall_clearance_ratio * p.particle_spacing,
-         static_cast<const double4*>(ctx->pack_wall[0]), static_cast<const double4*>(ctx->pack_wall[2]));
+  const UpdateArgs u{f,   wn.offsets, wn.indices, t.vx, t.vy, t.vz, p.time_step, ctx->device_dt, p.density, g.x, g.y, g.z,
+                     s.x, s.y,        s.z,        p.wall_clearance_ratio * p.particle_spacing, ctx->pack_wall[0],
+                     ctx->pack_wall[2]};
+  if (f.count <= kSmallUpdate)
+    launch(ctx, update_anti_penetration_small_kernel, dim3(div_up(static_cast<long long>(f.count), kUpdateGroups)),
+           dim3(kUpdateThreads), 0, u);
+  else
+    launch(ctx, update_anti_penetration_kernel, dim3(div_up(static_cast<long long>(f.count), kThreads)), dim3(kThreads), 0,
+           u);
   st = check_launch(ctx, "gradient/shifting, update/anti-penetration");
   if (!st) st = smooth_impl(ctx, f, fn, p, sm, true);
   return st;

@@ -58,6 +58,8 @@ def kernel_bytes(nf: int, nw: int, kf: int, kw: int, c: int, s: int = 8) -> dict
     for g in (1, 2):
         out[f"plain_sums_kernel<{g}>"] = 8 * (nf + 1) + 4 * kf + pos_f + sums
     out["wall_sums_kernel"] = moment_in - 4 * kf + 2 * sums
+    out["plain_sums_parts_kernel"] = out["plain_sums_kernel<1>"]
+    out["wall_sums_parts_kernel"] = out["wall_sums_kernel"]
     out["moment_finish_kernel<9>"] = 2 * (sums + moment_kind_out)
     lap = rows + 2 * pos_f + 2 * pos_w + 3 * s * nf
     # the two mixed stages in one kernel (row halves on two warps)
@@ -81,6 +83,7 @@ def kernel_bytes(nf: int, nw: int, kf: int, kw: int, c: int, s: int = 8) -> dict
                                         + 2 * (36 * 4 + 2 * s + 4) * nf)
     out["update_anti_penetration_kernel"] = (4 * (nf + 1) + 4 * kw + 4 * nf + 2 * pos_f + 3 * pos_f
                                              + 2 * pos_w + 2 * pos_f)
+    out["update_anti_penetration_small_kernel"] = out["update_anti_penetration_kernel"]
     out["smooth_kernel"] = 4 * (nf + 1) + 4 * kf + 2 * pos_f + 4 * nf + pos_f
     out["copy_kernel"] = 2 * pos_f
     # lane-parallel variants (LSMPS_KNOB_GATHER_LANES) move the same bytes

@@ -11,8 +11,8 @@ pytestmark = pytest.mark.gpu
 KEYS = ("inverse_matrices", "moment_trace", "regularization_added", "info")
 
 
-def moments(pkg, ctx, host, params, n, copies, kinds):
-    """The matrices of the first n particles of `host` (rows cut to entries below n), `copies` times over."""
+def repeated(pkg, host, n, copies):
+    """Device buffers of the first n particles of `host` (rows cut to entries below n), `copies` times over."""
     def rows(table, keep):
         o, i = host.csr_rows(table)
         o, i = o[: n + 1], i[: o[n]]
@@ -34,6 +34,11 @@ def moments(pkg, ctx, host, params, n, copies, kinds):
     put(dev.fluid_neighbors["indices"], (np.tile(fi, copies) + n * np.repeat(np.arange(copies), len(fi))).astype(np.int32))
     put(dev.wall_neighbors["offsets"], np.concatenate([[0], np.cumsum(np.tile(wc, copies))]).astype(np.int32))
     put(dev.wall_neighbors["indices"], np.tile(wi, copies).astype(np.int32))
+    return dev
+
+
+def moments(pkg, ctx, host, params, n, copies, kinds):
+    dev = repeated(pkg, host, n, copies)
     ctx.prepare_moments(dev, params, kinds)
     return {k: {f: dev.alloc.to_numpy(dev.moments[k][f]) for f in KEYS} for k in kinds}
 
