@@ -914,8 +914,11 @@ __device__ __forceinline__ void monomial_pairs(f32x2 (&t)[16], float sx, float s
   t[15] = pack2(wzz * low_half(q1), 0.0f);                // wzz qxx
 }
 
-__global__ void __launch_bounds__(kSumThreads) moment_sums_kernel(SumArgs a) {
+// (also clears the counts of the lists of FP64-route particles that the rows'
+// kernel fills: a memset between two kernels costs their overlap)
+__global__ void __launch_bounds__(kSumThreads) moment_sums_kernel(SumArgs a, unsigned* __restrict__ lists) {
   wait_for_previous();
+  if (blockIdx.x == 0 && threadIdx.x < 4) lists[threadIdx.x] = 0u;
   const index_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= a.n) return;
   const index_t i = visit(a.order, t);
@@ -1508,8 +1511,7 @@ lsmps_status launch_mixed(lsmps_ctx* ctx, index_t n, const lsmps_csr& fn, const 
     ra.list[k] = ctx->mixed_list[k];
   }
   ra.count = ctx->mixed_count;
-  // the lists of FP64-route particles start empty every time
-  cudaMemsetAsync(ctx->mixed_count, 0, 4 * sizeof(unsigned int), ctx->stream);
+  // (the lists of FP64-route particles start empty every time)
   ra.status = ctx->d_status;
   ra.order = ctx->order;
   auto pack_walls = [&]() {
@@ -1519,6 +1521,7 @@ lsmps_status launch_mixed(lsmps_ctx* ctx, index_t n, const lsmps_csr& fn, const 
     pack_wall_normals(ctx, walls);
   };
   if (split) {
+    cudaMemsetAsync(ctx->mixed_count, 0, 4 * sizeof(unsigned int), ctx->stream);
     pack_walls();
     // one kernel: row halves on two warps, one kind per warp
     if (full)
@@ -1527,7 +1530,7 @@ lsmps_status launch_mixed(lsmps_ctx* ctx, index_t n, const lsmps_csr& fn, const 
       launch(ctx, moment_mixed_split_kernel<false>, dim3(div_up(n, kWarp)), dim3(kRowThreads), 0, sa, ra);
     return LSMPS_OK;
   }
-  launch(ctx, moment_sums_kernel, dim3(div_up(n, kSumThreads)), dim3(kSumThreads), 0, sa);
+  launch(ctx, moment_sums_kernel, dim3(div_up(n, kSumThreads)), dim3(kSumThreads), 0, sa, ctx->mixed_count);
   pack_walls();
   const dim3 grid(div_up(n, kRowThreads), 2);
   if (full)
