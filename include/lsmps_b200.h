@@ -8,8 +8,8 @@
  * size_type = size_t), so a reference view can be passed by address.
  *
  * Memory: every device pointer in a view is owned by the caller.  The opaque
- * context owns only scratch (radix-sort ping-pong buffers, scan partials, the
- * device status word) and the CUDA stream the work is queued on.
+ * context owns only scratch (sort and scan buffers, moment sums, the device
+ * status word) and the CUDA stream the work is queued on.
  *
  * Errors: no entry point exits the process.  Each returns an lsmps_status; a
  * human-readable message for the last failure is available from
