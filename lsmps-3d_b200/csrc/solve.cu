@@ -312,13 +312,16 @@ __global__ void __launch_bounds__(kSolveThreads) project_kernel(SolveArgs a, int
 // w -= sum_k h2[k] v_k and its norm; the last block extends the Hessenberg
 // matrix by column j and applies the previous rotations and the one that zeroes
 // its subdiagonal.
+// (h2 is padded with zeros to K: with the additions under k <= j
+// each load waited for the one before it, 83 us at 2,000,000 rows against 49 of
+// project_kernel; 500,000 rows: a solve 17.8 -> 17.3 ms)
 template <int K>
 __global__ void __launch_bounds__(kSolveThreads) extend_kernel(SolveArgs a, int j) {
   wait_for_previous();
   SolveState* st = a.st;
   if (st->stop) return;
   __shared__ double sh[kMaxRestart + 1];
-  for (int k = threadIdx.x; k <= j; k += kSolveThreads) sh[k] = st->h2[k];
+  for (int k = threadIdx.x; k < K; k += kSolveThreads) sh[k] = k <= j ? st->h2[k] : 0.0;
   __syncthreads();
   double* __restrict__ w = a.w[(j + 1) & 1];
   double acc = 0.0;
@@ -327,8 +330,7 @@ __global__ void __launch_bounds__(kSolveThreads) extend_kernel(SolveArgs a, int 
 #pragma unroll
     for (int k = 0; k < K; ++k) v[k] = k <= j ? a.V[static_cast<size_t>(k) * a.ldv + i] : 0.0;
 #pragma unroll
-    for (int k = 0; k < K; ++k)
-      if (k <= j) wi = fma(-sh[k], v[k], wi);
+    for (int k = 0; k < K; ++k) wi = fma(-sh[k], v[k], wi);
     w[i] = wi;
     acc = fma(wi, wi, acc);
   }
