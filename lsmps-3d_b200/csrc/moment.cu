@@ -447,8 +447,9 @@ __global__ void __launch_bounds__(kPartThreads) plain_sums_parts_kernel(SumArgs 
     constexpr int kFirst = decltype(part)::value * kCount;
     walk_in_parts<4>(
         stage, a.fi, live ? a.fo[i] : 0, live ? a.fo[i + 1] : 0, self, [&](index_t j) { return ld4(a.fp, j); },
-        [&](const double4& q, bool, double (&v)[4]) {
-          const Scaled f = scaled(q, pi, a.inv_re);
+        [&](const double4& q, bool in, double (&v)[4]) {
+          // (own position: at distance 0, but NaN from itself where it is not finite)
+          const Scaled f = in ? scaled(q, pi, a.inv_re) : Scaled{0.0, 0.0, 0.0, 0.0};
           v[0] = f.x, v[1] = f.y, v[2] = f.z, v[3] = f.w;
         },
         [&](const double (&round)[kPartWarps][4][kWarp]) {
