@@ -266,7 +266,9 @@ __global__ void __launch_bounds__(kSurfaceThreads) classify_small_kernel(Surface
     double4 q = b + l < e ? ld4(rec, idx[b + l]) : own;
     index_t jn = b + G + l < e ? idx[b + G + l] : -1;
     for (index_t o = b; o < e; o += G) {
-      const Term v = term_of(q, own, re);  // (none past the row's end: own, at distance 0)
+      // none past the row's end, where the record is the particle's own (at distance
+      // 0, but NaN from itself where it is not finite)
+      const Term v = o + l < e ? term_of(q, own, re) : Term{0.0, 0.0, 0.0, 0.0, 0.0, 0};
       q = jn >= 0 ? ld4(rec, jn) : own;
       jn = o + 2 * G + l < e ? idx[o + 2 * G + l] : -1;
       weighted += v.counted;

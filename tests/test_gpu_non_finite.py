@@ -48,3 +48,22 @@ def test_moments_of_an_empty_row(pkg, device_api, bad, kind, n):
     inverse = dev.alloc.to_numpy(m["inverse_matrices"])[2 * size * size:3 * size * size].reshape(size, size)
     assert dev.alloc.to_numpy(m["moment_trace"])[2] == 0.0 and dev.alloc.to_numpy(m["info"])[2] == 0
     assert np.allclose(inverse, np.eye(size) / p.lsmps_regularization, rtol=1e-15, atol=0.0)
+
+
+@pytest.mark.parametrize("n", [3, 131073], ids=["lanes", "threads"])
+def test_label_sums_beyond_the_radius(pkg, device_api, n):
+    # particle 2 is infinitely far from the one neighbour of its row: no weight, no sum
+    import torch
+
+    x = np.zeros(n)
+    x[1], x[2] = 0.25, np.inf
+    dev, p = buffers(pkg, x, [[1], [0], [0]] + [[] for _ in range(n - 3)])
+    names = [k for k, _ in pkg.abi.SurfaceDiagnostics._fields_]
+    out = {k: torch.full((n,), 7, dtype=torch.int32 if "count" in k else torch.float64, device="cuda") for k in names}
+    ctx = device_api.Context(0)
+    try:
+        ctx.classify_surface(dev, p, pkg.abi.SurfaceDiagnostics(*(out[k].data_ptr() for k in names)))
+    finally:
+        ctx.close()
+    assert [float(out[k][2]) for k in ("number_density", "number_density_ratio", "anisotropy")] == [0.0, 0.0, 0.0]
+    assert float(out["number_density"][0]) == float(out["number_density"][1]) > 0.0
