@@ -531,7 +531,7 @@ __device__ __forceinline__ void wall_sums(const WallArgs& a) {
         if (o + 3 < we) j2 = a.wi[o + 3];
         const Scaled next = scaled(q, pi, a.inv_re);
         const double w = a.wall_scale * v.w;
-        if (w > 0.0) acc_monomials(s, v.x, v.y, v.z, w);
+        if (!(w <= 0.0)) acc_monomials(s, v.x, v.y, v.z, w);  // (NaN is added)
         v = next;
       }
 #pragma unroll
@@ -630,7 +630,7 @@ __global__ void __launch_bounds__(kPartThreads) wall_sums_parts_kernel(WallArgs 
             [&](const double4& q, bool in, double (&v)[10]) {
               const Scaled f = scaled(q, pi, a.inv_re);
               const double w = a.wall_scale * f.w;
-              const bool counts = in && w > 0.0;
+              const bool counts = in && !(w <= 0.0);  // (NaN is added)
               v[0] = counts ? f.x : 0.0, v[1] = counts ? f.y : 0.0, v[2] = counts ? f.z : 0.0, v[3] = counts ? w : 0.0;
             },
             [&](const double (&round)[kPartWarps][10][kWarp]) {

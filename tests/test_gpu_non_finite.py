@@ -67,3 +67,20 @@ def test_label_sums_beyond_the_radius(pkg, device_api, n):
         ctx.close()
     assert [float(out[k][2]) for k in ("number_density", "number_density_ratio", "anisotropy")] == [0.0, 0.0, 0.0]
     assert float(out["number_density"][0]) == float(out["number_density"][1]) > 0.0
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2])
+@pytest.mark.parametrize("n", [2, 2049], ids=["parts", "threads"])
+def test_moments_beside_a_wall_at_nan(pkg, device_api, kind, n):
+    # the matrix of a particle that lists such a wall is NaN (info: the first pivot is not positive); others are not
+    rows = [[1], [0]] + [[] for _ in range(n - 2)]
+    dev, p = buffers(pkg, [0.0, 0.25] + [0.0] * (n - 2), rows, [-0.25, np.nan], [[0, 1, 0], [0, 0]] + [[] for _ in range(n - 2)])
+    ctx = device_api.Context(0)
+    try:
+        ctx.prepare_moments(dev, p, [kind])
+    finally:
+        ctx.close()
+    m = dev.moments[kind]
+    trace, info = dev.alloc.to_numpy(m["moment_trace"]), dev.alloc.to_numpy(m["info"])
+    assert np.isnan(trace[0]) and info[0] != 0
+    assert np.isfinite(trace[1:]).all() and info[1] == 0
