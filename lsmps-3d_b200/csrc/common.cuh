@@ -294,7 +294,7 @@ struct lsmps_ctx {
   // boundaries ([31][n], then [45][n]), all by visiting position.
   double* moment_sums = nullptr;
   int32_t* moment_walled = nullptr;   // plain form: visiting positions of the particles with walls
-  unsigned int* moment_walls = nullptr;  // ... and how many (0 between calls)
+  unsigned int* moment_walls = nullptr;  // ... and how many (cleared by each call's fluid pack)
   size_t moment_cap = 0;
   // Mixed form (LSMPS_PRECISION_MIXED): per fluid particle the compact FP32
   // operator rows of the velocity

@@ -91,7 +91,6 @@ bool ensure_moment_sums(lsmps_ctx* ctx, size_t nf) {
   }
   ctx->moment_walls = reinterpret_cast<unsigned int*>(ctx->moment_sums + doubles);
   ctx->moment_walled = reinterpret_cast<int32_t*>(ctx->moment_walls + 1);
-  cudaMemsetAsync(ctx->moment_walls, 0, sizeof(unsigned int), ctx->stream);
   ctx->moment_cap = nf;
   return true;
 }

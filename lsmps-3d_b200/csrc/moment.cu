@@ -506,7 +506,7 @@ __device__ __forceinline__ void neumann_vector(double dx, double dy, double dz, 
 // long, and looking for walls from every particle's lanes 0.27.
 template <bool Neumann>
 __device__ __forceinline__ void wall_sums(const WallArgs& a) {
-  const index_t many = static_cast<index_t>(*a.walls);
+  const index_t many = static_cast<index_t>(min(*a.walls, static_cast<unsigned>(a.n)));
   const size_t n = static_cast<size_t>(a.n);
   for (index_t g = blockIdx.x * blockDim.x + threadIdx.x; g < many; g += gridDim.x * blockDim.x) {
     const index_t t = a.walled[g];
@@ -608,7 +608,7 @@ __global__ void __launch_bounds__(kPartThreads) wall_sums_parts_kernel(WallArgs 
   wait_for_previous();
   __shared__ PartStage<10> stage;
   const int lane = threadIdx.x & (kWarp - 1);
-  const index_t many = static_cast<index_t>(*a.walls);
+  const index_t many = static_cast<index_t>(min(*a.walls, static_cast<unsigned>(a.n)));
   const size_t n = static_cast<size_t>(a.n);
   const bool neumann = blockIdx.y + first != 0;
   for (index_t g0 = static_cast<index_t>(blockIdx.x) * kWarp; g0 < many; g0 += static_cast<index_t>(gridDim.x) * kWarp) {
@@ -698,7 +698,6 @@ struct FinishArgs {
   KindOut k[3];
   DeviceStatus* status;
   const int32_t* order;
-  unsigned* walls;  // emptied for the next call's list
 };
 
 // X = L^-T L^-1 in place of the inverted factor (lower triangles): row r of X
@@ -773,10 +772,7 @@ __global__ void __launch_bounds__(kFinishThreads, N == 9 ? 16 : 10) moment_finis
   __shared__ double s_stage[27][kWarp + 1];
   const KindOut& ko = a.k[blockIdx.y];
   const index_t t = blockIdx.x * kFinishThreads + threadIdx.x;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    if (ko.count) atomicAdd(ko.count, 1);
-    if (blockIdx.y == 0) *a.walls = 0u;
-  }
+  if (blockIdx.x == 0 && threadIdx.x == 0 && ko.count) atomicAdd(ko.count, 1);
   const unsigned active = __ballot_sync(0xffffffffu, t < a.n);
   if (t >= a.n) return;
   const index_t i = visit(a.order, t);
@@ -1598,8 +1594,10 @@ lsmps_status prepare_moments_impl(lsmps_ctx* ctx, const lsmps_fluid& fluid, cons
                    mk.inversion_count};
   };
   if (!ensure_packs(ctx, fluid.count, walls.count)) return fail(ctx, LSMPS_CUDA_ERROR, "pack allocation failed");
+  if (!ensure_moment_sums(ctx, fluid.count)) return fail(ctx, LSMPS_CUDA_ERROR, "moment sums allocation failed");
   const index_t* srows = sorted_rows_of(ctx, fn, fluid.count);
-  pack_fluid_positions(ctx, fluid, srows ? ctx->order : nullptr);
+  // (the list of particles with walls starts empty every time)
+  pack_fluid_positions(ctx, fluid, srows ? ctx->order : nullptr, ctx->moment_walls);
   const bool fused = velocity_a >= 0 && pressure_a >= 0;
   const bool mixed = fused && ctx->precision == LSMPS_PRECISION_MIXED;
   if (mixed) {
@@ -1626,7 +1624,6 @@ lsmps_status prepare_moments_impl(lsmps_ctx* ctx, const lsmps_fluid& fluid, cons
     ++(kinds[k].kind == LSMPS_MOMENT_PRESSURE_WALL_NEUMANN_B ? many10 : many9);
   }
   if (many9 + many10 == 0) return check_launch(ctx, "moment matrices");
-  if (!ensure_moment_sums(ctx, fluid.count)) return fail(ctx, LSMPS_CUDA_ERROR, "moment sums allocation failed");
   const size_t cap = ctx->moment_cap;
   double* wall_velocity = ctx->moment_sums + cap * kMonomialsB;
   double* wall_pressure = wall_velocity + cap * kMonomials;
@@ -1651,7 +1648,7 @@ lsmps_status prepare_moments_impl(lsmps_ctx* ctx, const lsmps_fluid& fluid, cons
              dirichlet ? 0 : 1);
   }
   a9 = FinishArgs{n, ctx->moment_sums, wall_velocity, wall_pressure, wn.offsets, p.lsmps_regularization,
-                  {},  ctx->d_status,     ctx->order,    ctx->moment_walls};
+                  {},  ctx->d_status,     ctx->order};
   a10 = a9;
   many9 = many10 = 0;
   for (int k = 0; k < count; ++k) {

@@ -5,8 +5,9 @@ namespace lsmps {
 
 __global__ void pack4_kernel(const double* __restrict__ a, const double* __restrict__ b,
                              const double* __restrict__ c, const double* __restrict__ d, index_t n,
-                             double4* __restrict__ out, const index_t* __restrict__ order) {
+                             double4* __restrict__ out, const index_t* __restrict__ order, unsigned* zero) {
   wait_for_previous();
+  if (zero && blockIdx.x == 0 && threadIdx.x == 0) *zero = 0u;
   for (index_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const index_t j = order ? order[i] : i;
     out[i] = make_double4(a[j], b[j], c[j], d ? d[j] : 0.0);
@@ -43,11 +44,11 @@ void forget(lsmps_ctx* ctx, const double4* out) {
 }  // namespace
 
 void pack4(lsmps_ctx* ctx, const double* a, const double* b, const double* c, const double* d, size_t n,
-           double4* out, const index_t* order) {
+           double4* out, const index_t* order, unsigned* zero) {
   forget(ctx, out);
   if (n == 0) return;
   launch(ctx, pack4_kernel, dim3(stream_blocks(ctx, n)), dim3(256), 0, a, b, c, d, static_cast<index_t>(n), out,
-         order);
+         order, zero);
 }
 
 void pack4_label(lsmps_ctx* ctx, const double* a, const double* b, const double* c, const int32_t* label, size_t n,
@@ -70,9 +71,12 @@ void pack_wall_normals(lsmps_ctx* ctx, const lsmps_walls& w) {
   if (ctx->step_packs) ctx->packs_ready |= kWallNormals;
 }
 
-void pack_fluid_positions(lsmps_ctx* ctx, const lsmps_fluid& f, const index_t* order) {
-  if (ctx->step_packs && (ctx->packs_ready & kFluidPositions) && ctx->packs_fluid_order == order) return;
-  pack4(ctx, f.x, f.y, f.z, nullptr, f.count, ctx->pack_fluid[0], order);
+void pack_fluid_positions(lsmps_ctx* ctx, const lsmps_fluid& f, const index_t* order, unsigned* zero) {
+  if (ctx->step_packs && (ctx->packs_ready & kFluidPositions) && ctx->packs_fluid_order == order) {
+    if (zero) cudaMemsetAsync(zero, 0, sizeof(unsigned), ctx->stream);
+    return;
+  }
+  pack4(ctx, f.x, f.y, f.z, nullptr, f.count, ctx->pack_fluid[0], order, zero);
   if (ctx->step_packs) {
     ctx->packs_ready |= kFluidPositions;
     ctx->packs_fluid_order = order;
