@@ -228,10 +228,8 @@ __global__ void __launch_bounds__(kAdjThreads, 5) operators_forward_kernel(Opera
         r[7] -= coef;
       }
     }
-    if (ppe) {
-      a.columns[slot + 1 + o - nb] = j;
-      a.values[slot + 1 + o - nb] = coef;
-    }
+    if (a.columns) a.columns[slot + 1 + o - nb] = j;
+    if (ppe) a.values[slot + 1 + o - nb] = coef;
   }
   if (Walls) {
     const index_t we = a.wo[i + 1];
@@ -265,22 +263,25 @@ __global__ void __launch_bounds__(kAdjThreads, 5) operators_forward_kernel(Opera
   const double t = r[0];
   const double diag = __shfl_sync(0xffffffffu, t, 28);
   if ((lane & 3) != 0) return;
+  // (each output by its own pointer: any may be missing)
   if (base < 3) {
-    if (a.grad[0]) a.grad[base][i] = Walls && splash_row(a.label, i) ? 0.0 : t * a.inv_re;
+    double* grad = base == 0 ? a.grad[0] : base == 1 ? a.grad[1] : a.grad[2];
+    if (grad) grad[i] = Walls && splash_row(a.label, i) ? 0.0 : t * a.inv_re;
   } else if (base < (Walls ? 6 : 4)) {
-    double* lap = Walls ? a.lap_u[base - 3] : a.lap_f;
+    double* lap = !Walls ? a.lap_f : base == 3 ? a.lap_u[0] : base == 4 ? a.lap_u[1] : a.lap_u[2];
     if (lap) lap[i] = 2.0 * t * a.inv_re * a.inv_re;
   } else if (base == 6) {
     const double div = dir ? 0.0 : t * a.inv_re;
     if (dir) wall_rhs = 0.0;
     if (a.div) a.div[i] = div;
     if (Walls && a.wall_rhs) a.wall_rhs[i] = wall_rhs;
-    if (a.rhs && (Walls || ppe)) a.rhs[i] = dir ? 0.0 : div * a.inv_dt - wall_rhs;
-    if (!ppe) return;
-    a.row_offsets[i] = slot;
-    if (i + 1 == a.n) a.row_offsets[a.n] = a.n + ne;
-    a.columns[slot] = i;
-    a.values[slot] = dir ? 1.0 : diag;
+    if (a.rhs) a.rhs[i] = dir ? 0.0 : div * a.inv_dt - wall_rhs;
+    if (a.row_offsets) {
+      a.row_offsets[i] = slot;
+      if (i + 1 == a.n) a.row_offsets[a.n] = a.n + ne;
+    }
+    if (a.columns) a.columns[slot] = i;
+    if (ppe) a.values[slot] = dir ? 1.0 : diag;
   }
 }
 
