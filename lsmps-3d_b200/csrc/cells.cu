@@ -6,14 +6,15 @@
 //
 // A counting sort, both sets in the same launches: every particle takes a
 // number in its cell (in no particular order), the cells' counts are scanned
-// into ranges, the particles are put there by number, and each cell's few
-// particles are then ordered by index.  No block waits on another.  The
-// radix-sort kernels at the end of the kernels' list are those of the
-// allocation-free entry point (cells_noalloc.cu).
+// into ranges, the particles are put there by number, and each cell's
+// particles are then ordered by index.  No block waits on another.  A set with
+// many particles a cell is sorted by a stable radix sort instead, whose kernels
+// the allocation-free entry point (cells_noalloc.cu) uses too.
 #include <climits>
 #include <cmath>
 
 #include "cells.cuh"
+#include "packed.cuh"
 #include "scan.cuh"
 
 namespace lsmps {
@@ -238,66 +239,117 @@ __global__ void __launch_bounds__(kCellThreads) cell_place_kernel(CellArgs a) {
   }
 }
 
-// A cell of more particles than this is ordered by a walk over the whole set
-// instead of by comparing its particles with one another.
-constexpr index_t kManyInCell = 1024;
+// A cell of more particles than this and than a 32nd of its set (so at most 32 of
+// them) is ordered by a walk over the set's keys, the places of the others by
+// comparison.  Comparing takes 14 ns a particle of the cell, for the chain of one
+// thread's loads (more once the threads fill the GPU), and the walk 0.6 ns a particle
+// of the set: a cell of 9,000 among 20,000 costs 127 us compared and 10 walked; among
+// 2,000,000, 106 us compared and 1,100 walked; of 100,000 there, 2,400 and 1,100.
+constexpr index_t kComparedCell = 1024;
+constexpr int kOrderThreads = 256;
+constexpr int kOrderWarps = kOrderThreads / kWarp;
 
-// Orders the particles of cell c of set s by index (one warp), writes its
-// stretch of the sorted list and, where asked for, the sorted positions.
-__device__ __forceinline__ void order_cell(const CellArgs& a, const CellSet& set, index_t first, index_t n, index_t c,
-                                           index_t b, index_t e) {
-  const int lane = threadIdx.x & (kWarp - 1);
-  const index_t* __restrict__ placed = a.placed + first;
-  const auto put = [&](index_t at, index_t i) {
-    set.sorted[at] = i;
-    set.ids[at] = c;
-    if (set.pos) set.pos[at] = make_double4(set.x[i], set.y[i], set.z[i], 0.0);
-  };
-  const index_t many = e - b;
-  if (many <= kWarp) {
-    const index_t v = lane < many ? placed[b + lane] : INT_MAX;
-    index_t rank = 0;
-    for (index_t k = 0; k < many; ++k) rank += __shfl_sync(0xffffffffu, v, k) < v ? 1 : 0;
-    if (lane < many) put(b + rank, v);
-  } else if (many <= kManyInCell) {
-    for (index_t k = b + lane; k < e; k += kWarp) {
-      const index_t v = placed[k];
-      index_t rank = 0;
-      for (index_t q = b; q < e; ++q) rank += placed[q] < v ? 1 : 0;
-      put(b + rank, v);
-    }
-  } else {
-    index_t at = b;
-    for (index_t k = 0; k < n; k += kWarp) {
-      const bool mine = k + lane < n && a.key[first + k + lane] == c;
-      const unsigned in = __ballot_sync(0xffffffffu, mine);
-      if (mine) put(at + __popc(in & ((1u << lane) - 1u)), k + lane);
-      at += __popc(in);
-    }
-  }
+// The cell's list entry `at` is particle i; its position where asked for.
+__device__ __forceinline__ void put_in_cell(const CellSet& set, index_t c, index_t at, index_t i) {
+  set.sorted[at] = i;
+  set.ids[at] = c;
+  if (set.pos) set.pos[at] = make_double4(set.x[i], set.y[i], set.z[i], 0.0);
 }
 
-// Each warp orders the non-empty ones of `span` (1 .. 32) consecutive cells.
-__global__ void __launch_bounds__(kCellThreads) cell_order_kernel(CellArgs a, int span) {
+// One block finds cell c's particles among the keys first .. last - 1 of its set, in
+// index order: each warp counts those of its stretch, then lists them.
+__device__ __forceinline__ void order_by_walk(const CellSet& set, const index_t* __restrict__ key, index_t first,
+                                              index_t last, index_t c) {
+  __shared__ index_t s_found[kOrderWarps];
+  constexpr int kLoads = 4;  // of four keys, in flight per lane
+  constexpr int kRound = kLoads * 4 * kWarp;
+  const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
+  const unsigned below = (1u << lane) - 1u;
+  const long long start = first & ~3;
+  const long long share = (last - start + kRound * kOrderWarps - 1) / (kRound * kOrderWarps) * kRound;  // of a warp
+  const long long k0 = start + warp * share, k1 = min(static_cast<long long>(last), k0 + share);
+  // visit(index of the lane's four keys, which of them are the cell's)
+  const auto walk = [&](auto visit) {
+    for (long long k = k0 + 4 * lane; k - 4 * lane < k1; k += kRound) {
+      int4 v[kLoads];
+#pragma unroll
+      for (int u = 0; u < kLoads; ++u) {
+        const long long at = k + u * 4 * kWarp;
+        v[u] = at < k1 ? *reinterpret_cast<const int4*>(key + at) : make_int4(-1, -1, -1, -1);
+      }
+#pragma unroll
+      for (int u = 0; u < kLoads; ++u) {
+        const long long at = k + u * 4 * kWarp;
+        const auto mine = [&](int w, int x) { return x == c && at + w >= first && at + w < k1; };
+        const bool in[4] = {mine(0, v[u].x), mine(1, v[u].y), mine(2, v[u].z), mine(3, v[u].w)};
+        visit(at, in);
+      }
+    }
+  };
+  index_t found = 0;
+  walk([&](long long, const bool(&in)[4]) { found += in[0] + in[1] + in[2] + in[3]; });
+  found = __reduce_add_sync(0xffffffffu, found);
+  if (lane == 0) s_found[warp] = found;
+  __syncthreads();
+  index_t at = set.begin[c];
+  for (int w = 0; w < warp; ++w) at += s_found[w];
+  walk([&](long long k, const bool(&in)[4]) {
+    index_t before = 0, many = 0;  // of the lanes below, of the warp
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const unsigned all = __ballot_sync(0xffffffffu, in[w]);
+      before += __popc(all & below);
+      many += __popc(all);
+    }
+#pragma unroll
+    for (int w = 0; w < 4; ++w)
+      if (in[w]) put_in_cell(set, c, at + before++, static_cast<index_t>(k + w - first));
+    at += many;
+  });
+}
+
+// Orders each cell's particles by index: a thread takes one of the unordered list's
+// places, finds how many of its cell come before its particle and writes the
+// particle to its own place of the sorted list.  The comparisons of a warp are with
+// one or two cells' particles, four a load, and those of a crowded cell are spread
+// over as many threads as it has particles.  Bound by latency.  A list of 2,000,000
+// particles, 27 a cell: 91 us in all (93 with one warp per cell, which took 15,100
+// with 1,025 of them in one cell; 91 here); 300,000: 34 (34; 2,340; 41).
+__global__ void __launch_bounds__(kOrderThreads) cell_order_kernel(const __grid_constant__ CellArgs a) {
   wait_for_previous();
-  const int lane = threadIdx.x & (kWarp - 1);
-  const long long cells = static_cast<long long>(a.sets) * a.ncell;
-  const long long warps = static_cast<long long>(gridDim.x) * (kCellThreads / kWarp);
-  for (long long g = static_cast<long long>(blockIdx.x) * (kCellThreads / kWarp) + threadIdx.x / kWarp;
-       g * span < cells; g += warps) {
-    const long long c = g * span + lane;
-    const bool mine = lane < span && c < cells;
-    const int s = c >= a.ncell ? 1 : 0;
-    const index_t at = static_cast<index_t>(c - (s ? a.ncell : 0));
-    const index_t b = mine ? a.set[s].begin[at] : -1, e = mine ? a.set[s].end[at] : -1;
-    for (unsigned rem = __ballot_sync(0xffffffffu, b >= 0); rem; rem &= rem - 1) {
-      const int k = __ffs(rem) - 1;
-      const int sk = __shfl_sync(0xffffffffu, s, k);
-      const index_t ck = __shfl_sync(0xffffffffu, at, k), bk = __shfl_sync(0xffffffffu, b, k),
-                    ek = __shfl_sync(0xffffffffu, e, k);
-      order_cell(a, a.set[sk], sk ? a.first1 : 0, sk ? a.total - a.first1 : a.first1, ck, bk, ek);
+  __shared__ index_t s_huge;
+  __shared__ int s_set;
+  const long long place = static_cast<long long>(blockIdx.x) * kOrderThreads + threadIdx.x;
+  const index_t p = static_cast<index_t>(place);
+  bool huge = false;
+  if (place < a.total) {
+    const int s = p >= a.first1 ? 1 : 0;
+    const CellSet& set = a.set[s];
+    const index_t first = s ? a.first1 : 0;
+    const index_t i = a.placed[p], c = a.key[first + i];
+    const index_t b = set.begin[c], e = set.end[c];
+    const index_t many = s ? a.total - a.first1 : a.first1;
+    if (e - b > max(kComparedCell, many / 32)) {
+      huge = p == first + b;  // (one such place in a block's stretch, at most)
+      if (huge) {
+        s_huge = c;
+        s_set = s;
+      }
+    } else {
+      index_t at = b, q = first + b;
+      const index_t end = first + e;
+      for (; q < end && (q & 3) != 0; ++q) at += a.placed[q] < i ? 1 : 0;
+#pragma unroll 8
+      for (; q + 4 <= end; q += 4) {
+        const int4 v = *reinterpret_cast<const int4*>(a.placed + q);
+        at += (v.x < i) + (v.y < i) + (v.z < i) + (v.w < i);
+      }
+      for (; q < end; ++q) at += a.placed[q] < i ? 1 : 0;
+      put_in_cell(set, c, at, i);
     }
   }
+  if (__syncthreads_or(huge))
+    order_by_walk(a.set[s_set], a.key, s_set ? a.first1 : 0, s_set ? a.total : a.first1, s_huge);
 }
 
 }  // namespace
@@ -316,9 +368,17 @@ lsmps_status validate_grid(lsmps_ctx* ctx, const lsmps_grid& grid) {
   return LSMPS_OK;
 }
 
+// A set of more particles than this per cell on average is sorted by cell id
+// instead of counted, as the comparisons grow with the number per cell and the sort
+// does not: 2,000,000 particles 116 us counted at 128 a cell and 152 at 250, sorted
+// 104; 300,000: 38, 49 and 55 (and 84 counted at 585 a cell); 20,000: 24 at 160, 34
+// at 740, and 28.
+constexpr size_t kCrowdedMean = 128;
+
 size_t cell_list_scratch_bytes(size_t n, size_t ncell) {
-  // keys, numbers and placed particles; the cells' counts; their scan
-  return 3 * (n * sizeof(index_t) + 256) + ncell * sizeof(index_t) + scan_scratch_bytes(ncell) + 4096;
+  // keys, numbers and placed particles; the cells' counts; their scan (the sort of a
+  // crowded set takes less: keys and particles once more, its table of digits)
+  return 3 * (n * sizeof(index_t) + 256) + ncell * sizeof(index_t) + scan_scratch_bytes(ncell) + 8192;
 }
 
 lsmps_status check_cell_set(lsmps_ctx* ctx, const CellSet& set, size_t count, const lsmps_grid& grid,
@@ -336,19 +396,65 @@ lsmps_status check_cell_set(lsmps_ctx* ctx, const CellSet& set, size_t count, co
   return LSMPS_OK;
 }
 
+namespace {
+
+// The cell list of one set by a stable radix sort of (cell id, particle index),
+// whose time does not depend on how many particles a cell has.
+lsmps_status sort_cell_list(lsmps_ctx* ctx, Scratch& scratch, const CellSet& set, index_t n, const lsmps_grid& grid) {
+  const long long ncell = static_cast<long long>(grid.dims[0]) * grid.dims[1] * grid.dims[2];
+  const int passes = (key_bits(ncell) + kRadixBits - 1) / kRadixBits;
+  const int tiles = div_up(n, kSortTile);
+  index_t* other[2] = {scratch.take<index_t>(static_cast<size_t>(n) + 1), scratch.take<index_t>(static_cast<size_t>(n) + 1)};
+  index_t* hist = scratch.take<index_t>(static_cast<size_t>(tiles) * kRadixBins + 1);
+  if (!other[0] || !other[1] || !hist) return fail(ctx, LSMPS_CUDA_ERROR, "cell list scratch exhausted");
+  // back and forth so that the last pass ends in the caller's arrays
+  index_t* from[2] = {passes % 2 ? other[0] : set.ids, passes % 2 ? other[1] : set.sorted};
+  index_t* to[2] = {passes % 2 ? set.ids : other[0], passes % 2 ? set.sorted : other[1]};
+  const auto blocks = [&](long long work) {
+    return dim3(static_cast<int>(std::min<long long>(div_up(work, kCellThreads), ctx->sm_count * 8LL)));
+  };
+  launch(ctx, hash_kernel, blocks(std::max<long long>(n, ncell)), dim3(kCellThreads), 0, set.x, set.y, set.z, n, grid,
+         from[0], from[1], set.begin, set.end, static_cast<index_t>(ncell), ctx->d_status);
+  for (int p = 0; p < passes; ++p) {
+    launch(ctx, radix_hist_kernel, dim3(tiles), dim3(kSortThreads), 0, static_cast<const index_t*>(from[0]), n,
+           p * kRadixBits, hist, tiles);
+    if (const lsmps_status st =
+            exclusive_scan_i32(ctx, scratch, hist, hist, static_cast<size_t>(tiles) * kRadixBins, nullptr, nullptr))
+      return st;
+    launch(ctx, radix_scatter_kernel, dim3(tiles), dim3(kSortThreads), 0, static_cast<const index_t*>(from[0]),
+           static_cast<const index_t*>(from[1]), to[0], to[1], n, p * kRadixBits, static_cast<const index_t*>(hist), tiles);
+    std::swap(from[0], to[0]);
+    std::swap(from[1], to[1]);
+  }
+  launch(ctx, ranges_kernel, blocks(n), dim3(kCellThreads), 0, static_cast<const index_t*>(set.ids), n, set.begin, set.end);
+  if (set.pos) pack4(ctx, set.x, set.y, set.z, nullptr, static_cast<size_t>(n), set.pos, set.sorted);
+  return check_launch(ctx, "cell list");
+}
+
+}  // namespace
+
 lsmps_status build_cell_lists_impl(lsmps_ctx* ctx, Scratch& scratch, CellSet* sets, const size_t* counts,
                                    const lsmps_cells* const* cells, int many, const lsmps_grid& grid,
                                    const BoxGrid* boxes) {
   lsmps_status st = validate_grid(ctx, grid);
   for (int s = 0; s < many && !st; ++s) st = check_cell_set(ctx, sets[s], counts[s], grid, *cells[s]);
   if (st) return st;
+  for (int s = 0; s < many; ++s) {
+    sets[s].ids = cells[s]->cell_ids;
+    sets[s].sorted = cells[s]->sorted_indices;
+    sets[s].begin = cells[s]->cell_begin;
+    sets[s].end = cells[s]->cell_end;
+  }
+  const size_t ncell = cells[0]->cell_count;
+  const auto coarse = [&](int s) { return !boxes && counts[s] > kCrowdedMean * ncell; };
   // both sets' particles in one index range: one after the other where that
   // would pass 32 bits
-  if (many == 2 && counts[0] + counts[1] > static_cast<size_t>(INT_MAX)) {
+  if (many == 2 && (counts[0] + counts[1] > static_cast<size_t>(INT_MAX) || coarse(0) || coarse(1))) {
     for (int s = 0; s < 2 && !st; ++s)
       st = build_cell_lists_impl(ctx, scratch, sets + s, counts + s, cells + s, 1, grid, boxes);
     return st;
   }
+  if (coarse(0)) return sort_cell_list(ctx, scratch, sets[0], static_cast<index_t>(counts[0]), grid);
   CellArgs a{};
   a.sets = many;
   a.grid = grid;
@@ -360,10 +466,6 @@ lsmps_status build_cell_lists_impl(lsmps_ctx* ctx, Scratch& scratch, CellSet* se
   a.status = ctx->d_status;
   for (int s = 0; s < many; ++s) {
     a.set[s] = sets[s];
-    a.set[s].ids = cells[s]->cell_ids;
-    a.set[s].sorted = cells[s]->sorted_indices;
-    a.set[s].begin = cells[s]->cell_begin;
-    a.set[s].end = cells[s]->cell_end;
   }
   const size_t m = static_cast<size_t>(many) * a.ncell;
   a.key = scratch.take<index_t>(static_cast<size_t>(a.total) + 1);
@@ -389,12 +491,7 @@ lsmps_status build_cell_lists_impl(lsmps_ctx* ctx, Scratch& scratch, CellSet* se
   }
   if (a.total == 0) return check_launch(ctx, "cell lists");
   launch(ctx, cell_place_kernel, dim3(blocks), dim3(kCellThreads), 0, a);
-  // cells per warp: few enough to give every SM 32 warps, up to 32
-  const long long span = std::min<long long>(
-      32, std::max<long long>(1, static_cast<long long>(m) / (ctx->sm_count * 32LL)));
-  const int order_blocks = static_cast<int>(std::min<long long>(
-      div_up(div_up(static_cast<long long>(m), static_cast<int>(span)), kCellThreads / kWarp), ctx->sm_count * 32LL));
-  launch(ctx, cell_order_kernel, dim3(order_blocks), dim3(kCellThreads), 0, a, static_cast<int>(span));
+  launch(ctx, cell_order_kernel, dim3(div_up(static_cast<long long>(a.total), kOrderThreads)), dim3(kOrderThreads), 0, a);
   return check_launch(ctx, "cell lists");
 }
 

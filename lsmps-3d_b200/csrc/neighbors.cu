@@ -628,7 +628,7 @@ lsmps_status build_tables(lsmps_ctx* ctx, Scratch& scratch, const CsrTables& tab
 }  // namespace
 
 size_t neighbor_scratch_bytes(size_t n_fluid, size_t n_wall, size_t ncell) {
-  return cell_list_scratch_bytes(n_fluid + n_wall, 2 * ncell) + cell_list_scratch_bytes(0, ncell) +
+  return cell_list_scratch_bytes(n_fluid, ncell) + cell_list_scratch_bytes(n_wall, ncell) + scan_scratch_bytes(ncell) +
          2 * scan_scratch_bytes(n_fluid + 1) + 2 * n_fluid * kMaskWords * sizeof(unsigned) +
          (n_fluid + n_wall) * sizeof(double4) + 8192;
 }
