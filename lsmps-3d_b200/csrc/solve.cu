@@ -19,8 +19,10 @@
 // Each kernel's last block to finish adds the blocks' partial sums in a fixed
 // order, and that of the third extends the Hessenberg matrix by its column and
 // rotates it, so a solve is bitwise reproducible, nothing waits for the host
-// within a restart cycle, and a cycle that has converged lets its remaining
-// launches return at once.
+// within a restart cycle, and what is queued of a cycle that has converged returns
+// at once.  How far a cycle is the device writes to host memory, so that the host
+// queues nothing for a system that starts converged and, where a step is long,
+// little that would not be wanted.
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
@@ -38,6 +40,15 @@ constexpr int kMaxRestart = 64;
 // Rows up to which a product and its dot products are one kernel (measured at
 // product_dots_kernel).
 constexpr index_t kFusedRows = 100000;
+
+// A progress past every step's: nothing more of this cycle is wanted.
+constexpr int kStopped = 1 << 30;
+// Where the first projection is a kernel of its own (above kFusedRows), a step is
+// queued once the last but one has finished: one that converges in its first step
+// takes 255 us at 500,000 rows, and 500 with up to twenty steps queued that then
+// return at once (31,250 blocks each in the product).  Below, the write to host
+// memory would cost a step 0.8 of its 16 us (8,000 rows) and the launches cost less.
+constexpr int kAhead = 1;
 
 // The solve's scalars, in device memory.
 struct SolveState {
@@ -60,14 +71,15 @@ struct SolveArgs {
   const index_t* ci;
   const double* va;
   const double* dinv;        // Jacobi: 1 / a_ii, or NULL
-  double* V;                 // [restart + 1][ldv]
+  double* V;                 // [restart][ldv]
   size_t ldv;
   double* w[2];  // the vector to be normalised next, and its product
   double* x;
   const double* b;
   double* partial;  // [kMaxRestart + 1][gridDim.x]
   SolveState* st;
-  volatile int* stopped;  // host memory: set with st->stop
+  volatile int* progress;  // host memory: 1 + the cycle's finished steps (counted with `follow`), kStopped with st->stop
+  int follow;
   int restart;
   int max_iters;
   double tolerance;
@@ -187,6 +199,7 @@ __global__ void __launch_bounds__(kSolveThreads) residual_kernel(SolveArgs a, in
   st->g[0] = beta;
   st->converged = beta <= st->target ? 1 : 0;
   st->stop = st->converged || st->iters >= a.max_iters;
+  if (report) *a.progress = st->stop ? kStopped : 1;
 }
 
 // Step j: v_j = scale w[j & 1] into the basis, w[(j + 1) & 1] = A v_j.
@@ -368,10 +381,9 @@ __global__ void __launch_bounds__(kSolveThreads) extend_kernel(SolveArgs a, int 
     st->iters += 1;
     // hnext == 0: the Krylov space is invariant (the correction solves the
     // system on it); the cycle stops there.
-    if (fabs(s * g) <= st->target || hnext == 0.0 || st->iters >= a.max_iters) {
-      st->stop = 1;
-      *a.stopped = 1;
-    }
+    const bool stop = fabs(s * g) <= st->target || hnext == 0.0 || st->iters >= a.max_iters;
+    if (stop) st->stop = 1;
+    if (stop || a.follow) *a.progress = stop ? kStopped : j + 2;
   }
   __syncthreads();
   for (int k = threadIdx.x; k <= j; k += kSolveThreads) st->H[static_cast<size_t>(j) * (kMaxRestart + 1) + k] = col[k];
@@ -535,18 +547,19 @@ lsmps_status solve_ppe_impl(lsmps_ctx* ctx, const lsmps_csr_matrix& A, const dou
   a.st = scratch.take<SolveState>(1);
   if (!a.V || !a.w[0] || !a.w[1] || !dinv || !a.partial || !a.st)
     return fail(ctx, LSMPS_CUDA_ERROR, "scratch exhausted");
-  // pinned: the state's leading scalars read back after a cycle, and the flag
-  // that the device sets when a cycle stops early
+  // pinned: the state's leading scalars read back after a cycle, and how far the
+  // cycle is
   struct Pinned {
     SolveState state;
-    volatile int stopped;
+    volatile int progress;
   };
   static thread_local Pinned* pinned = nullptr;
   if (!pinned && cudaMallocHost(&pinned, sizeof(Pinned)) != cudaSuccess) {
     pinned = nullptr;
     return fail(ctx, LSMPS_CUDA_ERROR, "pinned allocation failed");
   }
-  a.stopped = &pinned->stopped;
+  a.progress = &pinned->progress;
+  a.follow = g.fused ? 0 : 1;
   a.x = x;
   a.b = b;
   a.restart = m;
@@ -558,22 +571,30 @@ lsmps_status solve_ppe_impl(lsmps_ctx* ctx, const lsmps_csr_matrix& A, const dou
     a.dinv = dinv;
   }
   cudaMemsetAsync(&a.st->tickets, 0, sizeof(unsigned), ctx->stream);
-  launch_residual(ctx, a, !opt.use_initial_guess, true, g);
   const SolveState& st = pinned->state;
+  pinned->progress = 0;
+  launch_residual(ctx, a, !opt.use_initial_guess, true, g);
   const auto read = [&]() {
     return cudaMemcpyAsync(&pinned->state, a.st, offsetof(SolveState, tickets), cudaMemcpyDeviceToHost, ctx->stream) ==
                cudaSuccess &&
            cudaStreamSynchronize(ctx->stream) == cudaSuccess;
   };
-  // The first cycle is queued without waiting for the first residual: a system
-  // that starts converged lets its launches return at once.
-  for (;;) {
-    pinned->stopped = 0;
-    for (int j = 0; j < m && !pinned->stopped; ++j) launch_step(ctx, a, j, g);
-    launch(ctx, correct_kernel, dim3(g.stream), dim3(kSolveThreads), 0, a);
-    launch_residual(ctx, a, false, false, g);
+  // Waits until the cycle has come to `reached`, or until nothing is queued.
+  const auto wait = [&](int reached) {
+    for (unsigned spins = 1; pinned->progress < reached; ++spins)
+      if (spins % 4096 == 0 && cudaStreamQuery(ctx->stream) != cudaErrorNotReady) break;
+    return pinned->progress != kStopped;
+  };
+  for (bool first = true;; first = false) {
+    int j = 0;
+    for (; j < m && wait(j > 0 && a.follow ? j + 1 - kAhead : 1); ++j) launch_step(ctx, a, j, g);
+    if (j > 0) launch(ctx, correct_kernel, dim3(g.stream), dim3(kSolveThreads), 0, a);
+    // (without a step the residual stands, but one of x = 0 has not met A yet,
+    // whose NaN would show there)
+    if (j > 0 || (first && !opt.use_initial_guess)) launch_residual(ctx, a, false, false, g);
     if (!read()) return check_launch(ctx, "PPE solve");
     if (st.converged || st.iters >= opt.max_iters) break;
+    pinned->progress = 1;
   }
   if (opt.clamp_negative) launch(ctx, clamp_kernel, dim3(div_up(n, kSolveThreads)), dim3(kSolveThreads), 0, n, x);
   if (report) *report = lsmps_solver_report{st.iters, st.converged ? 1 : 0, st.beta0, st.beta};
