@@ -588,17 +588,69 @@ __global__ void __launch_bounds__(kAdjThreads, 4) operators_backward_kernel(cons
   }
 }
 
+// Entries ranked at a time in the last pass of the deterministic backward.
+constexpr int kRankWindow = 128, kRankPer = kRankWindow / kWarp;
+
+// The entry id of record e, and the place of the e-th in order where a row has more
+// than kRankWindow records: the halves of a record's last double.
+__device__ __forceinline__ int* record_half(double4* rec, int e, int upper) {
+  return reinterpret_cast<int*>(rec + 2 * static_cast<size_t>(e) + 1) + 6 + upper;
+}
+
+// rank[k] += how many of ids[0 .. many - 1] come before mine[k] (past the end:
+// INT32_MAX, before none).
+__device__ __forceinline__ void add_ranks(const int* ids, int many, const int (&mine)[kRankPer], int (&rank)[kRankPer]) {
+  for (int c = 0; c < many; c += 4) {
+    const int4 v = *reinterpret_cast<const int4*>(ids + c);
+#pragma unroll
+    for (int k = 0; k < kRankPer; ++k)
+      rank[k] += (v.x < mine[k]) + (v.y < mine[k]) + (v.z < mine[k]) + (v.w < mine[k]);
+  }
+}
+
+// The order of more than kRankWindow records, into their upper halves.
+__device__ __noinline__ void order_long_row(double4* rec, int count, int* ids) {
+  const int lane = threadIdx.x & (kWarp - 1);
+  for (int e0 = 0; e0 < count; e0 += kRankWindow) {
+    int mine[kRankPer], rank[kRankPer];
+#pragma unroll
+    for (int k = 0; k < kRankPer; ++k) {
+      const int e = e0 + k * kWarp + lane;
+      mine[k] = e < count ? *record_half(rec, e, 0) : INT32_MAX;
+      rank[k] = 0;
+    }
+    for (int c0 = 0; c0 < count; c0 += kRankWindow) {
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < kRankPer; ++k) {
+        const int c = c0 + k * kWarp + lane;
+        ids[k * kWarp + lane] = c < count ? *record_half(rec, c, 0) : INT32_MAX;
+      }
+      __syncwarp();
+      add_ranks(ids, min(kRankWindow, count - c0), mine, rank);
+    }
+#pragma unroll
+    for (int k = 0; k < kRankPer; ++k) {
+      const int e = e0 + k * kWarp + lane;
+      if (e < count) *record_half(rec, rank[k], 1) = e;
+    }
+  }
+  __syncwarp();
+}
+
 // Deterministic form, last pass: particle j adds its incoming entries' terms
 // in ascending entry order, whatever order their records arrived in (lane l
 // takes the l-th, the (l + 32)-th, ..., then a fixed tree), to its own row's.
-// One warp per particle; the arrival order is undone by ranking the entry ids,
-// up to 128 at a time.  A row of 108 costs the ranking about 900 warp
-// instructions, half of what the 64-byte records' own transfer takes.
+// One warp per particle; the arrival order is undone by ranking the entry ids.
+// A row of 108 costs the ranking about 900 warp instructions, half of what the
+// 64-byte records' own transfer takes; one of more than 128 is ranked 128 at a
+// time against 128.  The whole backward of 64,000 particles with rows of 281
+// entries 2.4 ms, of 956 10.4, of 4,000 with 3,999 10.1 (3.5, 42.7 and 260 with the
+// ranks found anew for every 128 in order).
 __global__ void __launch_bounds__(kAdjThreads) operators_collect_kernel(OperatorArgs a) {
   wait_for_previous();
-  constexpr int kWindow = 128, kPer = kWindow / kWarp;
-  __shared__ __align__(16) int s_id[kAdjWarps][kWindow];
-  __shared__ int s_at[kAdjWarps][kWindow];
+  __shared__ __align__(16) int s_id[kAdjWarps][kRankWindow];
+  __shared__ int s_at[kAdjWarps][kRankWindow];
   const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
   const index_t j = a.j0 + blockIdx.x * kAdjWarps + warp;
   if (j >= a.j1) return;  // the whole warp
@@ -607,54 +659,40 @@ __global__ void __launch_bounds__(kAdjThreads) operators_collect_kernel(Operator
   const double4* rec = a.records + 2 * first;
   int* ids = s_id[warp];
   int* at = s_at[warp];
+  const bool few = count <= kRankWindow;
+  if (few) {
+    int mine[kRankPer], rank[kRankPer];
+#pragma unroll
+    for (int k = 0; k < kRankPer; ++k) {
+      const int e = k * kWarp + lane;
+      mine[k] = e < count ? static_cast<int>(__double_as_longlong(rec[2 * static_cast<size_t>(e) + 1].w)) : INT32_MAX;
+      rank[k] = 0;
+      ids[e] = mine[k];
+    }
+    __syncwarp();
+    add_ranks(ids, count, mine, rank);
+#pragma unroll
+    for (int k = 0; k < kRankPer; ++k) {
+      const int e = k * kWarp + lane;
+      if (e < count) at[rank[k]] = e;
+    }
+    __syncwarp();
+  } else {
+    order_long_row(a.records + 2 * first, count, ids);
+  }
   double acc[7];
 #pragma unroll
   for (int c = 0; c < 7; ++c) acc[c] = 0.0;
-  for (int w0 = 0; w0 < count; w0 += kWindow) {  // records ranked w0 .. w0 + 127
-    for (int e0 = 0; e0 < count; e0 += kWindow) {
-      int mine[kPer], rank[kPer];
-#pragma unroll
-      for (int k = 0; k < kPer; ++k) {
-        const int e = e0 + k * kWarp + lane;
-        mine[k] = e < count ? static_cast<int>(__double_as_longlong(rec[2 * static_cast<size_t>(e) + 1].w)) : INT32_MAX;
-        rank[k] = 0;
-      }
-      for (int c0 = 0; c0 < count; c0 += kWindow) {
-        const int many = min(kWindow, count - c0);
-        __syncwarp();
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-          const int c = c0 + k * kWarp + lane;
-          ids[k * kWarp + lane] =
-              c0 == e0 ? mine[k]
-                       : c < count ? static_cast<int>(__double_as_longlong(rec[2 * static_cast<size_t>(c) + 1].w)) : INT32_MAX;
-        }
-        __syncwarp();
-        for (int c = 0; c < many; c += 4) {  // past the end: INT32_MAX, smaller than none
-          const int4 v = *reinterpret_cast<const int4*>(ids + c);
-#pragma unroll
-          for (int k = 0; k < kPer; ++k)
-            rank[k] += (v.x < mine[k]) + (v.y < mine[k]) + (v.z < mine[k]) + (v.w < mine[k]);
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < kPer; ++k) {
-        const int e = e0 + k * kWarp + lane;
-        if (e < count && rank[k] >= w0 && rank[k] < w0 + kWindow) at[rank[k] - w0] = e;
-      }
-    }
-    __syncwarp();
-    const int many = min(kWindow, count - w0);
-    for (int k = lane; k < many; k += kWarp) {
-      const double4 r0 = ld4(rec, 2 * at[k]), r1 = ld4(rec, 2 * at[k] + 1);
-      acc[0] += r0.x;
-      acc[1] += r0.y;
-      acc[2] += r0.z;
-      acc[3] += r0.w;
-      acc[4] += r1.x;
-      acc[5] += r1.y;
-      acc[6] += r1.z;
-    }
+  for (int k = lane; k < count; k += kWarp) {
+    const int e = few ? at[k] : __ldcg(record_half(a.records + 2 * first, k, 1));
+    const double4 r0 = ld4(rec, 2 * e), r1 = ld4(rec, 2 * e + 1);
+    acc[0] += r0.x;
+    acc[1] += r0.y;
+    acc[2] += r0.z;
+    acc[3] += r0.w;
+    acc[4] += r1.x;
+    acc[5] += r1.y;
+    acc[6] += r1.z;
   }
   int base = 0, left = 7;
   lane_totals<7, 16>(acc, base, left);
