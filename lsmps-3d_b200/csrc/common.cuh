@@ -290,12 +290,16 @@ struct lsmps_ctx {
   size_t pack_fluid_cap = 0;
   size_t pack_wall_cap = 0;
   // Moment stage: per fluid particle the 31 (Type-B: 35) FP64 fluid moment
-  // sums ([sum][n]) and, plain form, at moment_cap x 35 the wall terms of both
-  // boundaries ([31][n], then [45][n]), all by visiting position.
+  // sums ([sum][n]), by visiting position.
   double* moment_sums = nullptr;
-  int32_t* moment_walled = nullptr;   // plain form: visiting positions of the particles with walls
-  unsigned int* moment_walls = nullptr;  // ... and how many (cleared by each call's fluid pack)
   size_t moment_cap = 0;
+  // Plain form with walls: the wall terms of both boundaries ([31][n], then at
+  // moment_terms_cap x 31 [45][n]), the visiting positions of the particles with
+  // walls and how many (cleared by each call's fluid pack).
+  double* moment_terms = nullptr;
+  int32_t* moment_walled = nullptr;
+  unsigned int* moment_walls = nullptr;
+  size_t moment_terms_cap = 0;
   // Mixed form (LSMPS_PRECISION_MIXED): per fluid particle the compact FP32
   // operator rows of the velocity
   // and pressure inverses ([n][36]: Laplacian row, then rows 0, 1, 2), both
@@ -375,8 +379,10 @@ bool ensure_sorted_rows(lsmps_ctx* ctx, size_t entries, size_t nf);
 // Grow the mixed-form arrays to nf fluid particles (outside stream capture).
 bool ensure_mixed(lsmps_ctx* ctx, size_t nf);
 void free_mixed(lsmps_ctx* ctx);
-// Grow the moment stage's sums to nf fluid particles (outside stream capture).
+// Grow the moment stage's sums, and the plain form's wall terms, to nf fluid
+// particles (outside stream capture).
 bool ensure_moment_sums(lsmps_ctx* ctx, size_t nf);
+bool ensure_moment_terms(lsmps_ctx* ctx, size_t nf);
 void free_moment_sums(lsmps_ctx* ctx);
 // Grow / free the operator pair's scratch (adjoint.cu).
 bool ensure_adjoint(lsmps_ctx* ctx, size_t n);

@@ -68,30 +68,54 @@ bool ensure_mixed(lsmps_ctx* ctx, size_t nf) {
 
 void free_moment_sums(lsmps_ctx* ctx) {
   if (ctx->moment_sums) cudaFree(ctx->moment_sums);
+  if (ctx->moment_terms) cudaFree(ctx->moment_terms);
   ctx->moment_sums = nullptr;
+  ctx->moment_cap = 0;
+  ctx->moment_terms = nullptr;
   ctx->moment_walled = nullptr;
   ctx->moment_walls = nullptr;
-  ctx->moment_cap = 0;
+  ctx->moment_terms_cap = 0;
 }
 
-bool ensure_moment_sums(lsmps_ctx* ctx, size_t nf) {
-  if (nf <= ctx->moment_cap) return true;
+namespace {
+
+// *p, of `bytes` from now on (outside stream capture).
+bool renew(lsmps_ctx* ctx, double** p, size_t bytes) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   cudaStreamIsCapturing(ctx->stream, &cap);
   if (cap != cudaStreamCaptureStatusNone) return false;
   cudaStreamSynchronize(ctx->stream);
-  free_moment_sums(ctx);
-  // one allocation: the sums and both boundaries' wall terms, the list of
-  // particles with walls and its count
-  const size_t doubles = nf * (35 + 31 + 45);
-  if (cudaMalloc(&ctx->moment_sums, doubles * sizeof(double) + (nf + 1) * sizeof(int32_t)) != cudaSuccess) {
-    cudaGetLastError();
-    ctx->moment_sums = nullptr;
+  if (*p) cudaFree(*p);
+  *p = nullptr;
+  if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+  cudaGetLastError();
+  *p = nullptr;
+  return false;
+}
+
+}  // namespace
+
+bool ensure_moment_sums(lsmps_ctx* ctx, size_t nf) {
+  if (nf <= ctx->moment_cap) return true;
+  if (!renew(ctx, &ctx->moment_sums, nf * 35 * sizeof(double))) {
+    if (!ctx->moment_sums) ctx->moment_cap = 0;
     return false;
   }
-  ctx->moment_walls = reinterpret_cast<unsigned int*>(ctx->moment_sums + doubles);
-  ctx->moment_walled = reinterpret_cast<int32_t*>(ctx->moment_walls + 1);
   ctx->moment_cap = nf;
+  return true;
+}
+
+bool ensure_moment_terms(lsmps_ctx* ctx, size_t nf) {
+  if (nf <= ctx->moment_terms_cap) return true;
+  // both boundaries' wall terms, the count of particles with walls and their list
+  const size_t doubles = nf * (31 + 45);
+  if (!renew(ctx, &ctx->moment_terms, doubles * sizeof(double) + (nf + 1) * sizeof(int32_t))) {
+    if (!ctx->moment_terms) ctx->moment_terms_cap = 0;
+    return false;
+  }
+  ctx->moment_walls = reinterpret_cast<unsigned int*>(ctx->moment_terms + doubles);
+  ctx->moment_walled = reinterpret_cast<int32_t*>(ctx->moment_walls + 1);
+  ctx->moment_terms_cap = nf;
   return true;
 }
 
@@ -328,7 +352,8 @@ lsmps_status lsmps_ctx_reserve(lsmps_ctx* ctx, size_t fluid_capacity, size_t wal
   Scratch s(ctx);
   if (!s.reserve(need)) return fail(ctx, LSMPS_CUDA_ERROR, "scratch allocation failed");
   if (!ensure_packs(ctx, fluid_capacity, wall_capacity)) return fail(ctx, LSMPS_CUDA_ERROR, "pack allocation failed");
-  if (!ensure_moment_sums(ctx, fluid_capacity))
+  if (!ensure_moment_sums(ctx, fluid_capacity) ||
+      (ctx->precision == LSMPS_PRECISION_PLAIN && wall_capacity > 0 && !ensure_moment_terms(ctx, fluid_capacity)))
     return fail(ctx, LSMPS_CUDA_ERROR, "moment sums allocation failed");
   if (ctx->precision == LSMPS_PRECISION_MIXED && !ensure_mixed(ctx, fluid_capacity))
     return fail(ctx, LSMPS_CUDA_ERROR, "mixed-form allocation failed");

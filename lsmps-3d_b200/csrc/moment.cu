@@ -693,7 +693,7 @@ struct FinishArgs {
   const double* sums;
   const double* velocity;
   const double* pressure;
-  const index_t* wo;
+  const index_t* wo;  // NULL: no walls
   double lambda;
   KindOut k[3];
   DeviceStatus* status;
@@ -777,7 +777,7 @@ __global__ void __launch_bounds__(kFinishThreads, N == 9 ? 16 : 10) moment_finis
   if (t >= a.n) return;
   const index_t i = visit(a.order, t);
   const size_t n = static_cast<size_t>(a.n);
-  const bool walls = ko.boundary != 0 && a.wo[i] < a.wo[i + 1];
+  const bool walls = a.wo && ko.boundary != 0 && a.wo[i] < a.wo[i + 1];
   double m[N * (N + 1) / 2];
   if (N == 9 && walls && ko.boundary == 2) {
 #pragma unroll
@@ -1594,12 +1594,23 @@ lsmps_status prepare_moments_impl(lsmps_ctx* ctx, const lsmps_fluid& fluid, cons
                    mk.inversion_count};
   };
   if (!ensure_packs(ctx, fluid.count, walls.count)) return fail(ctx, LSMPS_CUDA_ERROR, "pack allocation failed");
-  if (!ensure_moment_sums(ctx, fluid.count)) return fail(ctx, LSMPS_CUDA_ERROR, "moment sums allocation failed");
+  const bool mixed = velocity_a >= 0 && pressure_a >= 0 && ctx->precision == LSMPS_PRECISION_MIXED;
+  // The plain kinds share one pass over the rows.
+  int many9 = 0, many10 = 0;
+  bool dirichlet = false, neumann_terms = false;
+  for (int k = 0; k < count; ++k) {
+    if (mixed && (k == velocity_a || k == pressure_a)) continue;
+    const int boundary = boundary_of(kinds[k].kind);
+    dirichlet |= boundary == 1;
+    neumann_terms |= boundary == 2;
+    ++(kinds[k].kind == LSMPS_MOMENT_PRESSURE_WALL_NEUMANN_B ? many10 : many9);
+  }
+  const bool with_walls = (dirichlet || neumann_terms) && walls.count > 0;
+  if (!ensure_moment_sums(ctx, fluid.count) || (with_walls && !ensure_moment_terms(ctx, fluid.count)))
+    return fail(ctx, LSMPS_CUDA_ERROR, "moment sums allocation failed");
   const index_t* srows = sorted_rows_of(ctx, fn, fluid.count);
   // (the list of particles with walls starts empty every time)
-  pack_fluid_positions(ctx, fluid, srows ? ctx->order : nullptr, ctx->moment_walls);
-  const bool fused = velocity_a >= 0 && pressure_a >= 0;
-  const bool mixed = fused && ctx->precision == LSMPS_PRECISION_MIXED;
+  pack_fluid_positions(ctx, fluid, srows ? ctx->order : nullptr, with_walls ? ctx->moment_walls : nullptr);
   if (mixed) {
     // Mixed form: FP32 assembly and factorisation with FP64 refinement; the
     // full inverse is written (FP64) for the caller's views.  (It packs the
@@ -1608,29 +1619,17 @@ lsmps_status prepare_moments_impl(lsmps_ctx* ctx, const lsmps_fluid& fluid, cons
         launch_mixed(ctx, n, fn, wn, p, out_of(kinds[velocity_a]), out_of(kinds[pressure_a]), true, walls);
     if (st) return st;
   }
-  // The other kinds share one pass over the rows.
+  if (many9 + many10 == 0) return check_launch(ctx, "moment matrices");
   FinishArgs a9{}, a10{};
-  int many9 = 0, many10 = 0;
-  bool dirichlet = false, neumann_terms = false;
   const auto finish = [&](FinishArgs& a, int& many, auto kernel, const char* name) {
     launch_named(ctx, name, kernel, dim3(div_up(n, kFinishThreads), many), dim3(kFinishThreads), 0, a);
     many = 0;
   };
-  for (int k = 0; k < count; ++k) {
-    if (mixed && (k == velocity_a || k == pressure_a)) continue;
-    const int boundary = boundary_of(kinds[k].kind);
-    dirichlet |= boundary == 1;
-    neumann_terms |= boundary == 2;
-    ++(kinds[k].kind == LSMPS_MOMENT_PRESSURE_WALL_NEUMANN_B ? many10 : many9);
-  }
-  if (many9 + many10 == 0) return check_launch(ctx, "moment matrices");
-  const size_t cap = ctx->moment_cap;
-  double* wall_velocity = ctx->moment_sums + cap * kMonomialsB;
-  double* wall_pressure = wall_velocity + cap * kMonomials;
+  double* wall_velocity = ctx->moment_terms;
+  double* wall_pressure = wall_velocity + ctx->moment_terms_cap * kMonomials;
   const index_t* fi = srows ? srows : fn.indices;
   const SumArgs sa{n, ctx->pack_fluid[0], fn.offsets, fi, 1.0 / p.support_radius, ctx->moment_sums, ctx->order,
                    srows ? 1 : 0};
-  const bool with_walls = (dirichlet || neumann_terms) && walls.count > 0;
   launch_plain_sums(ctx, sa, with_walls ? static_cast<const index_t*>(wn.offsets) : nullptr, many10 > 0);
   if (with_walls) {
     pack_wall_positions(ctx, walls);
@@ -1647,8 +1646,8 @@ lsmps_status prepare_moments_impl(lsmps_ctx* ctx, const lsmps_fluid& fluid, cons
       launch(ctx, wall_sums_kernel, dim3(std::min(groups, ctx->sm_count * 12), kinds_on), dim3(kWallThreads), 0, wa,
              dirichlet ? 0 : 1);
   }
-  a9 = FinishArgs{n, ctx->moment_sums, wall_velocity, wall_pressure, wn.offsets, p.lsmps_regularization,
-                  {},  ctx->d_status,     ctx->order};
+  a9 = FinishArgs{n, ctx->moment_sums, wall_velocity, wall_pressure, with_walls ? wn.offsets : nullptr,
+                  p.lsmps_regularization, {}, ctx->d_status, ctx->order};
   a10 = a9;
   many9 = many10 = 0;
   for (int k = 0; k < count; ++k) {
