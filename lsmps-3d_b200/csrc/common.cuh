@@ -300,6 +300,7 @@ struct lsmps_ctx {
   int32_t* moment_walled = nullptr;
   unsigned int* moment_walls = nullptr;
   size_t moment_terms_cap = 0;
+  double* retired[2] = {nullptr, nullptr};  // what the two replaced under capture
   // Mixed form (LSMPS_PRECISION_MIXED): per fluid particle the compact FP32
   // operator rows of the velocity
   // and pressure inverses ([n][36]: Laplacian row, then rows 0, 1, 2), both
@@ -380,7 +381,8 @@ bool ensure_sorted_rows(lsmps_ctx* ctx, size_t entries, size_t nf);
 bool ensure_mixed(lsmps_ctx* ctx, size_t nf);
 void free_mixed(lsmps_ctx* ctx);
 // Grow the moment stage's sums, and the plain form's wall terms, to nf fluid
-// particles (outside stream capture).
+// particles (under capture too: they are the only scratch that a call may find
+// missing whose packs another call has grown).
 bool ensure_moment_sums(lsmps_ctx* ctx, size_t nf);
 bool ensure_moment_terms(lsmps_ctx* ctx, size_t nf);
 void free_moment_sums(lsmps_ctx* ctx);

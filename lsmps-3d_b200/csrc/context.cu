@@ -75,29 +75,45 @@ void free_moment_sums(lsmps_ctx* ctx) {
   ctx->moment_walled = nullptr;
   ctx->moment_walls = nullptr;
   ctx->moment_terms_cap = 0;
+  for (double* p : ctx->retired)
+    if (p) cudaFree(p);
+  ctx->retired[0] = ctx->retired[1] = nullptr;
 }
 
 namespace {
 
-// *p, of `bytes` from now on (outside stream capture).
-bool renew(lsmps_ctx* ctx, double** p, size_t bytes) {
+// *p, of `bytes` from now on.  Under capture the one it replaces may be part of
+// what was captured before: it is kept (one of each kind; a second time refuses).
+bool renew(lsmps_ctx* ctx, double** p, size_t bytes, double** retired) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   cudaStreamIsCapturing(ctx->stream, &cap);
-  if (cap != cudaStreamCaptureStatusNone) return false;
-  cudaStreamSynchronize(ctx->stream);
-  if (*p) cudaFree(*p);
-  *p = nullptr;
-  if (cudaMalloc(p, bytes) == cudaSuccess) return true;
-  cudaGetLastError();
-  *p = nullptr;
-  return false;
+  const bool capturing = cap != cudaStreamCaptureStatusNone;
+  if (capturing && *p && *retired) return false;
+  if (!capturing) {
+    cudaStreamSynchronize(ctx->stream);
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+  }
+  // (an allocation is no part of the capture)
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  double* fresh = nullptr;
+  const bool ok = cudaMalloc(&fresh, bytes) == cudaSuccess;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (!ok) {
+    cudaGetLastError();
+    return false;
+  }
+  if (*p) *retired = *p;
+  *p = fresh;
+  return true;
 }
 
 }  // namespace
 
 bool ensure_moment_sums(lsmps_ctx* ctx, size_t nf) {
   if (nf <= ctx->moment_cap) return true;
-  if (!renew(ctx, &ctx->moment_sums, nf * 35 * sizeof(double))) {
+  if (!renew(ctx, &ctx->moment_sums, nf * 35 * sizeof(double), &ctx->retired[0])) {
     if (!ctx->moment_sums) ctx->moment_cap = 0;
     return false;
   }
@@ -109,7 +125,7 @@ bool ensure_moment_terms(lsmps_ctx* ctx, size_t nf) {
   if (nf <= ctx->moment_terms_cap) return true;
   // both boundaries' wall terms, the count of particles with walls and their list
   const size_t doubles = nf * (31 + 45);
-  if (!renew(ctx, &ctx->moment_terms, doubles * sizeof(double) + (nf + 1) * sizeof(int32_t))) {
+  if (!renew(ctx, &ctx->moment_terms, doubles * sizeof(double) + (nf + 1) * sizeof(int32_t), &ctx->retired[1])) {
     if (!ctx->moment_terms) ctx->moment_terms_cap = 0;
     return false;
   }
