@@ -795,9 +795,11 @@ lsmps_status lsmps_step_operators_backward(lsmps_ctx* ctx, const lsmps_fluid* fl
  * 0 (default): deterministic -- each row's entries are evaluated once, the
  * neighbours' shares kept as records that every particle adds in a fixed order
  * (ascending entries); repeated calls give the same bits.  Costs 64 bytes of
- * scratch per entry, at most 16 GB: a larger table is done in passes.  1: each
- * row scatters its terms into its neighbours with FP64 atomics (no records;
- * the sums' order, and so the last bits, may vary between calls). */
+ * scratch per entry, 16 GiB at most (a larger table, or one whose records cannot
+ * be allocated, is done in passes), and 72 per particle; the context keeps it,
+ * as all its scratch, with up to 256 MiB to grow.  1: each row scatters its
+ * terms into its neighbours with FP64 atomics (no records; the sums' order, and
+ * so the last bits, may vary between calls). */
 lsmps_status lsmps_ctx_set_adjoint_atomic(lsmps_ctx* ctx, int on);
 
 #ifdef __cplusplus

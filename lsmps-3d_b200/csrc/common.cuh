@@ -351,6 +351,10 @@ struct lsmps_ctx {
 
 namespace lsmps {
 
+// Most bytes that the scratch takes beyond what a call asks for (a quarter of it, so
+// that slowly growing sets do not allocate in every call).
+constexpr size_t kScratchGrowth = size_t(256) << 20;
+
 // Bump allocator over the context's scratch; reset at the start of each API
 // call.  Grows (outside stream capture) when a call needs more.
 class Scratch {

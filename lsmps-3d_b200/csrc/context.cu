@@ -17,13 +17,16 @@ bool Scratch::reserve(size_t bytes) {
     ctx_->scratch = nullptr;
     ctx_->scratch_bytes = 0;
   }
-  const size_t grown = bytes + bytes / 4;
-  if (cudaMalloc(&ctx_->scratch, grown) != cudaSuccess) {
+  // room to grow, where there is any
+  for (const size_t more : {bytes / 4 < kScratchGrowth ? bytes / 4 : kScratchGrowth, size_t(0)}) {
+    if (cudaMalloc(&ctx_->scratch, bytes + more) == cudaSuccess) {
+      ctx_->scratch_bytes = bytes + more;
+      return true;
+    }
     cudaGetLastError();
-    return false;
+    ctx_->scratch = nullptr;
   }
-  ctx_->scratch_bytes = grown;
-  return true;
+  return false;
 }
 
 void free_mixed(lsmps_ctx* ctx) {
