@@ -331,6 +331,9 @@ struct lsmps_ctx {
   // Backward form: false = transpose + gather (deterministic, the default),
   // true = scatter with FP64 atomics (lsmps_ctx_set_adjoint_atomic).
   bool adjoint_atomic = false;
+  // The deterministic backward's records: the most that could be allocated when
+  // memory was short, or 0.
+  size_t record_limit = 0;
   // Merged batch (batch.cu): the boxes' grid table in device memory while
   // this context steps a merged particle set, else NULL.
   const lsmps::BoxGrid* boxes = nullptr;

@@ -15,6 +15,7 @@
 // memory, and in the backward the row is walked a second time for the entries'
 // own terms.
 #include <algorithm>
+#include <new>
 #include <vector>
 
 #include "adjoint.cuh"
@@ -769,11 +770,22 @@ lsmps_status operators_backward(lsmps_ctx* ctx, const lsmps_csr& fn, OperatorArg
   const size_t entry = 2 * sizeof(double4);
   const size_t fixed = 2 * (n + 1) * sizeof(index_t) + 8 * n * sizeof(double) + scan_scratch_bytes(n) + 4096;
   size_t most = std::min(kRecordBytes, static_cast<size_t>(total) * entry);
+  if (ctx->record_limit && most > ctx->record_limit) {
+    // memory was short before: no more is tried for (which would give up the scratch
+    // at hand) until there is that much
+    size_t room = 0, all = 0;
+    if (cudaMemGetInfo(&room, &all) == cudaSuccess && room + ctx->scratch_bytes >= fixed + most + kScratchGrowth)
+      ctx->record_limit = 0;
+    else
+      most = ctx->record_limit;
+  }
+  const size_t wanted = most;
   Scratch scratch(ctx);
   while (!scratch.reserve(fixed + most)) {  // less room: more passes
     most /= 2;
     if (most < (size_t(1) << 20)) return fail(ctx, LSMPS_CUDA_ERROR, "operator scratch allocation failed");
   }
+  if (most < wanted) ctx->record_limit = most;
   index_t* begin = scratch.take<index_t>(n + 1);
   a.begin = begin;
   a.next = scratch.take<index_t>(n + 1);
@@ -790,7 +802,11 @@ lsmps_status operators_backward(lsmps_ctx* ctx, const lsmps_csr& fn, OperatorArg
   if (!a.records) return fail(ctx, LSMPS_CUDA_ERROR, "operator scratch exhausted");
   std::vector<index_t> first;
   if (most < static_cast<size_t>(total) * entry) {
-    first.resize(n + 1);
+    try {
+      first.resize(n + 1);
+    } catch (const std::bad_alloc&) {
+      return fail(ctx, LSMPS_CUDA_ERROR, "operator scratch allocation failed");
+    }
     if (cudaMemcpyAsync(first.data(), begin, (n + 1) * sizeof(index_t), cudaMemcpyDeviceToHost, ctx->stream) !=
             cudaSuccess ||
         cudaStreamSynchronize(ctx->stream) != cudaSuccess)
