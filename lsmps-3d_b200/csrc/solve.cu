@@ -13,12 +13,12 @@
 // Algorithm: GMRES(m) of Saad and Schultz (1986) with right preconditioning
 // (none, or Jacobi: M = diag(A)).  Arnoldi uses classical Gram-Schmidt with
 // one re-orthogonalisation (CGS2), so every projection is a batch of
-// independent dot products.  An Arnoldi step is three kernels: the new basis
-// vector scaled, multiplied by A and projected (h = V^T w); the projection
-// taken off and the remainder projected again; that taken off, and the norm.
-// Each kernel's last block to finish adds the blocks' partial sums in a fixed
-// order, and that of the third extends the Hessenberg matrix by its column and
-// rotates it, so a solve is bitwise reproducible, nothing waits for the host
+// independent dot products.  An Arnoldi step is four kernels: the new basis
+// vector scaled and multiplied by A; the product projected (h = V^T w; with up to
+// 2,048 rows in the kernel before); the projection taken off and the remainder
+// projected again; that taken off, and the norm.  Each kernel's last block to
+// finish adds the blocks' partial sums in a fixed order, and that of the last
+// extends the Hessenberg matrix by its column and rotates it, so a solve is bitwise reproducible, nothing waits for the host
 // within a restart cycle, and what is queued of a cycle that has converged returns
 // at once.  How far a cycle is the device writes to host memory, so that the host
 // queues nothing for a system that starts converged and, where a step is long,
@@ -39,16 +39,17 @@ constexpr int kProductLanes = 16;  // ... in the products without
 constexpr int kMaxRestart = 64;
 // Rows up to which a product and its dot products are one kernel (measured at
 // product_dots_kernel).
-constexpr index_t kFusedRows = 100000;
+constexpr index_t kFusedRows = 2048;
 
 // A progress past every step's: nothing more of this cycle is wanted.
 constexpr int kStopped = 1 << 30;
-// Where the first projection is a kernel of its own (above kFusedRows), a step is
-// queued once the last but one has finished: one that converges in its first step
-// takes 255 us at 500,000 rows, and 500 with up to twenty steps queued that then
-// return at once (31,250 blocks each in the product).  Below, the write to host
-// memory would cost a step 0.8 of its 16 us (8,000 rows) and the launches cost less.
+// Above kFollowRows a step is queued once the last but one has finished: a solve
+// that converges in its first step takes 255 us at 500,000 rows, and 500 with up to
+// twenty steps queued that then return at once (31,250 blocks each in the product).
+// Below, the write to host memory would cost a step 0.8 of its 16 us (8,000 rows)
+// and the launches cost less.
 constexpr int kAhead = 1;
+constexpr index_t kFollowRows = 100000;
 
 // The solve's scalars, in device memory.
 struct SolveState {
@@ -219,11 +220,12 @@ __global__ void __launch_bounds__(kSolveThreads) product_kernel(SolveArgs a, int
   }
 }
 
-// The same with the product's dot products with v_0 .. v_j, for systems whose
-// matrix stays in L2: a row's eight lanes take the basis vectors lane, lane + 8,
-// ..., and the four rows of a warp read whole sectors of them.  8,000 rows: 10
-// us against 7 + 5 in two kernels; 61,250: 31 against 23 + 8; 500,000: 181
-// against 138 + 14 (the vectors' loads hold up the row's).
+// The same with the product's dot products with v_0 .. v_j: a row's eight lanes
+// take the basis vectors lane, lane + 8, ..., and the four rows of a warp read whole
+// sectors of them.  It saves a launch and costs a wait per row, as the vectors'
+// loads hold up the row's.  A solve of 100 iterations, fused and in two kernels: 343
+// rows 1,740 and 1,815 us, 1,000 1,968 and 2,018, 3,120 2,038 and 1,966, 8,000 2,180
+// and 2,068, 61,250 4,772 and 4,393, 163,840 9,225 and 8,132.
 template <int Dots>
 __global__ void __launch_bounds__(kSolveThreads) product_dots_kernel(SolveArgs a, int j) {
   wait_for_previous();
@@ -559,7 +561,7 @@ lsmps_status solve_ppe_impl(lsmps_ctx* ctx, const lsmps_csr_matrix& A, const dou
     return fail(ctx, LSMPS_CUDA_ERROR, "pinned allocation failed");
   }
   a.progress = &pinned->progress;
-  a.follow = g.fused ? 0 : 1;
+  a.follow = n > kFollowRows ? 1 : 0;
   a.x = x;
   a.b = b;
   a.restart = m;
