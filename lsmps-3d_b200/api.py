@@ -126,7 +126,7 @@ class Context:
 
     def set_adjoint_atomic(self, on: bool) -> None:
         """Operator backward: scatter with FP64 atomics (True) or the
-        deterministic transpose + gather (False, the default)."""
+        deterministic records added in entry order (False, the default)."""
         self.check(_lib.lsmps_ctx_set_adjoint_atomic(self.h, 1 if on else 0))
 
     def set_condition_threshold(self, threshold: float) -> None:

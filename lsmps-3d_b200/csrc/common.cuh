@@ -328,7 +328,7 @@ struct lsmps_ctx {
   int32_t* adj_info = nullptr;
   int32_t* adj_count = nullptr;
   size_t adj_cap = 0;
-  // Backward form: false = transpose + gather (deterministic, the default),
+  // Backward form: false = records added in entry order (deterministic, the default),
   // true = scatter with FP64 atomics (lsmps_ctx_set_adjoint_atomic).
   bool adjoint_atomic = false;
   // The deterministic backward's records: the most that could be allocated when
@@ -426,14 +426,15 @@ __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontr
 
 // Launches may be early: a kernel's blocks are allowed onto the GPU as the blocks
 // of the kernel before it leave, and wait there, so that a launch's latency and
-// the drain of the one before overlap (a chain of N short launches costs about 1.6
-// us less each).  Not under capture, where graphs keep plain edges.  Before and
-// after: step of 1,000 particles 345 and 296 us, 21,793 mixed 538 and 444, 500,000
-// 4,028 and 3,960; solve of 8,000 rows 2,098 and 1,700 us.  Letting them in
-// earlier, from the moment the last block of the kernel before has started
-// (griddepcontrol.launch_dependents), gains no more on small sets (292, 472, 1,800)
-// and costs half as much again on large ones (500,000: 6,030): the places are taken
-// by blocks that wait, and unevenly over the SMs.
+// the drain of the one before overlap (a chain of N short launches costs about 2 us
+// less each).  Not under capture, where graphs keep plain edges.  Without and with:
+// step of 1,000 particles 309 and 241 us, 21,793 mixed 499 and 421, 500,000 3,994
+// and 3,919; solve of 8,000 rows 2,242 and 1,560 us.  Letting them in earlier, from
+// the moment the last block of the kernel before has started
+// (griddepcontrol.launch_dependents), gained next to nothing on small sets (292 us
+// where this took 296, 472 and 444) and cost half as much again on large ones
+// (500,000: 6,030 and 3,960): the places are taken by blocks that wait, and
+// unevenly over the SMs.
 template <typename Kernel, typename... Args>
 inline void launch_named(lsmps_ctx* ctx, const char* name, Kernel kernel, dim3 grid, dim3 block, size_t smem,
                          Args... args) {

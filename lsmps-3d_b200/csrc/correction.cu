@@ -1009,9 +1009,9 @@ __global__ void __launch_bounds__(kThreads) update_anti_penetration_kernel(const
 // For sets of at most kSmallUpdate particles, where the latency of index, record
 // and test per wall is what it takes: a block moves as many particles as it has
 // lane groups, a thread each, and then takes those of them with walls a group
-// each.  Event times: 1,000 particles 31 -> 13 us, 21,793: 33 -> 16, 61,250: 41 ->
-// 25; 500,000: 72 against 120, 2,000,000: 143 against 400 (blocks of 128 particles
-// there: 82 and 150).
+// each.  Event times, one thread a particle and groups: 8,000 particles 31 and 13 us,
+// 61,250 38 and 25, 122,880 50 and 40, 147,456 50 and 46, 196,000 52 and 57, 500,000 72
+// and 120, 2,000,000 143 and 400 (blocks of 128 particles there: 82 and 150).
 constexpr size_t kSmallUpdate = 131072;
 constexpr int kUpdateGroups = kUpdateThreads / kWallLanes;
 

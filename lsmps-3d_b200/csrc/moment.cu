@@ -5,12 +5,14 @@
 // potrs-per-identity-column inversion (:430-471).
 //
 // Every entry of a moment matrix's fluid sum is one of 31 (Type-A) or 35
-// (Type-B) weighted monomials, the same for all kinds.  Two kernels:
-// plain_sums_kernel adds them up, several lanes to a particle, with the wall
-// terms of the particles that have walls; moment_finish_kernel assembles, regularises and inverts one particle and kind per thread: the
-// textbook Cholesky factorisation (Golub & Van Loan, Alg. 4.2.1) in registers,
-// the in-place inverse of the triangular factor, and X = L^-T L^-1, stored
-// column-major and symmetric like the reference's inverse_matrices.
+// (Type-B) weighted monomials, the same for all kinds.  Three kernels:
+// plain_sums_kernel adds them up, one lane to a particle (in parts for small
+// sets), and lists the particles with walls; wall_sums_kernel adds the wall terms
+// of those; moment_finish_kernel assembles, regularises and inverts one particle
+// and kind per thread: the textbook Cholesky factorisation (Golub & Van Loan,
+// Alg. 4.2.1) in registers, the in-place inverse of the triangular factor, and
+// X = L^-T L^-1, stored column-major and symmetric like the reference's
+// inverse_matrices.
 #include <algorithm>
 #include <cmath>
 #include <utility>
