@@ -1016,6 +1016,20 @@ def run_reference(args, world, rank, local):
     return base
 
 
+def summary_of(out):
+    """The result line of a whole run: without the launch lists and the error study's distributions, which make it ten times
+    as long (some readers keep the last few kB only); they are in the details on stderr."""
+    def short(v):
+        if not isinstance(v, dict):
+            return v
+        drop = ("kernels", "neighbour_count_histogram", "labels", "kappa_by_label", "kappa_estimate", "state", "reference")
+        if "ppe_coefficients_max_rel_rowwise" in v:
+            return {k: v[k] for k in ("fp64_route_matrices", "ppe_coefficients_max_rel_rowwise", "ppe_rhs_rel")}
+        return {k: short(x) for k, x in v.items() if k not in drop}
+
+    return {k: short(v) for k, v in out.items() if k != "kernels"}
+
+
 def main():
     args = parse_args()
     world, rank, local = dist_setup(args)
@@ -1049,7 +1063,8 @@ def main():
     if rank == 0:
         if world == 1 and not args.no_cpu_baseline:
             out["cpu_baseline"] = cpu_baseline(WORKLOADS[args.workload][0])
-        print(json.dumps(out), flush=True)
+        print("details:", json.dumps(out), file=sys.stderr, flush=True)
+        print(json.dumps(summary_of(out)), flush=True)
     if world > 1:
         import torch.distributed as dist
 
