@@ -108,6 +108,7 @@ extern "C" lsmps_status lsmps_batch_create(int device, int streams, lsmps_batch*
       b->ctxs.push_back(ctx);
       lsmps_ctx_set_stream(ctx, st);
       lsmps_ctx_set_synchronous(ctx, 0);
+      ctx->shared_percent = 55;
     }
   }
   if (!ok) {

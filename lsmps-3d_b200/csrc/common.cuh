@@ -284,6 +284,16 @@ struct lsmps_ctx {
   bool step_packs = false;
   unsigned packs_ready = 0;
   const int32_t* packs_fluid_order = nullptr;
+  // Share of an SM's L1 and shared memory that every kernel of this context asks to
+  // have as shared memory, in percent; 0: as the driver finds for each kernel.  Set
+  // for the worker contexts of a batch, whose kernels run beside one another: an SM
+  // that has been split for a table pass (26 KB a block, all of 228 KB) stays so
+  // while any of its blocks runs, and the gathers that come in beside it, bound by the
+  // L1, are left 28 KB of it.  64 boxes of 8,000 to 200,000 particles on eight
+  // streams, mixed and plain: 56.9 and 52.8 ms without, 43.5 and 41.5 at 55 (their 32
+  // largest 47.6 and 47.0 without, 46.5 and 38.8 at 25, 37.3 and 33.5 at 35, 35.6 and
+  // 32.7 at 45 and 55, 35.3 and 33.1 at 65, 36.6 and 34.7 at 80).
+  unsigned shared_percent = 0;
   // 32-byte neighbour records (packed.cuh): two fluid and three wall arrays.
   double4* pack_fluid[2] = {nullptr, nullptr};
   double4* pack_wall[3] = {nullptr, nullptr, nullptr};
@@ -446,13 +456,18 @@ inline void launch_named(lsmps_ctx* ctx, const char* name, Kernel kernel, dim3 g
   config.blockDim = block;
   config.dynamicSmemBytes = smem;
   config.stream = ctx->stream;
-  cudaLaunchAttribute early{};
-  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attrs[2]{};
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   cudaStreamIsCapturing(ctx->stream, &capture);
-  config.attrs = &early;
-  config.numAttrs = capture == cudaStreamCaptureStatusNone ? 1 : 0;
+  if (capture == cudaStreamCaptureStatusNone) {
+    attrs[config.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[config.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (ctx->shared_percent) {
+    attrs[config.numAttrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attrs[config.numAttrs++].val.sharedMemCarveout = ctx->shared_percent;
+  }
+  config.attrs = attrs;
   cudaLaunchKernelEx(&config, kernel, args...);
   if (rec) cudaEventRecord(rec->stop, ctx->stream);
   ++ctx->launches;
