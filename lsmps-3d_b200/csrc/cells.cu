@@ -312,9 +312,11 @@ __device__ __forceinline__ void order_by_walk(const CellSet& set, const index_t*
 // places, finds how many of its cell come before its particle and writes the
 // particle to its own place of the sorted list.  The comparisons of a warp are with
 // one or two cells' particles, four a load, and those of a crowded cell are spread
-// over as many threads as it has particles.  Bound by latency.  A list of 2,000,000
-// particles, 27 a cell: 91 us in all (93 with one warp per cell, which took 15,100
-// with 1,025 of them in one cell; 91 here); 300,000: 34 (34; 2,340; 41).
+// over as many threads as it has particles.  Bound by latency: 20 us for 500,000
+// particles and 186,225 walls (72 with one warp per cell), 2,000,000 with theirs 64
+// (112).  A list of 2,000,000 particles, 27 a cell, takes 91 us in all (93 with one
+// warp per cell, which took 15,100 with 1,025 of them in one cell; 92 here); 300,000:
+// 34 (34; 2,340; 41).
 __global__ void __launch_bounds__(kOrderThreads) cell_order_kernel(const __grid_constant__ CellArgs a) {
   wait_for_previous();
   __shared__ index_t s_huge;
