@@ -310,7 +310,8 @@ struct lsmps_ctx {
   int32_t* moment_walled = nullptr;
   unsigned int* moment_walls = nullptr;
   size_t moment_terms_cap = 0;
-  double* retired[2] = {nullptr, nullptr};  // what the two replaced under capture
+  double* moment_block[2] = {nullptr, nullptr};  // the allocations behind them
+  double* retired[2] = {nullptr, nullptr};       // what those replaced under capture
   // Mixed form (LSMPS_PRECISION_MIXED): per fluid particle the compact FP32
   // operator rows of the velocity
   // and pressure inverses ([n][36]: Laplacian row, then rows 0, 1, 2), both

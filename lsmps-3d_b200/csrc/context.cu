@@ -70,17 +70,14 @@ bool ensure_mixed(lsmps_ctx* ctx, size_t nf) {
 }
 
 void free_moment_sums(lsmps_ctx* ctx) {
-  if (ctx->moment_sums) cudaFree(ctx->moment_sums);
-  if (ctx->moment_terms) cudaFree(ctx->moment_terms);
-  ctx->moment_sums = nullptr;
-  ctx->moment_cap = 0;
-  ctx->moment_terms = nullptr;
+  for (double** p : {&ctx->moment_block[0], &ctx->moment_block[1], &ctx->retired[0], &ctx->retired[1]}) {
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+  }
+  ctx->moment_sums = ctx->moment_terms = nullptr;
   ctx->moment_walled = nullptr;
   ctx->moment_walls = nullptr;
-  ctx->moment_terms_cap = 0;
-  for (double* p : ctx->retired)
-    if (p) cudaFree(p);
-  ctx->retired[0] = ctx->retired[1] = nullptr;
+  ctx->moment_cap = ctx->moment_terms_cap = 0;
 }
 
 namespace {
@@ -116,25 +113,33 @@ bool renew(lsmps_ctx* ctx, double** p, size_t bytes, double** retired) {
 
 bool ensure_moment_sums(lsmps_ctx* ctx, size_t nf) {
   if (nf <= ctx->moment_cap) return true;
-  if (!renew(ctx, &ctx->moment_sums, nf * 35 * sizeof(double), &ctx->retired[0])) {
-    if (!ctx->moment_sums) ctx->moment_cap = 0;
-    return false;
+  const bool ok = renew(ctx, &ctx->moment_block[0], nf * 35 * sizeof(double), &ctx->retired[0]);
+  if (ok || !ctx->moment_block[0]) {
+    ctx->moment_sums = ctx->moment_block[0];
+    ctx->moment_cap = ok ? nf : 0;
   }
-  ctx->moment_cap = nf;
-  return true;
+  return ok;
 }
 
 bool ensure_moment_terms(lsmps_ctx* ctx, size_t nf) {
   if (nf <= ctx->moment_terms_cap) return true;
-  // both boundaries' wall terms, the count of particles with walls and their list
-  const size_t doubles = nf * (31 + 45);
-  if (!renew(ctx, &ctx->moment_terms, doubles * sizeof(double) + (nf + 1) * sizeof(int32_t), &ctx->retired[1])) {
-    if (!ctx->moment_terms) ctx->moment_terms_cap = 0;
-    return false;
+  // the sums where they are missing too (one allocation costs less than two), both
+  // boundaries' wall terms, the count of particles with walls and their list
+  const bool sums = nf > ctx->moment_cap;
+  const size_t doubles = nf * ((sums ? 35 : 0) + 31 + 45);
+  const bool ok =
+      renew(ctx, &ctx->moment_block[1], doubles * sizeof(double) + (nf + 1) * sizeof(int32_t), &ctx->retired[1]);
+  if (ok || !ctx->moment_block[1]) {
+    if (sums) {  // (those at hand may have been in the block that went)
+      ctx->moment_sums = ctx->moment_block[1];
+      ctx->moment_cap = ok ? nf : 0;
+    }
+    ctx->moment_terms_cap = ok ? nf : 0;
   }
-  ctx->moment_walls = reinterpret_cast<unsigned int*>(ctx->moment_terms + doubles);
+  if (!ok) return false;
+  ctx->moment_terms = ctx->moment_block[1] + (sums ? nf * 35 : 0);
+  ctx->moment_walls = reinterpret_cast<unsigned int*>(ctx->moment_block[1] + doubles);
   ctx->moment_walled = reinterpret_cast<int32_t*>(ctx->moment_walls + 1);
-  ctx->moment_terms_cap = nf;
   return true;
 }
 
@@ -371,8 +376,8 @@ lsmps_status lsmps_ctx_reserve(lsmps_ctx* ctx, size_t fluid_capacity, size_t wal
   Scratch s(ctx);
   if (!s.reserve(need)) return fail(ctx, LSMPS_CUDA_ERROR, "scratch allocation failed");
   if (!ensure_packs(ctx, fluid_capacity, wall_capacity)) return fail(ctx, LSMPS_CUDA_ERROR, "pack allocation failed");
-  if (!ensure_moment_sums(ctx, fluid_capacity) ||
-      (ctx->precision == LSMPS_PRECISION_PLAIN && wall_capacity > 0 && !ensure_moment_terms(ctx, fluid_capacity)))
+  if ((ctx->precision == LSMPS_PRECISION_PLAIN && wall_capacity > 0 && !ensure_moment_terms(ctx, fluid_capacity)) ||
+      !ensure_moment_sums(ctx, fluid_capacity))
     return fail(ctx, LSMPS_CUDA_ERROR, "moment sums allocation failed");
   if (ctx->precision == LSMPS_PRECISION_MIXED && !ensure_mixed(ctx, fluid_capacity))
     return fail(ctx, LSMPS_CUDA_ERROR, "mixed-form allocation failed");

@@ -1608,7 +1608,7 @@ lsmps_status prepare_moments_impl(lsmps_ctx* ctx, const lsmps_fluid& fluid, cons
     ++(kinds[k].kind == LSMPS_MOMENT_PRESSURE_WALL_NEUMANN_B ? many10 : many9);
   }
   const bool with_walls = (dirichlet || neumann_terms) && walls.count > 0;
-  if (!ensure_moment_sums(ctx, fluid.count) || (with_walls && !ensure_moment_terms(ctx, fluid.count)))
+  if ((with_walls && !ensure_moment_terms(ctx, fluid.count)) || !ensure_moment_sums(ctx, fluid.count))
     return fail(ctx, LSMPS_CUDA_ERROR, "moment sums allocation failed");
   const index_t* srows = sorted_rows_of(ctx, fn, fluid.count);
   // (the list of particles with walls starts empty every time)
