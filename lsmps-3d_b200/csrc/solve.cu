@@ -594,7 +594,8 @@ lsmps_status solve_ppe_impl(lsmps_ctx* ctx, const lsmps_csr_matrix& A, const dou
     // (without a step the residual stands, but one of x = 0 has not met A yet,
     // whose NaN would show there)
     if (j > 0 || (first && !opt.use_initial_guess)) launch_residual(ctx, a, false, false, g);
-    if (!read()) return check_launch(ctx, "PPE solve");
+    // (a launch that failed leaves the state as it was, and the cycle would come again)
+    if (!read() || cudaPeekAtLastError() != cudaSuccess) return check_launch(ctx, "PPE solve");
     if (st.converged || st.iters >= opt.max_iters) break;
     pinned->progress = 1;
   }
