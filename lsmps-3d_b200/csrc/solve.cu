@@ -25,7 +25,6 @@
 // little that would not be wanted.
 #include <algorithm>
 #include <cmath>
-#include <cstddef>
 
 #include "impl.cuh"
 
@@ -51,14 +50,18 @@ constexpr int kStopped = 1 << 30;
 constexpr int kAhead = 1;
 constexpr index_t kFollowRows = 100000;
 
-// The solve's scalars, in device memory.
-struct SolveState {
+// What the host reads after a cycle.
+struct SolveHead {
   double beta, beta0, target;
   double scale;  // 1 / norm of the vector that the next product takes
   int iters;
   int steps;      // of this cycle
   int converged;  // the residual has reached the target
   int stop;       // the rest of this cycle's launches return at once
+};
+
+// The solve's scalars, in device memory.
+struct SolveState : SolveHead {
   unsigned tickets;
   double h[kMaxRestart + 1];                       // first projection of the step
   double h2[kMaxRestart + 1];                      // second projection
@@ -549,10 +552,9 @@ lsmps_status solve_ppe_impl(lsmps_ctx* ctx, const lsmps_csr_matrix& A, const dou
   a.st = scratch.take<SolveState>(1);
   if (!a.V || !a.w[0] || !a.w[1] || !dinv || !a.partial || !a.st)
     return fail(ctx, LSMPS_CUDA_ERROR, "scratch exhausted");
-  // pinned: the state's leading scalars read back after a cycle, and how far the
-  // cycle is
+  // pinned: what is read back after a cycle, and how far the cycle is
   struct Pinned {
-    SolveState state;
+    SolveHead state;
     volatile int progress;
   };
   static thread_local Pinned* pinned = nullptr;
@@ -573,12 +575,12 @@ lsmps_status solve_ppe_impl(lsmps_ctx* ctx, const lsmps_csr_matrix& A, const dou
     a.dinv = dinv;
   }
   cudaMemsetAsync(&a.st->tickets, 0, sizeof(unsigned), ctx->stream);
-  const SolveState& st = pinned->state;
+  const SolveHead& st = pinned->state;
   pinned->progress = 0;
   launch_residual(ctx, a, !opt.use_initial_guess, true, g);
   const auto read = [&]() {
-    return cudaMemcpyAsync(&pinned->state, a.st, offsetof(SolveState, tickets), cudaMemcpyDeviceToHost, ctx->stream) ==
-               cudaSuccess &&
+    return cudaMemcpyAsync(&pinned->state, static_cast<SolveHead*>(a.st), sizeof(SolveHead), cudaMemcpyDeviceToHost,
+                           ctx->stream) == cudaSuccess &&
            cudaStreamSynchronize(ctx->stream) == cudaSuccess;
   };
   // Waits until the cycle has come to `reached`, or until nothing is queued.
