@@ -79,7 +79,7 @@ def parse_args():
                          "(ill-conditioned Surface/Splash matrices: the mixed form's FP64 route at full size)")
     ap.add_argument("--knobs", default=None,
                     help="comma-separated launch-shape knob values (moment variant, PPE lanes, gather lanes) to use "
-                         "instead of autotuning, e.g. 2,1,1 (what the autotuner picks at 2M)")
+                         "instead of autotuning, e.g. 1,2,1 (what the autotuner picks for the mixed form at 2M; plain 0,1,1)")
     ap.add_argument("--kappa-threshold", type=float, default=None,
                     help="mixed form: condition-estimate threshold of the FP64 route (library default if omitted)")
     ap.add_argument("--precision", choices=["both", "plain", "mixed"], default="both",
